@@ -283,12 +283,22 @@ __device__ void epilogue_hidden(uint32_t tmem, int row, const float* bias, __nv_
     __align__(16) __nv_bfloat162 b[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float z0 = v[2 * i] + bias[c0 + 2 * i], z1 = v[2 * i + 1] + bias[c0 + 2 * i + 1];
-      if (z_out) {
-        z_out[c0 + 2 * i] = z0;
-        z_out[c0 + 2 * i + 1] = z1;
+      v[2 * i] += bias[c0 + 2 * i];
+      v[2 * i + 1] += bias[c0 + 2 * i + 1];
+      b[i] = __floats2bfloat162_rn(silu(v[2 * i]), silu(v[2 * i + 1]));
+    }
+    if (z_out) {
+      // a thread stores its own row: 16 bytes at a time where the caller's
+      // buffer allows it (a quarter of the store instructions)
+      if ((reinterpret_cast<uintptr_t>(z_out) & 15u) == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          reinterpret_cast<float4*>(z_out + c0)[q] =
+              make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) z_out[c0 + i] = v[i];
       }
-      b[i] = __floats2bfloat162_rn(silu(z0), silu(z1));
     }
     *reinterpret_cast<uint4*>(base + tc::kmajor_offset(row, c0, H)) =
         *reinterpret_cast<uint4*>(&b[0]);
@@ -429,8 +439,10 @@ __global__ void __launch_bounds__(kGroups * 128, 1) mlp_fwd_kernel(RowsIO A, int
   uint32_t ph = 0;
   bool ok = true;
   const int ntiles = (rows + 127) / 128;
+  // groups of one CTA take tiles gridDim.x apart, so that a batch of fewer
+  // tiles than SMs runs one tile per SM
   const int tile_step = kGroups * gridDim.x;
-  for (int tile = kGroups * blockIdx.x + grp; tile < ntiles && ok; tile += tile_step) {
+  for (int tile = blockIdx.x + grp * gridDim.x; tile < ntiles && ok; tile += tile_step) {
     const int row = tile * 128 + lt;
     const bool act_row = row < rows;
     // input tile (K = 48)
@@ -1100,6 +1112,14 @@ __global__ void __launch_bounds__(kM2lThreads) m2l_pairs_kernel(FarIO F) {
 // opA[m][k] = tA ? A[k*lda + m] : A[m*lda + k]; same for B.  Grid (M/128, N/128,
 // splitK); each CTA runs its K range in chunks of 128 through TMEM and adds its
 // partial into C with FP32 atomics (C must be zeroed when accumulating).
+// The tensor work of a chunk is under 100 ns; staging bounds the kernel, so an
+// operand moves eight K elements of a row (one 16-byte core-matrix row) at a
+// time: a 16-byte load where K is contiguous, and eight 4-byte loads of two
+// rows transposed in registers where the rows are.  The seven GEMMs of a gradient
+// pass over 8,192 rows: 3,615 us staged one element at a time with eight K
+// splits, 93 us so with 32 (two 128-row chunks a CTA).
+constexpr int kGemmThreads = 256;
+
 struct GemmSmem {
   __nv_bfloat16 a[128 * 128];
   __nv_bfloat16 b[128 * 128];
@@ -1107,11 +1127,66 @@ struct GemmSmem {
   uint32_t tmem;
 };
 
-__global__ void __launch_bounds__(128) gemm_tn_kernel(const __nv_bfloat16* __restrict__ A, int lda,
-                                                      int tA, const __nv_bfloat16* __restrict__ B,
-                                                      int ldb, int tB, float* __restrict__ C,
-                                                      int ldc, int M, int N, int K, int kchunk,
-                                                      int atomic) {
+// Stages op(X)[r0 .. r0+R)[k0 .. k0+kc) (zero beyond `rows` and kc) as a K-major
+// canonical tile of R rows x kc16 columns; R is even, kc16 a multiple of 16.
+// wide: the aligned accesses of the plan (checked by the host) are allowed.
+__device__ __forceinline__ void stage_operand(__nv_bfloat16* dst, const __nv_bfloat16* __restrict__ X,
+                                              int ld, int trans, bool wide, int r0, int R, int rows,
+                                              int k0, int kc, int kc16) {
+  char* base = reinterpret_cast<char*>(dst);
+  const int n8 = kc16 >> 3;
+  if (!trans) {
+    for (int e = threadIdx.x; e < R * n8; e += kGemmThreads) {
+      const int r = e / n8, k = 8 * (e - r * n8);
+      const __nv_bfloat16* src = X + static_cast<int64_t>(r0 + r) * ld + k0 + k;
+      __align__(16) __nv_bfloat16 v[8];
+      if (wide && r0 + r < rows && k + 8 <= kc) {
+        *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(src);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          v[i] = r0 + r < rows && k + i < kc ? src[i] : __float2bfloat16(0.f);
+      }
+      *reinterpret_cast<uint4*>(base + tc::kmajor_offset(r, k, kc16)) =
+          *reinterpret_cast<const uint4*>(v);
+    }
+    return;
+  }
+  const int half = R >> 1;
+  for (int e = threadIdx.x; e < half * n8; e += kGemmThreads) {
+    const int k8 = e / half, r = 2 * (e - k8 * half), k = 8 * k8;
+    const __nv_bfloat16* src = X + static_cast<int64_t>(k0 + k) * ld + r0 + r;
+    __align__(16) __nv_bfloat16 v0[8], v1[8];
+    if (wide && r0 + r + 2 <= rows && k + 8 <= kc) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const __nv_bfloat162 p =
+            *reinterpret_cast<const __nv_bfloat162*>(src + static_cast<int64_t>(i) * ld);
+        v0[i] = p.x;
+        v1[i] = p.y;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const bool in = k + i < kc;
+        v0[i] = in && r0 + r < rows ? src[static_cast<int64_t>(i) * ld] : __float2bfloat16(0.f);
+        v1[i] = in && r0 + r + 1 < rows ? src[static_cast<int64_t>(i) * ld + 1]
+                                        : __float2bfloat16(0.f);
+      }
+    }
+    *reinterpret_cast<uint4*>(base + tc::kmajor_offset(r, k, kc16)) =
+        *reinterpret_cast<const uint4*>(v0);
+    *reinterpret_cast<uint4*>(base + tc::kmajor_offset(r + 1, k, kc16)) =
+        *reinterpret_cast<const uint4*>(v1);
+  }
+}
+
+// wide_a, wide_b: the operand's 16-byte (4-byte where transposed) accesses are
+// aligned; wide_c: four columns of C are one aligned 16-byte access.
+__global__ void __launch_bounds__(kGemmThreads) gemm_tn_kernel(
+    const __nv_bfloat16* __restrict__ A, int lda, int tA, int wide_a,
+    const __nv_bfloat16* __restrict__ B, int ldb, int tB, int wide_b, float* __restrict__ C,
+    int ldc, int wide_c, int M, int N, int K, int kchunk, int atomic) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   GemmSmem& S = *reinterpret_cast<GemmSmem*>(smem_raw);
   if (threadIdx.x < 32) tc::tmem_alloc(&S.tmem, 128);
@@ -1132,21 +1207,8 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(const __nv_bfloat16* __res
   for (int k0 = kb; k0 < ke; k0 += 128) {
     const int kc = min(128, ke - k0);
     const int kc16 = (kc + 15) & ~15;
-    // stage op(A)[m0 .. m0+128][k0 .. k0+kc16] and op(B)[n0 .. n0+nt16][...]
-    for (int e = threadIdx.x; e < 128 * kc16; e += blockDim.x) {
-      const int r = tA ? e % 128 : e / kc16, k = tA ? e / 128 : e % kc16;
-      const int gm = m0 + r, gk = k0 + k;
-      __nv_bfloat16 v = __float2bfloat16(0.f);
-      if (gm < M && k < kc) v = tA ? A[static_cast<int64_t>(gk) * lda + gm] : A[static_cast<int64_t>(gm) * lda + gk];
-      *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<char*>(S.a) + tc::kmajor_offset(r, k, kc16)) = v;
-    }
-    for (int e = threadIdx.x; e < nt16 * kc16; e += blockDim.x) {
-      const int r = tB ? e % nt16 : e / kc16, k = tB ? e / nt16 : e % kc16;
-      const int gn = n0 + r, gk = k0 + k;
-      __nv_bfloat16 v = __float2bfloat16(0.f);
-      if (r < nt && k < kc) v = tB ? B[static_cast<int64_t>(gk) * ldb + gn] : B[static_cast<int64_t>(gn) * ldb + gk];
-      *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<char*>(S.b) + tc::kmajor_offset(r, k, kc16)) = v;
-    }
+    stage_operand(S.a, A, lda, tA, wide_a, m0, 128, M, k0, kc, kc16);
+    stage_operand(S.b, B, ldb, tB, wide_b, n0, nt16, N, k0, kc, kc16);
     tc::fence_smem_to_async();
     tc::fence_before_sync();
     __syncthreads();
@@ -1160,20 +1222,34 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(const __nv_bfloat16* __res
     }
   }
   if (ok && any) {
+    // warps 0-3 read the accumulator's 128 rows in the first half of the
+    // 16-column groups' alternation, warps 4-7 in the other
+    const int row = threadIdx.x & 127;
     const uint32_t lb = static_cast<uint32_t>(32 * ((threadIdx.x >> 5) & 3)) << 16;
-    const int gm = m0 + threadIdx.x;
-    for (int c0 = 0; c0 < nt16; c0 += 16) {
+    const int gm = m0 + row;
+    for (int c0 = 16 * (threadIdx.x >> 7); c0 < nt16; c0 += 32) {
       float v[16];
       tc::tmem_ld16(tmem + lb + c0, v);
       if (gm >= M) continue;
+      float* p = C + static_cast<int64_t>(gm) * ldc + n0 + c0;
+      if (wide_c && c0 + 16 <= nt) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float4 x = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          if (atomic)
+            atomicAdd(reinterpret_cast<float4*>(p) + q, x);
+          else
+            reinterpret_cast<float4*>(p)[q] = x;
+        }
+        continue;
+      }
+#pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const int gn = n0 + c0 + i;
         if (c0 + i >= nt) break;
-        float* p = C + static_cast<int64_t>(gm) * ldc + gn;
         if (atomic)
-          atomicAdd(p, v[i]);
+          atomicAdd(p + i, v[i]);
         else
-          *p = v[i];
+          p[i] = v[i];
       }
     }
   }
@@ -1405,8 +1481,8 @@ int fvx_mlp_forward(const void* X, int rows, const void* W, const float* bias, f
   }
   const RowsIO A{static_cast<const __nv_bfloat16*>(X), Y, z_store,
                  static_cast<__nv_bfloat16*>(h_store)};
-  const int nctas = ((rows + 127) / 128 + kGroups - 1) / kGroups;
-  const int grid = nctas < fvx::device_sm_count() ? nctas : fvx::device_sm_count();
+  const int ntiles = (rows + 127) / 128;
+  const int grid = ntiles < fvx::device_sm_count() ? ntiles : fvx::device_sm_count();
   // without stores it is inference: the arithmetic the treecode far field runs
   auto kern = (z_store || h_store) ? mlp_fwd_kernel<false> : mlp_fwd_kernel<true>;
   kern<<<grid, kGroups * 128, sizeof(FwdSmem), static_cast<cudaStream_t>(stream)>>>(
@@ -1430,9 +1506,17 @@ int fvx_mlp_gemm(const void* A, int lda, int tA, const void* B, int ldb, int tB,
   kchunk = (kchunk + 127) & ~127;
   const int sk = (K + kchunk - 1) / kchunk;
   dim3 grid((M + 127) / 128, (N + 127) / 128, sk);
-  gemm_tn_kernel<<<grid, 128, sizeof(GemmSmem), static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(A), lda, tA, static_cast<const __nv_bfloat16*>(B), ldb,
-      tB, C, ldc, M, N, K, kchunk, accumulate);
+  // wide accesses only where every row's start is aligned (K chunks start at
+  // multiples of 128, tiles at multiples of 128 rows)
+  auto wide = [](const void* p, int ld, int trans) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    return trans ? (a % 4 == 0 && ld % 2 == 0) : (a % 16 == 0 && ld % 8 == 0);
+  };
+  const int wide_c = reinterpret_cast<uintptr_t>(C) % 16 == 0 && ldc % 4 == 0;
+  gemm_tn_kernel<<<grid, kGemmThreads, sizeof(GemmSmem), static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(A), lda, tA, wide(A, lda, tA),
+      static_cast<const __nv_bfloat16*>(B), ldb, tB, wide(B, ldb, tB), C, ldc, wide_c, M, N, K,
+      kchunk, accumulate);
   FVX_LAUNCH_CHECK();
   return FVX_OK;
 }

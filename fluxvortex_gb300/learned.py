@@ -157,7 +157,7 @@ class FarFieldMLP:
                                           None if weights is None else weights.data_ptr(),
                                           bf["dY"].data_ptr(), bf["dY32"].data_ptr(),
                                           bf["loss"].data_ptr(), st))
-        split = max(1, rows // 1024)
+        split = max(1, rows // 256)      # two 128-row chunks per CTA
         gw, wb = self.gw.data_ptr(), self.wb.data_ptr()
         es_w, es_b = self.gw.element_size(), self.wb.element_size()
         # output layer
