@@ -140,7 +140,7 @@ __device__ void build_lattice(Smem& S, const FlutterParams& p) {
     S.normal[k][1] = cy / nrm;
     S.normal[k][2] = cz / nrm;
     S.area[k] = 0.5 * nrm;
-    seg::prep_vortex<FVX_LEGS_RING>(S.bound[k], br, fr, fl, bl, 1.0, p.rc0, 0.0, p.nu);
+    seg::prep_vortex<FVX_LEGS_RING, true>(S.bound[k], br, fr, fl, bl, 1.0, p.rc0, 0.0, p.nu);
   }
 }
 
@@ -212,7 +212,7 @@ __device__ void build_lattice_reference(Smem& S, const FlutterParams& p) {
     S.normal[k][1] = cy / nrm;
     S.normal[k][2] = cz / nrm;
     S.area[k] = 0.5 * nrm;
-    seg::prep_vortex<FVX_LEGS_RING>(S.bound[k], br, fr, fl, bl, 1.0, p.rc0, 0.0, p.nu);
+    seg::prep_vortex<FVX_LEGS_RING, true>(S.bound[k], br, fr, fl, bl, 1.0, p.rc0, 0.0, p.nu);
   }
 }
 
@@ -297,7 +297,7 @@ __device__ void wake_induction(Smem& S, const FlutterParams& p, const FlutterSta
       vz = fz;
     } else {
       for (int r = sl + crank * slices; r < R * p.ns; r += slices * CL)
-        seg::vortex_velocity<FVX_LEGS_RING>(S.wake[r], px, py, pz, vx, vy, vz, cnt);
+        seg::vortex_velocity_general<FVX_LEGS_RING, true>(S.wake[r], px, py, pz, vx, vy, vz, cnt);
     }
   }
   // particles, staged in tiles, oldest first
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
     }
     for (int k = threadIdx.x; k < R * p.ns; k += blockDim.x) {
       const int r = k / p.ns, j = k % p.ns;
-      seg::prep_vortex<FVX_LEGS_RING>(S.wake[k], S.W[r + 1][j + 1], S.W[r][j + 1], S.W[r][j],
+      seg::prep_vortex<FVX_LEGS_RING, true>(S.wake[k], S.W[r + 1][j + 1], S.W[r][j + 1], S.W[r][j],
                                       S.W[r + 1][j], S.wgam[r][j], p.rc0, S.wage[r], p.nu);
     }
     __syncthreads();
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
       const int i = e / P, j = e % P;
       double vx = 0.0, vy = 0.0, vz = 0.0;
       int cnt[4] = {0, 0, 0, 0};
-      seg::vortex_velocity<FVX_LEGS_RING>(S.bound[j], S.colloc[i][0], S.colloc[i][1],
+      seg::vortex_velocity_general<FVX_LEGS_RING, true>(S.bound[j], S.colloc[i][0], S.colloc[i][1],
                                           S.colloc[i][2], vx, vy, vz, cnt);
       S.A[i][j] = vx * S.normal[i][0] + vy * S.normal[i][1] + vz * S.normal[i][2];
     }
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
       double vx = 0.0, vy = 0.0, vz = 0.0;
       int cnt[4] = {0, 0, 0, 0};
       for (int j = 0; j < P; ++j)
-        seg::vortex_velocity<FVX_LEGS_RING>(S.bound[j], S.legc[k][0], S.legc[k][1], S.legc[k][2],
+        seg::vortex_velocity_general<FVX_LEGS_RING, true>(S.bound[j], S.legc[k][0], S.legc[k][1], S.legc[k][2],
                                             vx, vy, vz, cnt);
       const double Vx = (ux - S.vleg[k][0]) + (S.Vind[P + k][0] + vx);
       const double Vy = (uy - S.vleg[k][1]) + (S.Vind[P + k][1] + vy);

