@@ -11,14 +11,21 @@
 //   in FP64 or -- mixed precision -- in FP32 on FP64 offsets with compensated
 //   particle sums (particles staged through shared memory, split over thread
 //   slices, slices reduced in fixed order); the
-//   right-hand side; an in-place LU solve with partial pivoting (first
-//   largest pivot, as LAPACK's getrf); Kutta-Joukowski forces on the bound
+//   right-hand side; an LU solve with partial pivoting (first largest
+//   pivot, as LAPACK's getrf); Kutta-Joukowski forces on the bound
 //   legs with the full induced velocity and the unsteady term; station lift
 //   and torque about the elastic axis distributed to the beam nodes; the
 //   Newmark average-acceleration step with the precomputed inverse of the
 //   effective stiffness; the tip history; the wake update (convect with the
 //   freestream, shed the trailing-edge row at the new geometry, convert the
 //   row past n_keep into 4 particles per ring, FIFO-capped particle store).
+// The FP64 pipe bounds a step (1.7 operations per clock and SM), so the step's
+// serial parts are spread over the warps and the mixed-precision sums keep off
+// it (diff_f32) -- all bit for bit the sums they were, since the FP32 ring law
+// amplifies a rounding difference anywhere upstream.  64 airspeeds, 20 chords,
+// mixed precision: 104.3 ms with the loads' bound rings on one warp, both CTAs
+// forming the whole AIC, one thread searching the pivots and converting rows,
+// and eleven FP64 operations and conversions per particle; 37.5 ms so.
 // Reference: src/fluxvortex/aeroelastic_solver.py:68-221 and beam_fe.py:231-351
 // around PteraSoftware's ring-vortex UVLM; the PteraSoftware-free model is
 // described in fluxvortex_gb300/flutter.py.
@@ -39,28 +46,70 @@ constexpr int kMaxDof = 48;     // beam DOF (all nodes)
 constexpr int kTile = 128;      // particles staged per tile
 constexpr double kC = -0.07957747154594767;  // -1/(4 pi): particle strength scaling
 
+constexpr int kLegItems = 256;  // (point, ring) pairs per pass of the loads' leg terms
+constexpr int kLegStride = 17;  // doubles per pair: 4 legs of (c4, r3), one of padding
+
+// A wake ring for the mixed-precision sweep: corners in FP64 and as the sum of
+// two floats, and the leg constants rounded once here instead of per point.
+struct RingF32 {
+  double c[4][3];
+  float hi[4][3], lo[4][3];
+  float c2[4], tol[4];
+  float c1;
+  int valid;
+};
+
 struct Smem {
   double verts[kMaxNV][3], vvel[kMaxNV][3];
   double colloc[kMaxP][3], normal[kMaxP][3], legc[kMaxP][3], legv[kMaxP][3];
   double vcol[kMaxP][3], vleg[kMaxP][3], area[kMaxP];
   seg::VortexRec bound[kMaxP];
-  seg::VortexRec wake[kMaxRows * kMaxNS];
-  double A[kMaxP][kMaxP + 1];
+  union {  // the wake's rings, FP64 or mixed precision
+    seg::VortexRec wake[kMaxRows * kMaxNS];
+    RingF32 wakef[kMaxRows * kMaxNS];
+  };
+  double A[kMaxP][kMaxP + 1];  // AIC; the right-hand side is column P of the LU
   double rhs[kMaxP], gam[kMaxP], gprev[kMaxP];
   double Vind[2 * kMaxP][3];
   double Vsum[2 * kMaxP][3];  // cluster form: both CTAs' partial inductions summed
+  double Vbound[kMaxP][3];    // bound rings at the bound-leg centres
   double W[kMaxRows + 1][kMaxNS + 1][3];
   double wgam[kMaxRows][kMaxNS], wage[kMaxRows];
   double d[kMaxDof], v[kMaxDof], a[kMaxDof], F[kMaxDof], feff[kMaxDof], gd[kMaxDof];
   double tile[kTile][8];  // staged particles: x y z | a' (C-scaled) | sigma^2, 2.5 sigma^2
+  // mixed precision: x y z as two floats each, a', sigma^2, 2.5 sigma^2
+  __align__(16) float tile_hi[kTile][4], tile_lo[kTile][4], tile_a[kTile][4];
+  double legs[kLegItems * kLegStride];
+  int perm[kMaxP];
+  int lu_ok;
   double red[8];
-  int piv;
 };
 
-__device__ __forceinline__ void vadd(double* o, double x, double y, double z) {
-  o[0] += x;
-  o[1] += y;
-  o[2] += z;
+static_assert(sizeof(Smem) <= 227 * 1024, "the environment's state must fit shared memory");
+
+// float(x - y) of FP64 x and y, each given as hi + lo as well (hi = float(x),
+// lo = float(x - hi)): the float of the rounded FP64 difference, bit for bit,
+// without the FP64 pipe (one subtraction and one conversion cost it about 130
+// FP32 issue slots).  hi and lo differ from x by 2^-48 |x| at most; the exact
+// difference of the his (two_sum of Knuth) plus that of the los is within
+// 2^-44 (|x| + |y|) of x - y, FP64's own rounding included.  Where adding and
+// taking off that bound rounds to the same float, that float is the answer;
+// else (2^-20 |x| / |x - y| of the pairs) `same` is cleared and the caller
+// takes the FP64 way.
+__device__ __forceinline__ float diff_f32(float xh, float xl, float yh, float yl, bool& same) {
+  const float h = xh - yh;
+  const float bb = h - xh;
+  const float e = (xh - (h - bb)) - (yh + bb);
+  const float l = e + (xl - yl);
+  const float t = fabsf(xh) + fabsf(yh);
+  const float r0 = h + fmaf(t, -5.684341886080802e-14f, l);  // 2^-44
+  const float r1 = h + fmaf(t, 5.684341886080802e-14f, l);
+  same = same && r0 == r1;
+  return r0;
+}
+__device__ __forceinline__ void split_f32(double x, float& hi, float& lo) {
+  hi = static_cast<float>(x);
+  lo = static_cast<float>(x - static_cast<double>(hi));
 }
 
 // Deformed vertices and their velocities from the beam state in S.d / S.v.
@@ -229,35 +278,67 @@ __device__ void trailing_edge_reference(const Smem& S, const FlutterParams& p, d
   ref_move(p, w, sn, c1, out);
 }
 
-// One wake ring at point p in FP32 on offsets taken in FP64 (the ring-vortex
-// formula and skip tests of seg::vortex_velocity, ring leg set).
-__device__ __forceinline__ void ring_velocity_f32(const seg::VortexRec& R, double px, double py,
-                                                  double pz, float& vx, float& vy, float& vz) {
-  float dx[4], dy[4], dz[4], len[4];
+// The mixed-precision record of a wake ring (prep_vortex's constants, rounded).
+__device__ __forceinline__ void prep_ring_f32(RingF32& Q, const double* br, const double* fr,
+                                              const double* fl, const double* bl, double strength,
+                                              double rc0, double age, double nu) {
+  seg::VortexRec R;
+  seg::prep_vortex<FVX_LEGS_RING, true>(R, br, fr, fl, bl, strength, rc0, age, nu);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    dx[c] = static_cast<float>(R.c[c][0] - px);
-    dy[c] = static_cast<float>(R.c[c][1] - py);
-    dz[c] = static_cast<float>(R.c[c][2] - pz);
-    len[c] = sqrtf(dx[c] * dx[c] + dy[c] * dy[c] + dz[c] * dz[c]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      Q.c[c][k] = R.c[c][k];
+      split_f32(R.c[c][k], Q.hi[c][k], Q.lo[c][k]);
+    }
+    Q.c2[c] = static_cast<float>(R.c2[c]);
+    Q.tol[c] = static_cast<float>(R.tol[c]);
   }
-  const float c1 = static_cast<float>(R.c1);
+  Q.c1 = static_cast<float>(R.c1);
+  Q.valid = R.valid;
+}
+
+// A target point of the wake induction, in FP64 and as two floats.
+struct Point {
+  double p[3];
+  float hi[3], lo[3];
+};
+
+// One wake ring at a point in FP32 on the FP64 offsets' floats (the
+// ring-vortex formula and skip tests of seg::vortex_legs, ring leg set).
+__device__ __forceinline__ void ring_velocity_f32(const RingF32& R, const Point& P, float& vx,
+                                                  float& vy, float& vz) {
+  float d[4][3], len[4];
+  bool same = true;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      d[c][k] = diff_f32(R.hi[c][k], R.lo[c][k], P.hi[k], P.lo[k], same);
+  if (!same) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) d[c][k] = static_cast<float>(R.c[c][k] - P.p[k]);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    len[c] = sqrtf(d[c][0] * d[c][0] + d[c][1] * d[c][1] + d[c][2] * d[c][2]);
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
     const int a = l, b = (l + 1) & 3;
     if (!((R.valid >> l) & 1)) continue;
-    const float tol = static_cast<float>(R.tol[l]);
+    const float tol = R.tol[l];
     if (len[a] < tol || len[b] < tol) continue;
-    const float r3x = dy[a] * dz[b] - dz[a] * dy[b];
-    const float r3y = dz[a] * dx[b] - dx[a] * dz[b];
-    const float r3z = dx[a] * dy[b] - dy[a] * dx[b];
+    const float r3x = d[a][1] * d[b][2] - d[a][2] * d[b][1];
+    const float r3y = d[a][2] * d[b][0] - d[a][0] * d[b][2];
+    const float r3z = d[a][0] * d[b][1] - d[a][1] * d[b][0];
     const float r3_sq = r3x * r3x + r3y * r3y + r3z * r3z;
     const float r1r2 = len[a] * len[b];
     const float thr = 1.0e-10f * r1r2;
     if (r3_sq < 2.f * thr * thr && sqrtf(r3_sq) < thr) continue;
-    const float c3 = dx[a] * dx[b] + dy[a] * dy[b] + dz[a] * dz[b];
-    const float c4 = c1 * (len[a] + len[b]) * (r1r2 - c3) /
-                     (r1r2 * (r3_sq + static_cast<float>(R.c2[l])));
+    const float c3 = d[a][0] * d[b][0] + d[a][1] * d[b][1] + d[a][2] * d[b][2];
+    const float c4 = R.c1 * (len[a] + len[b]) * (r1r2 - c3) / (r1r2 * (r3_sq + R.c2[l]));
     vx += c4 * r3x;
     vy += c4 * r3y;
     vz += c4 * r3z;
@@ -278,11 +359,18 @@ __device__ void wake_induction(Smem& S, const FlutterParams& p, const FlutterSta
   const int tgt = threadIdx.x % T2, sl = threadIdx.x / T2;
   const bool active = sl < slices;
   double px = 0.0, py = 0.0, pz = 0.0;
+  Point pt = {};
   if (active) {
     const double* q = tgt < P ? S.colloc[tgt] : S.legc[tgt - P];
     px = q[0];
     py = q[1];
     pz = q[2];
+    if constexpr (F32) {
+      for (int k = 0; k < 3; ++k) {
+        pt.p[k] = q[k];
+        split_f32(q[k], pt.hi[k], pt.lo[k]);
+      }
+    }
   }
   // wake rings: slice sl takes rings sl, sl + slices, ...
   double vx = 0.0, vy = 0.0, vz = 0.0;
@@ -291,7 +379,7 @@ __device__ void wake_induction(Smem& S, const FlutterParams& p, const FlutterSta
     if constexpr (F32) {
       float fx = 0.f, fy = 0.f, fz = 0.f;
       for (int r = sl + crank * slices; r < R * p.ns; r += slices * CL)
-        ring_velocity_f32(S.wake[r], px, py, pz, fx, fy, fz);
+        ring_velocity_f32(S.wakef[r], pt, fx, fy, fz);
       vx = fx;
       vy = fy;
       vz = fz;
@@ -315,26 +403,44 @@ __device__ void wake_induction(Smem& S, const FlutterParams& p, const FlutterSta
       S.tile[e][0] = pp[3 * q];
       S.tile[e][1] = pp[3 * q + 1];
       S.tile[e][2] = pp[3 * q + 2];
-      S.tile[e][3] = kC * pa[3 * q];
-      S.tile[e][4] = kC * pa[3 * q + 1];
-      S.tile[e][5] = kC * pa[3 * q + 2];
-      S.tile[e][6] = s * s;
-      S.tile[e][7] = 2.5 * s * s;
+      if constexpr (F32) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          split_f32(S.tile[e][k], S.tile_hi[e][k], S.tile_lo[e][k]);
+          S.tile_a[e][k] = static_cast<float>(kC * pa[3 * q + k]);
+        }
+        S.tile_hi[e][3] = static_cast<float>(s * s);
+        S.tile_lo[e][3] = static_cast<float>(2.5 * s * s);
+      } else {
+        S.tile[e][3] = kC * pa[3 * q];
+        S.tile[e][4] = kC * pa[3 * q + 1];
+        S.tile[e][5] = kC * pa[3 * q + 2];
+        S.tile[e][6] = s * s;
+        S.tile[e][7] = 2.5 * s * s;
+      }
     }
     __syncthreads();
     if (!active) continue;
     for (int e = sl; e < nt; e += slices) {
       const double* s = S.tile[e];
       if constexpr (F32) {
-        // FP32 pair arithmetic on the exact FP64 offset, compensated sums
-        const float dx = static_cast<float>(px - s[0]), dy = static_cast<float>(py - s[1]),
-                    dz = static_cast<float>(pz - s[2]);
+        // FP32 pair arithmetic on the FP64 offset's float, compensated sums
+        const float4 sh = *reinterpret_cast<const float4*>(S.tile_hi[e]);
+        const float4 sl4 = *reinterpret_cast<const float4*>(S.tile_lo[e]);
+        const float4 av = *reinterpret_cast<const float4*>(S.tile_a[e]);
+        bool same = true;
+        float dx = diff_f32(pt.hi[0], pt.lo[0], sh.x, sl4.x, same);
+        float dy = diff_f32(pt.hi[1], pt.lo[1], sh.y, sl4.y, same);
+        float dz = diff_f32(pt.hi[2], pt.lo[2], sh.z, sl4.z, same);
+        if (!same) {
+          dx = static_cast<float>(px - s[0]);
+          dy = static_cast<float>(py - s[1]);
+          dz = static_cast<float>(pz - s[2]);
+        }
         const float r2 = dx * dx + dy * dy + dz * dz;
         float f, fpr;
-        pair::core_f32<FVX_KERNEL_WINCKELMANS, false>(r2, static_cast<float>(s[6]),
-                                                      static_cast<float>(s[7]), f, fpr);
-        const float ax = static_cast<float>(s[3]), ay = static_cast<float>(s[4]),
-                    az = static_cast<float>(s[5]);
+        pair::core_f32<FVX_KERNEL_WINCKELMANS, false>(r2, sh.w, sl4.w, f, fpr);
+        const float ax = av.x, ay = av.y, az = av.z;
         const float ex = f * dx, ey = f * dy, ez = f * dz;
         const float ux = ey * az - ez * ay, uy = ez * ax - ex * az, uz = ex * ay - ey * ax;
         float t = hx + ux;
@@ -407,71 +513,110 @@ __device__ void wake_induction(Smem& S, const FlutterParams& p, const FlutterSta
   }
 }
 
-// In-place LU solve of S.A x = S.rhs (partial pivoting, first largest |pivot|).
+// LU solve of S.A x = S.rhs into S.gam (partial pivoting, first largest
+// |pivot|).  Four warps (one per SM quarter's FP64 pipe) eliminate the rows
+// under each pivot, the right-hand side being column P; every warp finds the
+// pivot itself, by integer comparisons of the magnitudes' words, and rows are
+// permuted by index, so a step costs one barrier.  The chain of a step is
+// pivot search, reciprocal, one multiplier per row, one FMA per element.
+constexpr int kLuWarps = 4;
+
 __device__ bool lu_solve(Smem& S, int P) {
-  bool ok = true;
-  for (int k = 0; k < P; ++k) {
-    if (threadIdx.x == 0) {
-      int piv = k;
-      double best = fabs(S.A[k][k]);
-      for (int i = k + 1; i < P; ++i) {
-        const double v = fabs(S.A[i][k]);
-        if (v > best) {
-          best = v;
-          piv = i;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < P; i += blockDim.x) S.A[i][P] = S.rhs[i];
+  __syncthreads();
+  const int nw = min(kLuWarps, static_cast<int>(blockDim.x) >> 5);
+  if (warp < nw) {
+    int p0 = lane, p1 = lane + 32;  // physical rows of logical rows lane, lane + 32
+    bool ok = true;
+    for (int k = 0; k < P; ++k) {
+      // |A[i][k]| as (hi, lo) words; rows above k and NaNs count as zero
+      unsigned h0 = 0, l0 = 0, h1 = 0, l1 = 0;
+      bool nan_diag = false;
+      if (lane >= k && lane < P) {
+        const double v = S.A[p0][k];
+        h0 = __double2hiint(v) & 0x7fffffff;
+        l0 = __double2loint(v);
+        if (v != v) {
+          nan_diag = lane == k;
+          h0 = l0 = 0;
         }
       }
-      S.piv = best > 0.0 ? piv : -1;
-    }
-    __syncthreads();
-    const int piv = S.piv;
-    if (piv < 0) {
-      ok = false;
-      break;
-    }
-    if (piv != k) {
-      for (int j = threadIdx.x; j < P; j += blockDim.x) {
-        const double t = S.A[k][j];
-        S.A[k][j] = S.A[piv][j];
-        S.A[piv][j] = t;
+      if (lane + 32 >= k && lane + 32 < P) {
+        const double v = S.A[p1][k];
+        h1 = __double2hiint(v) & 0x7fffffff;
+        l1 = __double2loint(v);
+        if (v != v) {
+          nan_diag = nan_diag || lane + 32 == k;
+          h1 = l1 = 0;
+        }
       }
-      if (threadIdx.x == 0) {
-        const double t = S.rhs[k];
-        S.rhs[k] = S.rhs[piv];
-        S.rhs[piv] = t;
+      const unsigned hm = __reduce_max_sync(0xffffffffu, max(h0, h1));
+      const unsigned c0 = h0 == hm ? l0 : 0u, c1 = h1 == hm ? l1 : 0u;
+      const unsigned lm = __reduce_max_sync(0xffffffffu, max(c0, c1));
+      if (__any_sync(0xffffffffu, nan_diag) || (hm | lm) == 0) {
+        ok = false;
+        break;
       }
+      const unsigned b0 =
+          __ballot_sync(0xffffffffu, lane >= k && lane < P && h0 == hm && l0 == lm);
+      const unsigned b1 =
+          __ballot_sync(0xffffffffu, lane + 32 >= k && lane + 32 < P && h1 == hm && l1 == lm);
+      const int piv = b0 ? __ffs(b0) - 1 : 31 + __ffs(b1);
+      // swap logical rows k and piv
+      const int pk = __shfl_sync(0xffffffffu, k < 32 ? p0 : p1, k & 31);
+      const int pp = __shfl_sync(0xffffffffu, piv < 32 ? p0 : p1, piv & 31);
+      if (lane == k) p0 = pp;
+      if (lane + 32 == k) p1 = pp;
+      if (piv != k) {
+        if (lane == piv) p0 = pk;
+        if (lane + 32 == piv) p1 = pk;
+      }
+      const double inv = 1.0 / S.A[pp][k];
+      // this lane's rows' multipliers; the warp's rows take them by shuffles
+      double m0 = 0.0, m1 = 0.0;
+      if (lane > k && lane < P) m0 = S.A[p0][k] * inv;
+      if (lane + 32 > k && lane + 32 < P) m1 = S.A[p1][k] * inv;
+      // columns k + 1 .. P (P: the right-hand side)
+      const int j0 = k + 1 + lane, j1 = j0 + 32, j2 = j1 + 32;
+      const double u0 = j0 <= P ? S.A[pp][j0] : 0.0;
+      const double u1 = j1 <= P ? S.A[pp][j1] : 0.0;
+      const double u2 = j2 <= P ? S.A[pp][j2] : 0.0;
+      for (int i = k + 1 + warp; i < P; i += nw) {
+        const double l = __shfl_sync(0xffffffffu, i < 32 ? m0 : m1, i & 31);
+        const int r = __shfl_sync(0xffffffffu, i < 32 ? p0 : p1, i & 31);
+        if (j0 <= P) S.A[r][j0] -= l * u0;
+        if (j1 <= P) S.A[r][j1] -= l * u1;
+        if (j2 <= P) S.A[r][j2] -= l * u2;
+      }
+      asm volatile("bar.sync 1, %0;" ::"r"(32 * nw) : "memory");
     }
-    __syncthreads();
-    const double inv = 1.0 / S.A[k][k];
-    const int rows = P - k - 1;
-    for (int e = threadIdx.x; e < rows * (P - k); e += blockDim.x) {
-      const int i = k + 1 + e / (P - k), j = k + e % (P - k);
-      const double l = S.A[i][k] * inv;
-      if (j > k) S.A[i][j] -= l * S.A[k][j];
-    }
-    __syncthreads();
-    for (int i = k + 1 + threadIdx.x; i < P; i += blockDim.x) {
-      const double l = S.A[i][k] * inv;
-      S.rhs[i] -= l * S.rhs[k];
-      S.A[i][k] = l;
-    }
-    __syncthreads();
-  }
-  if (!ok) return false;
-  if (threadIdx.x == 0) {
-    for (int i = P - 1; i >= 0; --i) {
-      double s = S.rhs[i];
-      for (int j = i + 1; j < P; ++j) s -= S.A[i][j] * S.gam[j];
-      S.gam[i] = s / S.A[i][i];
+    if (warp == 0) {
+      if (lane < P) S.perm[lane] = p0;
+      if (lane + 32 < P) S.perm[lane + 32] = p1;
+      if (lane == 0) S.lu_ok = ok;
+      __syncwarp();
+      // back substitution, each row's terms in order: one thread's chain
+      if (ok && lane == 0) {
+        for (int i = P - 1; i >= 0; --i) {
+          const double* row = S.A[S.perm[i]];
+          double s = row[P];
+          const double diag = row[i];
+#pragma unroll 4
+          for (int j = i + 1; j < P; ++j) s -= row[j] * S.gam[j];
+          S.gam[i] = s / diag;
+        }
+      }
     }
   }
   __syncthreads();
-  return true;
+  return S.lu_ok != 0;
 }
 
 // CL CTAs per environment (a cluster, launched with that cluster size): they
-// run the same step redundantly, except the wake induction, which they share
-// (wake_induction); rank 0 alone writes the environment's global state, and a
+// share the wake induction (wake_induction), the AIC's rows and the loads'
+// points, through distributed shared memory, and run the rest of the step
+// redundantly; rank 0 alone writes the environment's global state, and a
 // cluster barrier at the start of every step makes its particle writes of
 // the last step visible to the others.
 template <bool F32, int CL>
@@ -507,7 +652,7 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
   int has_prev = st.has_prev[env];
   int head = st.phead[env], count = st.pcount[env];
   __syncthreads();
-  bool ok = true;
+  bool ok = true, first = true;
   for (; step < last && ok; ++step) {
     if constexpr (CL > 1) {
       __threadfence();
@@ -517,26 +662,44 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
     if (ref) {
       build_lattice_reference(S, p);
     } else {
-      deform(S, p);
+      // the last step's deform already holds this step's vertices
+      if (first) deform(S, p);
+      first = false;
       __syncthreads();
       build_lattice(S, p);
     }
-    for (int k = threadIdx.x; k < R * p.ns; k += blockDim.x) {
+    // the wake's rings on the threads after the lattice's warps
+    const int t0 = (P + 31) & ~31;
+    for (int k = threadIdx.x >= t0 ? threadIdx.x - t0 : threadIdx.x + blockDim.x - t0;
+         k < R * p.ns; k += blockDim.x) {
       const int r = k / p.ns, j = k % p.ns;
-      seg::prep_vortex<FVX_LEGS_RING, true>(S.wake[k], S.W[r + 1][j + 1], S.W[r][j + 1], S.W[r][j],
-                                      S.W[r + 1][j], S.wgam[r][j], p.rc0, S.wage[r], p.nu);
+      if constexpr (F32)
+        prep_ring_f32(S.wakef[k], S.W[r + 1][j + 1], S.W[r][j + 1], S.W[r][j], S.W[r + 1][j],
+                      S.wgam[r][j], p.rc0, S.wage[r], p.nu);
+      else
+        seg::prep_vortex<FVX_LEGS_RING, true>(S.wake[k], S.W[r + 1][j + 1], S.W[r][j + 1],
+                                              S.W[r][j], S.W[r + 1][j], S.wgam[r][j], p.rc0,
+                                              S.wage[r], p.nu);
     }
     __syncthreads();
     // 2. wake + particles at collocation points and bound-leg centres
     wake_induction<F32, CL>(S, p, st, env, R, head, count, crank);
-    // 3. AIC (written after the induction, whose scratch overlaps it) and rhs
-    for (int e = threadIdx.x; e < P * P; e += blockDim.x) {
-      const int i = e / P, j = e % P;
+    // 3. AIC (written after the induction, whose scratch overlaps it) and rhs;
+    // each CTA of a cluster takes a share of the rows and stores them in all
+    const int rows = (P + CL - 1) / CL, row0 = crank * rows, row1 = min(P, row0 + rows);
+    for (int e = threadIdx.x; e < (row1 - row0) * P; e += blockDim.x) {
+      const int i = row0 + e / P, j = e % P;
       double vx = 0.0, vy = 0.0, vz = 0.0;
       int cnt[4] = {0, 0, 0, 0};
-      seg::vortex_velocity_general<FVX_LEGS_RING, true>(S.bound[j], S.colloc[i][0], S.colloc[i][1],
-                                          S.colloc[i][2], vx, vy, vz, cnt);
-      S.A[i][j] = vx * S.normal[i][0] + vy * S.normal[i][1] + vz * S.normal[i][2];
+      seg::vortex_velocity_general<FVX_LEGS_RING, true>(S.bound[j], S.colloc[i][0],
+                                                        S.colloc[i][1], S.colloc[i][2], vx, vy,
+                                                        vz, cnt);
+      const double w = vx * S.normal[i][0] + vy * S.normal[i][1] + vz * S.normal[i][2];
+      S.A[i][j] = w;
+      if constexpr (CL > 1) {
+        for (int r = 0; r < CL; ++r)
+          if (r != crank) *cooperative_groups::this_cluster().map_shared_rank(&S.A[i][j], r) = w;
+      }
     }
     for (int i = threadIdx.x; i < P; i += blockDim.x) {
       const double wx = (ux - S.vcol[i][0]) + S.Vind[i][0];
@@ -544,7 +707,10 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
       const double wz = (uz - S.vcol[i][2]) + S.Vind[i][2];
       S.rhs[i] = -(wx * S.normal[i][0] + wy * S.normal[i][1] + wz * S.normal[i][2]);
     }
-    __syncthreads();
+    if constexpr (CL > 1)
+      cooperative_groups::this_cluster().sync();  // all rows are in place
+    else
+      __syncthreads();
     // 4. strengths
     if (!lu_solve(S, P)) {
       ok = false;
@@ -555,12 +721,58 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
     __syncthreads();
     double* Fz = &S.A[0][0];     // P station-force z components (A is free now)
     double* arm = Fz + kMaxP;
+    // A pass forms the leg terms of up to kLegItems (point, ring) pairs side by
+    // side, then a thread per point and component adds them in ring and leg
+    // order; each CTA of a cluster takes the points of its AIC rows.
+    {
+      const int np = row1 - row0;
+      const int per = max(1, kLegItems / max(np, 1));  // rings per pass
+      double acc[2] = {0.0, 0.0};  // values 3 point + component: this thread's (at most two)
+      for (int jb = 0; jb < P; jb += per) {
+        const int nj = min(per, P - jb);
+        for (int e = threadIdx.x; e < np * nj; e += blockDim.x) {
+          const int k = row0 + e / nj, j = jb + e % nj;
+          double* o = S.legs + e * kLegStride;
+          seg::vortex_legs<FVX_LEGS_RING, true>(
+              S.bound[j], S.legc[k][0], S.legc[k][1], S.legc[k][2],
+              [&](int l, double c4, double r3x, double r3y, double r3z) {
+                o[4 * l] = c4;
+                o[4 * l + 1] = r3x;
+                o[4 * l + 2] = r3y;
+                o[4 * l + 3] = r3z;
+              },
+              [&](int l, int) { o[4 * l] = o[4 * l + 1] = o[4 * l + 2] = o[4 * l + 3] = 0.0; });
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const int v = threadIdx.x + m * blockDim.x;
+          if (v >= 3 * np) continue;
+          const double* o = S.legs + (v / 3) * nj * kLegStride;
+          for (int j = 0; j < nj; ++j, o += kLegStride)
+#pragma unroll
+            for (int l = 0; l < 4; ++l) acc[m] = fma(o[4 * l], o[4 * l + 1 + v % 3], acc[m]);
+        }
+        __syncthreads();
+      }
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int v = threadIdx.x + m * blockDim.x;
+        if (v >= 3 * np) continue;
+        double* o = &S.Vbound[row0][0] + v;
+        *o = acc[m];
+        if constexpr (CL > 1) {
+          for (int r = 0; r < CL; ++r)
+            if (r != crank) *cooperative_groups::this_cluster().map_shared_rank(o, r) = acc[m];
+        }
+      }
+      if constexpr (CL > 1)
+        cooperative_groups::this_cluster().sync();
+      else
+        __syncthreads();
+    }
     for (int k = threadIdx.x; k < P; k += blockDim.x) {
-      double vx = 0.0, vy = 0.0, vz = 0.0;
-      int cnt[4] = {0, 0, 0, 0};
-      for (int j = 0; j < P; ++j)
-        seg::vortex_velocity_general<FVX_LEGS_RING, true>(S.bound[j], S.legc[k][0], S.legc[k][1], S.legc[k][2],
-                                            vx, vy, vz, cnt);
+      const double vx = S.Vbound[k][0], vy = S.Vbound[k][1], vz = S.Vbound[k][2];
       const double Vx = (ux - S.vleg[k][0]) + (S.Vind[P + k][0] + vx);
       const double Vy = (uy - S.vleg[k][1]) + (S.Vind[P + k][1] + vy);
       const double Vz = (uz - S.vleg[k][2]) + (S.Vind[P + k][2] + vz);
@@ -579,32 +791,46 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
     __syncthreads();
     // the reference couples from step 1 to the step before the last
     const bool couple = !ref || (step >= 1 && step < p.n_steps[env] - 1);
-    // 6. station loads -> nodal forces (one thread, fixed order)
-    if (couple && threadIdx.x == 0) {
-      for (int k = 0; k < ndof; ++k) S.F[k] = 0.0;
-      for (int j = 0; j < p.ns; ++j) {
-        double lift = 0.0, torque = 0.0;
-        for (int i = 0; i < p.nc; ++i) lift += Fz[i * p.ns + j];
-        for (int i = 0; i < p.nc; ++i) torque += Fz[i * p.ns + j] * arm[i * p.ns + j];
-        const int n = p.station_node[j];
-        const double xi = p.station_xi[j];
-        S.F[3 * n] += lift * (1.0 - xi);
-        S.F[3 * (n + 1)] += lift * xi;
-        S.F[3 * n + 2] += torque * (1.0 - xi);
-        S.F[3 * (n + 1) + 2] += torque * xi;
-      }
+    // 6. station loads -> nodal forces: lift and torque per station, then each
+    // degree of freedom adds its stations' shares in station order
+    double* lift = arm + kMaxP;
+    double* torque = lift + kMaxNS;
+    if (couple && threadIdx.x < p.ns) {
+      const int j = threadIdx.x;
+      double lf = 0.0, tq = 0.0;
+      for (int i = 0; i < p.nc; ++i) lf += Fz[i * p.ns + j];
+      for (int i = 0; i < p.nc; ++i) tq += Fz[i * p.ns + j] * arm[i * p.ns + j];
+      lift[j] = lf;
+      torque[j] = tq;
     }
     __syncthreads();
+    for (int k = threadIdx.x; k < ndof && couple; k += blockDim.x) {
+      const int n = k / 3, c = k % 3;
+      double f = 0.0;
+      for (int j = 0; j < p.ns && c != 1; ++j) {
+        const double q = c == 0 ? lift[j] : torque[j], xi = p.station_xi[j];
+        if (p.station_node[j] == n) f += q * (1.0 - xi);
+        if (p.station_node[j] + 1 == n) f += q * xi;
+      }
+      S.F[k] = f;
+    }
     // 7. Newmark: F_eff = F + M (a0 d + a1 v + a2 a) + C (a3 d + a4 v + a5 a)
     const double b = p.beta, g = p.gamma;
     const double a0 = 1.0 / (b * dt * dt), a1 = 1.0 / (b * dt), a2 = 1.0 / (2.0 * b) - 1.0;
     const double a3 = g / (b * dt), a4 = g / b - 1.0, a5 = dt * (g / (2.0 * b) - 1.0);
+    double* xm = torque + kMaxNS;
+    double* xc = xm + kMaxDof;
+    for (int c = threadIdx.x; c < nf && couple; c += blockDim.x) {
+      const double dc = S.d[3 + c], vc = S.v[3 + c], ac = S.a[3 + c];
+      xm[c] = a0 * dc + a1 * vc + a2 * ac;
+      xc[c] = a3 * dc + a4 * vc + a5 * ac;
+    }
+    __syncthreads();
     for (int r = threadIdx.x; r < nf && couple; r += blockDim.x) {
       double fm = 0.0, fc = 0.0;
       for (int c = 0; c < nf; ++c) {
-        const double dc = S.d[3 + c], vc = S.v[3 + c], ac = S.a[3 + c];
-        fm += p.mr[r * nf + c] * (a0 * dc + a1 * vc + a2 * ac);
-        fc += p.cr[r * nf + c] * (a3 * dc + a4 * vc + a5 * ac);
+        fm += p.mr[r * nf + c] * xm[c];
+        fc += p.cr[r * nf + c] * xc[c];
       }
       S.feff[r] = S.F[3 + r] + fm + fc;
     }
@@ -676,52 +902,59 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
     if (threadIdx.x == 0) S.wage[0] = 0.0;
     ++R;
     __syncthreads();
-    // 9. rows >= n_keep -> particles (one thread appends in the reference order)
+    // 9. rows >= n_keep -> particles, appended in the reference's order (row,
+    // strip, edge): a lane per edge, its place by a count of the edges before
+    // it that convert.  Place t of this step goes to slot head + count + t of
+    // the ring buffer, full or not: when it is full that slot holds the oldest.
     if (R > p.n_keep) {
-      if (threadIdx.x == 0) {
-        for (int r = p.n_keep; r < R; ++r) {
-          for (int j = 0; j < p.ns; ++j) {
+      if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        const int edges = (R - p.n_keep) * p.ns * 4;
+        int added = 0;
+        for (int e0 = 0; e0 < edges; e0 += 32) {
+          const int e = e0 + lane;
+          const int r = p.n_keep + e / (4 * p.ns), j = (e / 4) % p.ns;
+          double a[3] = {}, bb[3] = {}, al[3] = {}, sg = 0.0;
+          bool take = false;
+          if (e < edges) {
             const double gr = S.wgam[r][j];
-            if (fabs(gr) < 1e-15) continue;
             const double* fl = S.W[r][j];
             const double* fr = S.W[r][j + 1];
             const double* bl = S.W[r + 1][j];
             const double* br = S.W[r + 1][j + 1];
-            auto dist = [](const double* x, const double* y) {
-              const double a = x[0] - y[0], b2 = x[1] - y[1], c = x[2] - y[2];
-              return sqrt(a * a + b2 * b2 + c * c);
-            };
-            const double sg =
-                1.3 * 0.25 * (dist(fl, fr) + dist(bl, fl) + dist(br, bl) + dist(fr, br));
-            const double* ends[4][2] = {{fr, fl}, {fl, bl}, {bl, br}, {br, fr}};
-            for (int e = 0; e < 4; ++e) {
-              const double* a = ends[e][0];
-              const double* bb = ends[e][1];
-              const double alx = gr * (bb[0] - a[0]), aly = gr * (bb[1] - a[1]),
-                           alz = gr * (bb[2] - a[2]);
-              if (!(alx * alx + aly * aly + alz * alz > 1e-30)) continue;
-              int q;
-              if (count < Pm) {
-                q = (head + count) % Pm;
-                ++count;
-              } else {
-                q = head;  // drop the oldest
-                head = (head + 1) % Pm;
-              }
-              if (writer) {
-                pp[3 * q] = 0.5 * (a[0] + bb[0]);
-                pp[3 * q + 1] = 0.5 * (a[1] + bb[1]);
-                pp[3 * q + 2] = 0.5 * (a[2] + bb[2]);
-                pa[3 * q] = alx;
-                pa[3 * q + 1] = aly;
-                pa[3 * q + 2] = alz;
-                ps[q] = sg;
-              }
+            const double* from = (e & 3) == 0 ? fr : ((e & 3) == 1 ? fl : ((e & 3) == 2 ? bl : br));
+            const double* to = (e & 3) == 0 ? fl : ((e & 3) == 1 ? bl : ((e & 3) == 2 ? br : fr));
+            for (int c = 0; c < 3; ++c) {
+              a[c] = from[c];
+              bb[c] = to[c];
+              al[c] = gr * (bb[c] - a[c]);
             }
+            take = !(fabs(gr) < 1e-15) && al[0] * al[0] + al[1] * al[1] + al[2] * al[2] > 1e-30;
+            auto dist = [](const double* x, const double* y) {
+              const double u = x[0] - y[0], v = x[1] - y[1], w = x[2] - y[2];
+              return sqrt(u * u + v * v + w * w);
+            };
+            sg = 1.3 * 0.25 * (dist(fl, fr) + dist(bl, fl) + dist(br, bl) + dist(fr, br));
           }
+          const unsigned m = __ballot_sync(0xffffffffu, take);
+          const int place = __popc(m & ((1u << lane) - 1u));
+          // (of two places in one slot, Pm apart, the later one stays)
+          if (take && writer && place + Pm >= __popc(m)) {
+            const int q = (head + (count + added + place) % Pm) % Pm;
+            for (int c = 0; c < 3; ++c) {
+              pp[3 * q + c] = 0.5 * (a[c] + bb[c]);
+              pa[3 * q + c] = al[c];
+            }
+            ps[q] = sg;
+          }
+          added += __popc(m);
+          __syncwarp();
         }
-        S.red[0] = static_cast<double>(head);
-        S.red[1] = static_cast<double>(count);
+        if (lane == 0) {
+          const int over = max(0, count + added - Pm);
+          S.red[0] = static_cast<double>((head + over) % Pm);
+          S.red[1] = static_cast<double>(count + added - over);
+        }
       }
       R = p.n_keep;
       __syncthreads();

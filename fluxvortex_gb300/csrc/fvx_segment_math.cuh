@@ -151,36 +151,44 @@ __device__ __forceinline__ void prep_vortex(VortexRec& R, const double* br, cons
   R.lo = fast ? max(kHiMin, far - kHiNear) : kHiMax;
 }
 
-// Velocity of one vortex (all legs) at point p; cnt[k] counts skips.  The
-// reference's own sequence of operations and tests, for the pairs that the
-// fast path leaves out.
-template <int LEGS, bool TOL>
-__device__ __forceinline__ void vortex_velocity_general(const VortexRec& R, double px, double py,
-                                                        double pz, double& vx, double& vy,
-                                                        double& vz, int cnt[4]) {
-  double dx[4], dy[4], dz[4], len[4];
+// The legs of one vortex at point p, in order, by the reference's own sequence
+// of operations: take(l, c4, r3) for a leg that contributes c4 r3, skip(l, k)
+// for one that skip test k leaves out.  The pairs that the fast path leaves
+// out take it, and callers that keep the reference's rounding.  The skip tests
+// are the reference's; where all distances are within the fast path's range
+// (no NaN among them) integer comparisons decide them as far as they can:
+// lengths and tolerances are not negative, so their words order them.
+template <int LEGS, bool TOL, typename Take, typename Skip>
+__device__ __forceinline__ void vortex_legs(const VortexRec& R, double px, double py, double pz,
+                                            Take take, Skip skip) {
+  double dx[4], dy[4], dz[4], sq[4], len[4];
+  int lo = 0x7fffffff, hi = 0;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     dx[c] = R.c[c][0] - px;
     dy[c] = R.c[c][1] - py;
     dz[c] = R.c[c][2] - pz;
-    len[c] = sqrt(dx[c] * dx[c] + dy[c] * dy[c] + dz[c] * dz[c]);
+    sq[c] = dx[c] * dx[c] + dy[c] * dy[c] + dz[c] * dz[c];
+    len[c] = sqrt(sq[c]);
+    lo = min(lo, __double2hiint(sq[c]));
+    hi = max(hi, __double2hiint(sq[c]));
   }
+  const bool in_range = lo >= kHiMin && hi < kHiMax;
   const int valid = R.valid;
 #pragma unroll
   for (int l = 0; l < Legs<LEGS>::n; ++l) {
     const int a = Legs<LEGS>::s(l), b = Legs<LEGS>::e(l);
     if (!((valid >> l) & 1)) {
-      cnt[0]++;
+      skip(l, 0);
       continue;
     }
     const double tol = TOL ? R.tol[l] : sqrt(R.r0sq[l]) * kTol;
-    if (len[a] < tol) {
-      cnt[1]++;
+    if (in_range ? __double_as_longlong(len[a]) < __double_as_longlong(tol) : len[a] < tol) {
+      skip(l, 1);
       continue;
     }
-    if (len[b] < tol) {
-      cnt[2]++;
+    if (in_range ? __double_as_longlong(len[b]) < __double_as_longlong(tol) : len[b] < tol) {
+      skip(l, 2);
       continue;
     }
     double r3x = dy[a] * dz[b] - dz[a] * dy[b];
@@ -188,17 +196,33 @@ __device__ __forceinline__ void vortex_velocity_general(const VortexRec& R, doub
     double r3z = dx[a] * dy[b] - dy[a] * dx[b];
     double r3_sq = r3x * r3x + r3y * r3y + r3z * r3z;
     double r1r2 = len[a] * len[b];
-    double thr = kTol * r1r2;
-    if (r3_sq < 2.0 * thr * thr && sqrt(r3_sq) < thr) {
-      cnt[3]++;
-      continue;
+    if (!in_range ||
+        __double2hiint(r3_sq) < __double2hiint(sq[a]) + (__double2hiint(sq[b]) + kHiLine)) {
+      const double thr = kTol * r1r2;
+      if (r3_sq < 2.0 * thr * thr && sqrt(r3_sq) < thr) {
+        skip(l, 3);
+        continue;
+      }
     }
     double c3 = dx[a] * dx[b] + dy[a] * dy[b] + dz[a] * dz[b];
     double c4 = R.c1 * (len[a] + len[b]) * (r1r2 - c3) / (r1r2 * (r3_sq + R.c2[l]));
-    vx += c4 * r3x;
-    vy += c4 * r3y;
-    vz += c4 * r3z;
+    take(l, c4, r3x, r3y, r3z);
   }
+}
+
+// Velocity of one vortex (all legs) at point p; cnt[k] counts skips.
+template <int LEGS, bool TOL>
+__device__ __forceinline__ void vortex_velocity_general(const VortexRec& R, double px, double py,
+                                                        double pz, double& vx, double& vy,
+                                                        double& vz, int cnt[4]) {
+  vortex_legs<LEGS, TOL>(
+      R, px, py, pz,
+      [&](int, double c4, double r3x, double r3y, double r3z) {
+        vx += c4 * r3x;
+        vy += c4 * r3y;
+        vz += c4 * r3z;
+      },
+      [&](int, int k) { cnt[k]++; });
 }
 
 template <int LEGS>
