@@ -17,6 +17,11 @@
 //   Taylor series of g(r)/r^3 (the reference's erf - c r exp form cancels
 //   there and is pure rounding noise at its r = 1e-12 self-pair clamp).
 //
+// FP64 sweeps (pairs_f64_kernel): the FP64 pipe bounds them, so the scalar core
+// of a pair (f, f'/r) is formed in three-float arithmetic on the FP32 pipe
+// (fvx_x3.cuh) and only the vector part stays in FP64; tiles with values outside
+// that arithmetic's range take the FP64 core (core_f64).
+//
 // Layout and tiling: a CTA owns 128 (FP64) or 256-512 (FP32, two or four per
 // thread) targets held in registers.  Source tiles of 128 particles (AoS pos, alpha,
 // sigma exactly as the caller stores them) are staged by 1-D TMA bulk copies
@@ -28,10 +33,10 @@
 // two-sum (hi, lo) pair per component.  When targets alone cannot fill the
 // SMs the source range is split over gridDim.y; partial sums go to scratch
 // and a second kernel adds them in fixed order.
-#include <type_traits>
-
 #include "fvx_common.cuh"
+#include "fvx_core_table.cuh"
 #include "fvx_pair_math.cuh"
+#include "fvx_x3.cuh"
 
 namespace fvx {
 namespace {
@@ -42,28 +47,25 @@ constexpr int kThreads = 128;
 constexpr int kSrcTile = 128;
 constexpr double kC = -0.07957747154594767;  // -1/(4 pi)
 
+template <int TILE>
 struct RawSrc {
-  double pos[kSrcTile * 3];
-  double alpha[kSrcTile * 3];
-  double sigma[kSrcTile];
+  double pos[TILE * 3];
+  double alpha[TILE * 3];
+  double sigma[TILE];
 };
 
-// Compute tile: two 4-vectors per source so that a thread fetches a source
-// with two 128-bit shared loads (FP32) and reuses it for all its targets.
-template <typename T>
-struct alignas(4 * sizeof(T)) Vec4 {
-  T x, y, z, w;
-};
-template <typename T>
+// Compute tile of the FP32 sweeps: two 4-vectors per source so that a thread
+// fetches a source with two 128-bit shared loads and reuses it for all its
+// targets.
 struct SrcTile {
-  Vec4<T> p[kSrcTile];  // x, y, z, sigma^2
-  Vec4<T> a[kSrcTile];  // C*alpha_x, C*alpha_y, C*alpha_z, k2
+  float4 p[kSrcTile];  // x, y, z, sigma^2
+  float4 a[kSrcTile];  // C*alpha_x, C*alpha_y, C*alpha_z, k2
 };
 
 // Targets per thread: more register blocking for the 3-component modes.
-template <int MODE, bool F32>
+template <int MODE>
 struct Blocking {
-  static constexpr int tpt = !F32 ? 1 : (ModeInfo<MODE>::ncomp <= 3 ? 4 : 2);
+  static constexpr int tpt = ModeInfo<MODE>::ncomp <= 3 ? 4 : 2;
 };
 
 struct PairArgs {
@@ -81,7 +83,8 @@ struct PairArgs {
   int use_tma;
 };
 
-__device__ void issue_src(const PairArgs& A, RawSrc& raw, int64_t j0, int cnt, uint64_t* bar) {
+template <int TILE>
+__device__ void issue_src(const PairArgs& A, RawSrc<TILE>& raw, int64_t j0, int cnt, uint64_t* bar) {
   BulkPlan pp = plan_bulk(A.pos, j0, cnt, 24, A.use_tma);
   BulkPlan pa = plan_bulk(A.alpha, j0, cnt, 24, A.use_tma);
   BulkPlan ps = plan_bulk(A.sigma, j0, cnt, 8, A.use_tma);
@@ -91,7 +94,8 @@ __device__ void issue_src(const PairArgs& A, RawSrc& raw, int64_t j0, int cnt, u
   if (ps.bulk_bytes) bulk_g2s(raw.sigma, A.sigma + j0, ps.bulk_bytes, bar);
 }
 
-__device__ void tail_src(const PairArgs& A, RawSrc& raw, int64_t j0, int cnt) {
+template <int TILE>
+__device__ void tail_src(const PairArgs& A, RawSrc<TILE>& raw, int64_t j0, int cnt) {
   BulkPlan p = plan_bulk(A.pos, j0, cnt, 24, A.use_tma);
   if (p.tail_bytes) plain_copy8(raw.pos, A.pos + 3 * j0, p.bulk_bytes, p.tail_bytes);
   p = plan_bulk(A.alpha, j0, cnt, 24, A.use_tma);
@@ -109,26 +113,21 @@ __device__ __forceinline__ void two_sum_fold(T& hi, T& lo, T p) {
   lo += err;
 }
 
-template <int MODE, int KERNEL, bool F32>
-__global__ void __launch_bounds__(kThreads) pairs_kernel(PairArgs A) {
-  using T = typename std::conditional<F32, float, double>::type;
-  constexpr int TPT = Blocking<MODE, F32>::tpt;  // targets per thread
+template <int MODE, int KERNEL>
+__global__ void __launch_bounds__(kThreads) pairs_f32_kernel(PairArgs A) {
+  using T = float;
+  constexpr int TPT = Blocking<MODE>::tpt;  // targets per thread
   constexpr int NC = ModeInfo<MODE>::ncomp;
   constexpr bool NEED_FPR = ModeInfo<MODE>::need_fpr;
   constexpr bool NEED_TG = ModeInfo<MODE>::need_tg;
 
-  __shared__ __align__(128) RawSrc raw[2];
-  __shared__ __align__(16) SrcTile<T> tile;
+  __shared__ __align__(128) RawSrc<kSrcTile> raw[2];
+  __shared__ __align__(16) SrcTile tile;
   __shared__ __align__(8) uint64_t bar[2];
 
   const int64_t base = static_cast<int64_t>(blockIdx.x) * (kThreads * TPT);
-  // Re-centring origin: the CTA's first target (FP32 only).
-  double ox = 0.0, oy = 0.0, oz = 0.0;
-  if (F32) {
-    ox = A.tgt[3 * base + 0];
-    oy = A.tgt[3 * base + 1];
-    oz = A.tgt[3 * base + 2];
-  }
+  // Re-centring origin: the CTA's first target.
+  const double ox = A.tgt[3 * base + 0], oy = A.tgt[3 * base + 1], oz = A.tgt[3 * base + 2];
   T tx[TPT], ty[TPT], tz[TPT], gx[TPT], gy[TPT], gz[TPT];
   bool act[TPT];
 #pragma unroll
@@ -195,7 +194,7 @@ __global__ void __launch_bounds__(kThreads) pairs_kernel(PairArgs A) {
     __syncthreads();
     for (int k = threadIdx.x; k < n; k += kThreads) {
       const double sg = raw[buf].sigma[k];
-      Vec4<T> pv, av;
+      float4 pv, av;
       pv.x = static_cast<T>(raw[buf].pos[3 * k + 0] - ox);
       pv.y = static_cast<T>(raw[buf].pos[3 * k + 1] - oy);
       pv.z = static_cast<T>(raw[buf].pos[3 * k + 2] - oz);
@@ -215,8 +214,8 @@ __global__ void __launch_bounds__(kThreads) pairs_kernel(PairArgs A) {
       for (int c = 0; c < NC; ++c) part[j][c] = T(0);
 #pragma unroll 2
     for (int k = 0; k < n; ++k) {
-      const Vec4<T> pv = tile.p[k];
-      const Vec4<T> av = tile.a[k];
+      const float4 pv = tile.p[k];
+      const float4 av = tile.a[k];
       const T sx = pv.x, sy = pv.y, sz = pv.z, s2 = pv.w;
       const T ax = av.x, ay = av.y, az = av.z, k2 = av.w;
 #pragma unroll
@@ -224,22 +223,14 @@ __global__ void __launch_bounds__(kThreads) pairs_kernel(PairArgs A) {
         const T dx = tx[j] - sx, dy = ty[j] - sy, dz = tz[j] - sz;
         const T r2 = dx * dx + dy * dy + dz * dz;
         T f, fpr = T(0);
-        if constexpr (F32)
-          core_f32<KERNEL, NEED_FPR>(r2, s2, k2, f, fpr);
-        else
-          core_f64<KERNEL, NEED_FPR>(r2, s2, k2, f, fpr);
+        core_f32<KERNEL, NEED_FPR>(r2, s2, k2, f, fpr);
         accumulate<MODE, T>(part[j], dx, dy, dz, r2, ax, ay, az, f, fpr, gx[j], gy[j], gz[j]);
       }
     }
 #pragma unroll
     for (int j = 0; j < TPT; ++j)
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if constexpr (F32)
-          two_sum_fold(hi[j][c], lo[j][c], part[j][c]);
-        else
-          hi[j][c] += part[j][c];
-      }
+      for (int c = 0; c < NC; ++c) two_sum_fold(hi[j][c], lo[j][c], part[j][c]);
     __syncthreads();
   }
   if (!ok) {
@@ -266,6 +257,317 @@ __global__ void __launch_bounds__(kThreads) pairs_kernel(PairArgs A) {
 #pragma unroll
       for (int c = NA; c < NC; ++c) A.out_b[i * (NC - NA) + (c - NA)] = v[c];
     }
+  }
+}
+
+// ---- FP64 sweeps ------------------------------------------------------------------
+// A staged source: scaled strength in FP64, position and core constants as three
+// floats each (96 bytes: six 16-byte broadcast loads).
+struct alignas(16) SrcX3 {
+  double a[3];
+  x3::F3 x[3];
+  x3::F3 s2, k, k5;  // x3::Core
+};
+static_assert(sizeof(SrcX3) == 96, "a source is six 16-byte words");
+
+// Sources per tile: short, so that two CTAs and their copies of the Gaussian
+// core's table (88 KB) fit an SM.
+constexpr int kSrc64 = 64;
+
+// Dynamic shared memory: raw tiles, compute tile, barriers, and for the
+// Gaussian core its polynomials ([interval][F, G or F alone][20]).
+struct F64Smem {
+  RawSrc<kSrc64> raw[2];
+  SrcX3 tile[kSrc64];
+  uint64_t bar[2];
+  alignas(16) float table[];
+};
+
+__device__ const __align__(16) float g_core_table[] = {FVX_CORE_TABLE};
+constexpr int kTableRows = x3::kCoreRows + x3::kFarRows;
+constexpr int kTableFloats = kTableRows * x3::kRowFloats;  // of F, and of G
+
+// coordinates up to 2^13, cores of 2^-22 .. 2^13 (high words; NaN and infinity
+// are beyond): the three-float arithmetic's range
+__device__ __forceinline__ bool x3_coord(double x) {
+  return (__double2hiint(x) & 0x7fffffff) < ((1023 + 13) << 20);
+}
+__device__ __forceinline__ bool x3_core(double s) {
+  const int h = __double2hiint(s);
+  return h >= ((1023 - 22) << 20) && h < ((1023 + 13) << 20);
+}
+
+// Sums of one pair in FP64 given f and f'/r (and, for the vorticity, iso = f'/r
+// r^2 + 2 f): accumulate() with every product fused into its sum.  The
+// Jacobian's antisymmetric part goes to acc[9..11] = sum of f a and is put in
+// place per tile (fold_tile).
+template <int MODE>
+struct F64Acc {
+  static constexpr int n = MODE == FVX_PAIR_JACOBIAN ? 12 : ModeInfo<MODE>::ncomp;
+};
+template <int MODE>
+__device__ __forceinline__ void accumulate_f64(double* acc, double dx, double dy, double dz,
+                                               double ax, double ay, double az, double f,
+                                               double fpr, double iso, double gx, double gy,
+                                               double gz) {
+  auto cross = [&](double* o, double vx, double vy, double vz) {
+    o[0] = fma(-vz, ay, fma(vy, az, o[0]));
+    o[1] = fma(-vx, az, fma(vz, ax, o[1]));
+    o[2] = fma(-vy, ax, fma(vx, ay, o[2]));
+  };
+  if (MODE == FVX_PAIR_VELOCITY || MODE == FVX_PAIR_VELOCITY_STRETCH)
+    cross(acc, f * dx, f * dy, f * dz);
+  if (MODE == FVX_PAIR_STRETCH || MODE == FVX_PAIR_VELOCITY_STRETCH) {
+    const double w = fpr * fma(dz, gz, fma(dy, gy, dx * gx));
+    cross(acc + (MODE == FVX_PAIR_STRETCH ? 0 : 3), fma(w, dx, f * gx), fma(w, dy, f * gy),
+          fma(w, dz, f * gz));
+  }
+  if (MODE == FVX_PAIR_JACOBIAN) {
+    const double px = fpr * fma(dy, az, -(dz * ay));
+    const double py = fpr * fma(dz, ax, -(dx * az));
+    const double pz = fpr * fma(dx, ay, -(dy * ax));
+    acc[0] = fma(px, dx, acc[0]);
+    acc[1] = fma(px, dy, acc[1]);
+    acc[2] = fma(px, dz, acc[2]);
+    acc[3] = fma(py, dx, acc[3]);
+    acc[4] = fma(py, dy, acc[4]);
+    acc[5] = fma(py, dz, acc[5]);
+    acc[6] = fma(pz, dx, acc[6]);
+    acc[7] = fma(pz, dy, acc[7]);
+    acc[8] = fma(pz, dz, acc[8]);
+    acc[9] = fma(f, ax, acc[9]);
+    acc[10] = fma(f, ay, acc[10]);
+    acc[11] = fma(f, az, acc[11]);
+  }
+  if (MODE == FVX_PAIR_VORTICITY) {
+    const double s = fpr * fma(dz, az, fma(dy, ay, dx * ax));
+    acc[0] = fma(-ax, iso, fma(dx, s, acc[0]));
+    acc[1] = fma(-ay, iso, fma(dy, s, acc[1]));
+    acc[2] = fma(-az, iso, fma(dz, s, acc[2]));
+  }
+}
+template <int MODE>
+__device__ __forceinline__ void fold_tile(double* sum, double* part) {
+  if (MODE == FVX_PAIR_JACOBIAN) {
+    part[1] += part[11];
+    part[2] -= part[10];
+    part[3] -= part[11];
+    part[5] += part[9];
+    part[6] += part[10];
+    part[7] -= part[9];
+  }
+#pragma unroll
+  for (int c = 0; c < ModeInfo<MODE>::ncomp; ++c) sum[c] += part[c];
+}
+
+// One target per thread and slice.  The FP64 pipe and the FP32 issue bound it
+// about alike: 9 (velocity), 16 (stretching), 21 (gradient), 10 (vorticity) FP64
+// operations per pair, the offset being converted from its three floats, against
+// 31, 40, 55 and 43 with the Winckelmans core in FP64 and 100 more with the
+// Gaussian one; and the 450 to 850 FP32 operations of the scalar core beside
+// them.  Velocity at 384 points of 131,071 particles 2.70 -> 0.94 ms (54e9
+// pairs/s); gradient of 7,001 particles at themselves, Gaussian core, 13.9 ->
+// 2.15 ms; the field step of 3,001 (three velocity, three stretching and a
+// vorticity sweep, Gaussian) 15.5 -> 2.3 ms.
+// Two slices of 128 threads share a CTA's targets, one taking the even sources,
+// the other the odd ones, and its table.  (One: 1,392 us for 384 targets x 131,071
+// sources with a CTA per SM, two: 1,017; four leave 64 registers a thread, and
+// the stretching sums then spill: 336 us against 150 for 2,049 particles.)
+constexpr int kSlices = 2;
+
+template <int MODE, int KERNEL>
+size_t f64_smem_bytes() {
+  const size_t table = KERNEL == FVX_KERNEL_GAUSSIANERF
+                           ? sizeof(float) * kTableFloats * (ModeInfo<MODE>::need_fpr ? 2 : 1)
+                           : 0;
+  const size_t tiles = sizeof(F64Smem) + table;
+  const size_t sums = sizeof(double) * (kSlices - 1) * kThreads * ModeInfo<MODE>::ncomp;
+  return tiles > sums ? tiles : sums;
+}
+
+template <int MODE, int KERNEL>
+__global__ void __launch_bounds__(kSlices* kThreads) pairs_f64_kernel(PairArgs A) {
+  constexpr int NC = ModeInfo<MODE>::ncomp;
+  constexpr bool FPR = ModeInfo<MODE>::need_fpr;
+  constexpr bool ISO = MODE == FVX_PAIR_VORTICITY;
+  constexpr bool GAUSS = KERNEL == FVX_KERNEL_GAUSSIANERF;
+  constexpr int kParts = FPR ? 2 : 1;  // polynomials staged per interval
+
+  extern __shared__ __align__(128) unsigned char f64_smem[];
+  F64Smem& S = *reinterpret_cast<F64Smem*>(f64_smem);
+
+  constexpr int kRun = 32;
+  constexpr int kAll = kSlices * kThreads;
+  const int slice = threadIdx.x / kThreads, lt = threadIdx.x % kThreads;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + lt;
+  const bool act = i < A.n_tgt;
+  double tx = 0, ty = 0, tz = 0, gx = 0, gy = 0, gz = 0;
+  if (act) {
+    tx = A.tgt[3 * i + 0];
+    ty = A.tgt[3 * i + 1];
+    tz = A.tgt[3 * i + 2];
+    if (ModeInfo<MODE>::need_tg) {
+      gx = A.tgt_gamma[3 * i + 0];
+      gy = A.tgt_gamma[3 * i + 1];
+      gz = A.tgt_gamma[3 * i + 2];
+    }
+  }
+  const bool tgt_ok = x3_coord(tx) && x3_coord(ty) && x3_coord(tz);
+  const x3::F3 px = x3::split(tx), py = x3::split(ty), pz = x3::split(tz);
+
+  const int64_t jb = static_cast<int64_t>(blockIdx.y) * A.chunk;
+  const int64_t je = min(jb + A.chunk, A.n_src);
+  const int ntiles = jb < je ? static_cast<int>((je - jb + kSrc64 - 1) / kSrc64) : 0;
+
+  if (threadIdx.x == 0) {
+    mbar_init(&S.bar[0], 1);
+    mbar_init(&S.bar[1], 1);
+    fence_mbar_init();
+  }
+  if constexpr (GAUSS) {
+    for (int e = threadIdx.x; e < kTableRows * kParts * (x3::kRowFloats / 4); e += kAll) {
+      const int row = e / (x3::kRowFloats / 4), q = e % (x3::kRowFloats / 4);
+      reinterpret_cast<float4*>(S.table)[e] = *reinterpret_cast<const float4*>(
+          g_core_table + (row * 2 / kParts) * x3::kRowFloats + 4 * q);
+    }
+  }
+  __syncthreads();
+
+  double sum[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) sum[c] = 0.0;
+
+  uint32_t phase[2] = {0u, 0u};
+  bool ok = true;
+  if (ntiles > 0 && threadIdx.x == 0)
+    issue_src(A, S.raw[0], jb, static_cast<int>(min64(kSrc64, je - jb)), &S.bar[0]);
+  int t = 0;
+  for (; t < ntiles; ++t) {
+    const int buf = t & 1;
+    const int64_t j0 = jb + static_cast<int64_t>(t) * kSrc64;
+    const int n = static_cast<int>(min64(kSrc64, je - j0));
+    if (t + 1 < ntiles && threadIdx.x == 0) {
+      const int64_t j1 = j0 + kSrc64;
+      issue_src(A, S.raw[buf ^ 1], j1, static_cast<int>(min64(kSrc64, je - j1)),
+                &S.bar[buf ^ 1]);
+    }
+    const bool got = mbar_wait(&S.bar[buf], phase[buf]);
+    if (!__syncthreads_and(got)) {
+      ok = false;
+      break;
+    }
+    phase[buf] ^= 1u;
+    RawSrc<kSrc64>& raw = S.raw[buf];
+    tail_src(A, raw, j0, n);
+    __syncthreads();
+    bool in_range = tgt_ok;
+    for (int k = threadIdx.x; k < n; k += kAll) {
+      const double sg = raw.sigma[k];
+      SrcX3 v = {};
+      in_range = in_range && x3_core(sg);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double p = raw.pos[3 * k + c];
+        v.a[c] = kC * raw.alpha[3 * k + c];
+        v.x[c] = x3::split(p);
+        in_range = in_range && x3_coord(p);
+      }
+      const x3::Core core = GAUSS ? x3::gaussian_core(sg) : x3::winckelmans_core(sg);
+      v.s2 = core.s2;
+      v.k = core.k;
+      v.k5 = core.k5;
+      S.tile[k] = v;
+    }
+    // sums of kRun sources at a time join the thread's: short partial sums
+    // round less than the whole tile's did
+    if (__syncthreads_and(in_range)) {
+#pragma unroll 1
+      for (int k0 = slice; k0 < n; k0 += kRun * kSlices) {
+        double part[F64Acc<MODE>::n] = {};
+        const int k1 = min(n, k0 + kRun * kSlices);
+#pragma unroll 1
+        for (int k = k0; k < k1; k += kSlices) {
+          const SrcX3& s = S.tile[k];
+          const x3::F3 x = x3::diff(px, s.x[0]), y = x3::diff(py, s.x[1]), z = x3::diff(pz, s.x[2]);
+          const x3::Core core{s.s2, s.k, s.k5};
+          x3::F3 f, fpr = {}, iso = {};
+          if constexpr (GAUSS)
+            x3::gaussian<FPR, ISO>(x, y, z, core, x3::kCoreEnd, x3::kCoreRows,
+                                   [&](int row, int part_) {
+                                     x3::Row r;
+                                     const float4* q = reinterpret_cast<const float4*>(
+                                         S.table + (row * kParts + part_) * x3::kRowFloats);
+  #pragma unroll
+                                     for (int w = 0; w < x3::kRowFloats / 4; ++w) {
+                                       const float4 v4 = q[w];
+                                       r.c[4 * w] = v4.x;
+                                       r.c[4 * w + 1] = v4.y;
+                                       r.c[4 * w + 2] = v4.z;
+                                       r.c[4 * w + 3] = v4.w;
+                                     }
+                                     return r;
+                                   },
+                                   f, fpr, iso);
+          else
+            x3::winckelmans<FPR, ISO>(x, y, z, core, f, fpr, iso);
+          accumulate_f64<MODE>(part, x3::to_double(x), x3::to_double(y), x3::to_double(z), s.a[0],
+                               s.a[1], s.a[2], x3::to_double(f), FPR ? x3::to_double(fpr) : 0.0,
+                               ISO ? x3::to_double(iso) : 0.0, gx, gy, gz);
+        }
+        fold_tile<MODE>(sum, part);
+      }
+    } else {
+      // the same sums with the core in FP64
+#pragma unroll 1
+      for (int k0 = slice; k0 < n; k0 += kRun * kSlices) {
+        double part[F64Acc<MODE>::n] = {};
+        const int k1 = min(n, k0 + kRun * kSlices);
+#pragma unroll 1
+        for (int k = k0; k < k1; k += kSlices) {
+          const double sg = raw.sigma[k];
+          const double dx = tx - raw.pos[3 * k], dy = ty - raw.pos[3 * k + 1],
+                       dz = tz - raw.pos[3 * k + 2];
+          const double r2 = dx * dx + dy * dy + dz * dz;
+          double f, fpr = 0.0;
+          core_f64<KERNEL, FPR>(r2, sg * sg, GAUSS ? 1.0 / sg : 2.5 * sg * sg, f, fpr);
+          accumulate_f64<MODE>(part, dx, dy, dz, kC * raw.alpha[3 * k], kC * raw.alpha[3 * k + 1],
+                               kC * raw.alpha[3 * k + 2], f, fpr, fpr * r2 + (f + f), gx, gy, gz);
+        }
+        fold_tile<MODE>(sum, part);
+      }
+    }
+    __syncthreads();
+  }
+  if (!ok) {
+    flag_status(kStatusTimeout);
+    if (threadIdx.x == 0 && t + 1 < ntiles) mbar_wait(&S.bar[(t + 1) & 1], phase[(t + 1) & 1]);
+    return;
+  }
+  {
+    // the slices' sums, in slice order (tiles, barriers and table are done with)
+    double* q = reinterpret_cast<double*>(f64_smem);
+    if (slice > 0) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) q[((slice - 1) * NC + c) * kThreads + lt] = sum[c];
+    }
+    __syncthreads();
+    if (slice > 0) return;
+#pragma unroll
+    for (int s = 0; s < kSlices - 1; ++s)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) sum[c] += q[(s * NC + c) * kThreads + lt];
+  }
+  if (!act) return;
+  if (gridDim.y > 1) {
+    double* o = A.partial + (static_cast<int64_t>(blockIdx.y) * A.n_tgt + i) * NC;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) o[c] = sum[c];
+  } else {
+    constexpr int NA = ModeInfo<MODE>::na;
+#pragma unroll
+    for (int c = 0; c < NA; ++c) A.out_a[i * NA + c] = sum[c];
+#pragma unroll
+    for (int c = NA; c < NC; ++c) A.out_b[i * (NC - NA) + (c - NA)] = sum[c];
   }
 }
 
@@ -315,15 +617,13 @@ int targets_per_cta(int mode, int precision) {
   return kThreads * (mode_ncomp(mode) <= 3 ? 4 : 2);
 }
 
-int pair_splits(int mode, int precision, int64_t n_tgt, int64_t n_src, int64_t* chunk) {
-  const int per_cta = targets_per_cta(mode, precision);
-  const int64_t gx = (n_tgt + per_cta - 1) / per_cta;
-  // six resident CTAs per SM (80 registers x 128 threads): few targets
-  // (the panel points against every particle) split the sources that far
+// Splits of the source range for six resident CTAs per SM (80 registers x 128
+// threads), of at least two source tiles: few targets (the panel points against
+// every particle) split the sources that far.
+int splits_f32(int64_t gx, int64_t n_src, int64_t* chunk) {
   const int64_t want = 6LL * device_sm_count();
   int64_t s = gx >= want ? 1 : (want + gx - 1) / gx;
-  // keep at least two source tiles per split
-  int64_t maxs = (n_src + 2 * kSrcTile - 1) / (2 * kSrcTile);
+  const int64_t maxs = (n_src + 2 * kSrcTile - 1) / (2 * kSrcTile);
   if (s > maxs) s = maxs;
   if (s < 1) s = 1;
   int64_t c = (n_src + s - 1) / s;
@@ -333,12 +633,55 @@ int pair_splits(int mode, int precision, int64_t n_tgt, int64_t n_src, int64_t* 
   return static_cast<int>(s);
 }
 
+// An FP64 sweep takes as long as the SM with the most CTAs: `rounds` CTAs of
+// `chunk` sources each and a prologue that costs as much as kPrologue of them (the
+// first tile's latency, the Gaussian core's table), and an eighth longer where
+// the SM has only one CTA's warps to overlap (less with more: 1,017, 955 and 916 us
+// with 1, 4 .. 8 and 8 .. 16 rounds for 384 targets x 131,071 sources).  The
+// number of rounds, up to 24, that makes the least of that: one for 240 targets
+// x 2,001 sources (24 us; 28 with 4, 35 with 8), 3 for 2,049 x 2,049.
+int splits_f64(int64_t gx, int64_t n_src, int64_t* chunk) {
+  constexpr int64_t kPrologue = 4;
+  const int64_t sms = device_sm_count();
+  int64_t best = -1, best_c = n_src;
+  for (int64_t rounds = 1; rounds <= 24; ++rounds) {
+    int64_t s = rounds * sms / gx;
+    if (s < 1) continue;
+    if (s > n_src) s = n_src;
+    int64_t c = (n_src + s - 1) / s;
+    c = (c + 1) & ~int64_t(1);
+    const int64_t per_sm = (gx * ((n_src + c - 1) / c) + sms - 1) / sms;
+    const int64_t cost = (per_sm * 8 + 1) * (c + kPrologue);
+    if (best < 0 || cost < best) {
+      best = cost;
+      best_c = c;
+    }
+  }
+  *chunk = best_c;
+  return static_cast<int>((n_src + best_c - 1) / best_c);
+}
+
+// coarse: the FP32 rule for FP64 too, for a caller whose scratch holds no more
+int pair_splits(int mode, int precision, int64_t n_tgt, int64_t n_src, int64_t* chunk,
+                bool coarse = false) {
+  const int per_cta = targets_per_cta(mode, precision);
+  const int64_t gx = (n_tgt + per_cta - 1) / per_cta;
+  return precision == FVX_PREC_F32C || coarse ? splits_f32(gx, n_src, chunk)
+                                              : splits_f64(gx, n_src, chunk);
+}
+
 template <int MODE, int KERNEL>
 void launch_mode(int precision, dim3 grid, cudaStream_t stream, const PairArgs& A) {
-  if (precision == FVX_PREC_F32C)
-    pairs_kernel<MODE, KERNEL, true><<<grid, kThreads, 0, stream>>>(A);
-  else
-    pairs_kernel<MODE, KERNEL, false><<<grid, kThreads, 0, stream>>>(A);
+  if (precision == FVX_PREC_F32C) {
+    pairs_f32_kernel<MODE, KERNEL><<<grid, kThreads, 0, stream>>>(A);
+    return;
+  }
+  const size_t smem = f64_smem_bytes<MODE, KERNEL>();
+  // (each call: the attribute is the current device's; a failure shows at the launch)
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(pairs_f64_kernel<MODE, KERNEL>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  pairs_f64_kernel<MODE, KERNEL><<<grid, kSlices * kThreads, smem, stream>>>(A);
 }
 
 template <int KERNEL>
@@ -397,11 +740,15 @@ int particle_pairs_launch(int mode, int kernel, int precision, const double* tgt
   }
   FVX_ARG_CHECK(pos && alpha && sigma, "null source array");
   int64_t chunk = 0;
-  const int splits = pair_splits(mode, precision, n_tgt, n_src, &chunk);
-  const size_t need = splits > 1 ? sizeof(double) * static_cast<size_t>(nc) * n_tgt * splits : 0;
-  if (need > 0 && (scratch == nullptr || scratch_bytes < need)) {
-    set_last_error("particle_pairs needs %zu scratch bytes, got %zu", need, scratch_bytes);
-    return FVX_ERR_SCRATCH;
+  int splits = pair_splits(mode, precision, n_tgt, n_src, &chunk);
+  const size_t row = sizeof(double) * static_cast<size_t>(nc) * n_tgt;
+  if (splits > 1 && (scratch == nullptr || scratch_bytes < row * splits)) {
+    const size_t need = row * splits;
+    splits = pair_splits(mode, precision, n_tgt, n_src, &chunk, true);
+    if (splits > 1 && (scratch == nullptr || scratch_bytes < row * splits)) {
+      set_last_error("particle_pairs needs %zu scratch bytes, got %zu", need, scratch_bytes);
+      return FVX_ERR_SCRATCH;
+    }
   }
   PairArgs A;
   A.tgt = tgt;
