@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(kSlices* kThreads) pairs_f64_kernel(PairArgs A
     }
   }
   const bool tgt_ok = x3_coord(tx) && x3_coord(ty) && x3_coord(tz);
-  const x3::F3 px = x3::split(tx), py = x3::split(ty), pz = x3::split(tz);
+  const x3::F3 px = x3::split_fast(tx), py = x3::split_fast(ty), pz = x3::split_fast(tz);
 
   const int64_t jb = static_cast<int64_t>(blockIdx.y) * A.chunk;
   const int64_t je = min(jb + A.chunk, A.n_src);
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(kSlices* kThreads) pairs_f64_kernel(PairArgs A
       for (int c = 0; c < 3; ++c) {
         const double p = raw.pos[3 * k + c];
         v.a[c] = kC * raw.alpha[3 * k + c];
-        v.x[c] = x3::split(p);
+        v.x[c] = x3::split_fast(p);
         in_range = in_range && x3_coord(p);
       }
       const x3::Core core = GAUSS ? x3::gaussian_core(sg) : x3::winckelmans_core(sg);

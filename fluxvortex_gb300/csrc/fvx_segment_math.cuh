@@ -21,10 +21,12 @@
 //   * every skip test is first a comparison of the high words, as integers,
 //     with a threshold on the safe side; only a pair inside that margin takes
 //     the tests themselves.
-// About 140 FP64 operations per ring and point against about 300; 10,000 points x
-// 10,000 rings: 61.5 ms before, 25.4 ms so (with equal runs per CTA,
-// fvx_segments.cu).  Against extended precision the error of a wake's velocities
-// falls from 1.4e-14 to 1.2e-15 (collapsed rings): it was la lb - c3's.
+// About 140 FP64 operations per ring and point against about 300.  The sweeps
+// (fvx_segments.cu) go further and form the scalar parts in three floats
+// (fvx_segment_x3.cuh), which pays where a vortex's record serves many points.
+// Against extended precision the error of a wake's velocities falls from
+// 1.4e-14 to 1.2e-15 (collapsed rings; 4e-16 in three floats): it was
+// la lb - c3's.
 #pragma once
 
 #include "fvx_common.cuh"

@@ -24,10 +24,15 @@
 //   expanded   one thread per vortex, looping over a few target points, so
 //              that a warp writes 32 consecutive (point, vortex, 3) records.
 //
-// Arithmetic per (point, leg): fvx_segment_math.cuh.  The four skip tests take
-// the reference's decisions (warp_kernels.py:46-96).
+// Arithmetic per (point, leg): fvx_segment_x3.cuh.  The four skip tests take
+// the reference's decisions (warp_kernels.py:46-96).  10,000 points x 10,000
+// rings: 61.4 ms with the reference's sequence in FP64, 25.4 ms with its roots,
+// divisions and tests replaced (fvx_segment_math.cuh), 12.5 ms so; 501 points x
+// 1,003 horseshoes expanded 213, 145 and 87 us; 200 points x 100 rings 30, 27
+// and 18 us on the device.
 #include "fvx_common.cuh"
 #include "fvx_segment_math.cuh"
+#include "fvx_segment_x3.cuh"
 
 namespace fvx {
 namespace {
@@ -35,6 +40,8 @@ namespace {
 using namespace seg;
 
 constexpr int kCollThreads = 128;  // target points per collapsed CTA
+constexpr int kCollSlices = 2;     // threads per point, each with every other vortex:
+                                   // 16 warps per SM from the two CTAs' worth of runs
 constexpr int kTile = 64;          // vortices per shared-memory tile
 constexpr int kExpThreads = 64;    // vortices per expanded CTA
 __device__ __forceinline__ void flush_counts(int cnt[4], int64_t* counts) {
@@ -128,10 +135,13 @@ __device__ __forceinline__ int64_t div_small(int64_t a, int64_t b) {
 }
 
 template <int LEGS>
-__global__ void __launch_bounds__(kCollThreads) collapsed_kernel(SegArgs A) {
+__global__ void __launch_bounds__(kCollSlices* kCollThreads) collapsed_kernel(SegArgs A) {
   __shared__ __align__(128) RawTile raw[2];
   __shared__ __align__(16) VortexRec rec[kTile];
+  __shared__ __align__(16) RingX3 recx[kTile];
+  __shared__ double other[3][kCollThreads];  // the second slice's sums
   __shared__ __align__(8) uint64_t bar[2];
+  const int slice = threadIdx.x / kCollThreads, lt = threadIdx.x % kCollThreads;
 
   if (threadIdx.x == 0) {
     mbar_init(&bar[0], 1);
@@ -151,7 +161,7 @@ __global__ void __launch_bounds__(kCollThreads) collapsed_kernel(SegArgs A) {
     const int64_t vb = pos - blk * A.n_vort;
     const int64_t ve = min64(vb + (end - pos), A.n_vort);
     const int ntiles = static_cast<int>((ve - vb + kTile - 1) / kTile);
-    const int64_t i = blk * kCollThreads + threadIdx.x;
+    const int64_t i = blk * kCollThreads + lt;
     const bool active = i < A.n_points;
     double px = 0.0, py = 0.0, pz = 0.0;
     if (active) {
@@ -159,6 +169,8 @@ __global__ void __launch_bounds__(kCollThreads) collapsed_kernel(SegArgs A) {
       py = A.points[3 * i + 1];
       pz = A.points[3 * i + 2];
     }
+    const x3::F3 p[3] = {x3::split_fast(px), x3::split_fast(py), x3::split_fast(pz)};
+    const bool in_range = x3_range(px) && x3_range(py) && x3_range(pz);
     double vx = 0.0, vy = 0.0, vz = 0.0;
     if (threadIdx.x == 0)
       issue_tile(A, raw[buf], vb, static_cast<int>(min64(kTile, ve - vb)), &bar[buf]);
@@ -180,24 +192,34 @@ __global__ void __launch_bounds__(kCollThreads) collapsed_kernel(SegArgs A) {
       phase[buf] ^= 1u;
       tail_tile(A, raw[buf], v0, n);
       __syncthreads();
-      for (int k = threadIdx.x; k < n; k += kCollThreads) {
+      for (int k = threadIdx.x; k < n; k += kCollSlices * kCollThreads) {
         prep_vortex<LEGS>(rec[k], &raw[buf].c[0][3 * k], &raw[buf].c[1][3 * k],
                           &raw[buf].c[2][3 * k], &raw[buf].c[3][3 * k], raw[buf].strength[k],
                           raw[buf].rc0[k], A.ages ? raw[buf].age[k] : 0.0, A.nu);
+        prep_x3<LEGS>(recx[k], rec[k]);
       }
       __syncthreads();
       if (active) {
 #pragma unroll 1
-        for (int k = 0; k < n; ++k) vortex_velocity<LEGS>(rec[k], px, py, pz, vx, vy, vz, cnt);
+        for (int k = slice; k < n; k += kCollSlices)
+          vortex_velocity_x3<LEGS>(RingView{recx[k]}, p, in_range, vx, vy, vz, cnt,
+                                   [&](double* v, int* c) {
+                                     vortex_velocity_rare<LEGS>(rec[k], px, py, pz, v, c);
+                                   });
       }
       __syncthreads();
     }
-    if (active) {
-      double* o =
-          vb == 0 ? A.out + 3 * i : A.partial + 3 * (A.runs.row(blockIdx.x) + threadIdx.x);
-      o[0] = vx;
-      o[1] = vy;
-      o[2] = vz;
+    if (slice == 1) {
+      other[0][lt] = vx;
+      other[1][lt] = vy;
+      other[2][lt] = vz;
+    }
+    __syncthreads();
+    if (slice == 0 && active) {
+      double* o = vb == 0 ? A.out + 3 * i : A.partial + 3 * (A.runs.row(blockIdx.x) + lt);
+      o[0] = vx + other[0][lt];
+      o[1] = vy + other[1][lt];
+      o[2] = vz + other[2][lt];
     }
     pos += ve - vb;
   }
@@ -231,24 +253,78 @@ __global__ void reduce_runs_kernel(const double* __restrict__ partial, int64_t n
   if (active && lane == 0) out[v] += s;
 }
 
+// The general path of one (point, vortex) pair of an expanded call.
+template <int LEGS>
+__device__ __noinline__ void expanded_rare(const SegArgs& A, int64_t m, int64_t p, double* v,
+                                           int* cnt) {
+  VortexRec R;
+  prep_vortex<LEGS>(R, A.corner[0] + 3 * m, A.corner[1] + 3 * m, A.corner[2] + 3 * m,
+                    A.corner[3] + 3 * m, A.strengths[m], A.rc0s[m], A.ages ? A.ages[m] : 0.0,
+                    A.nu);
+  vortex_velocity_rare<LEGS>(R, A.points[3 * p], A.points[3 * p + 1], A.points[3 * p + 2], v, cnt);
+}
+
+// A thread's own vortex in shared memory, word w of thread t at [w][t] (no bank
+// conflicts; the legs' loop indexes corners and legs, which registers cannot).
+constexpr int kRingWords = 48;  // 12 coordinates and 4 leg lengths as three floats
+struct RingColumn {
+  const float* w;
+  const double* c;  // [c2 x 4][half c1]
+  float near_;
+  __device__ __forceinline__ x3::F3 f3(int i) const {
+    return x3::F3{w[3 * i * kExpThreads], w[(3 * i + 1) * kExpThreads],
+                  w[(3 * i + 2) * kExpThreads]};
+  }
+  __device__ __forceinline__ x3::F3 corner(int c_, int k) const { return f3(3 * c_ + k); }
+  __device__ __forceinline__ x3::F3 r0sq(int l) const { return f3(12 + l); }
+  __device__ __forceinline__ double c2(int l) const { return c[l * kExpThreads]; }
+  __device__ __forceinline__ double half_c1() const { return c[4 * kExpThreads]; }
+  __device__ __forceinline__ float near() const { return near_; }
+};
+
 template <int LEGS>
 __global__ void __launch_bounds__(kExpThreads) expanded_kernel(SegArgs A, int points_per_cta) {
-  extern __shared__ double pts[];  // points_per_cta x 3
+  extern __shared__ x3::F3 pts[];  // points_per_cta x 3
+  __shared__ float words[kRingWords * kExpThreads];
+  __shared__ double consts[5 * kExpThreads];
   const int64_t m = static_cast<int64_t>(blockIdx.x) * kExpThreads + threadIdx.x;
   const int64_t p0 = static_cast<int64_t>(blockIdx.y) * points_per_cta;
   const int np = static_cast<int>(min64(points_per_cta, A.n_points - p0));
-  for (int k = threadIdx.x; k < 3 * np; k += kExpThreads) pts[k] = A.points[3 * p0 + k];
+  for (int k = threadIdx.x; k < 3 * np; k += kExpThreads) {
+    const double x = A.points[3 * p0 + k];
+    pts[k] = x3::split_fast(x);
+    if (!x3_range(x)) pts[k].h = __int_as_float(0x7fffffff);  // NaN: the general path
+  }
+  RingColumn col{words + threadIdx.x, consts + threadIdx.x, 0.0f};
+  if (m < A.n_vort) {
+    VortexRec R;
+    RingX3 X;
+    prep_vortex<LEGS>(R, A.corner[0] + 3 * m, A.corner[1] + 3 * m, A.corner[2] + 3 * m,
+                      A.corner[3] + 3 * m, A.strengths[m], A.rc0s[m],
+                      A.ages ? A.ages[m] : 0.0, A.nu);
+    prep_x3<LEGS>(X, R);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const x3::F3 v = i < 12 ? X.c[i / 3][i % 3] : X.r0sq[i & 3];
+      words[(3 * i) * kExpThreads + threadIdx.x] = v.h;
+      words[(3 * i + 1) * kExpThreads + threadIdx.x] = v.m;
+      words[(3 * i + 2) * kExpThreads + threadIdx.x] = v.l;
+    }
+#pragma unroll
+    for (int l = 0; l < 4; ++l) consts[l * kExpThreads + threadIdx.x] = X.c2[l];
+    consts[4 * kExpThreads + threadIdx.x] = X.half_c1;
+    col.near_ = X.near;
+  }
   __syncthreads();
   if (np <= 0) return;
   int cnt[4] = {0, 0, 0, 0};
   if (m < A.n_vort) {
-    VortexRec R;
-    prep_vortex<LEGS>(R, A.corner[0] + 3 * m, A.corner[1] + 3 * m, A.corner[2] + 3 * m,
-                      A.corner[3] + 3 * m, A.strengths[m], A.rc0s[m],
-                      A.ages ? A.ages[m] : 0.0, A.nu);
+#pragma unroll 1
     for (int k = 0; k < np; ++k) {
       double vx = 0.0, vy = 0.0, vz = 0.0;
-      vortex_velocity<LEGS>(R, pts[3 * k], pts[3 * k + 1], pts[3 * k + 2], vx, vy, vz, cnt);
+      vortex_velocity_x3<LEGS>(col, pts + 3 * k, true, vx, vy, vz, cnt, [&](double* v, int* c) {
+        expanded_rare<LEGS>(A, m, p0 + k, v, c);
+      });
       double* o = A.out + ((p0 + k) * A.n_vort + m) * 3;
       o[0] = vx;
       o[1] = vy;
@@ -346,13 +422,13 @@ int segments_collapsed_launch(const double* points, int64_t n_points, const doub
   const unsigned grid = static_cast<unsigned>(ctas);
   switch (leg_set) {
     case FVX_LEGS_RING:
-      collapsed_kernel<FVX_LEGS_RING><<<grid, kCollThreads, 0, stream>>>(A);
+      collapsed_kernel<FVX_LEGS_RING><<<grid, kCollSlices * kCollThreads, 0, stream>>>(A);
       break;
     case FVX_LEGS_CHORDWISE:
-      collapsed_kernel<FVX_LEGS_CHORDWISE><<<grid, kCollThreads, 0, stream>>>(A);
+      collapsed_kernel<FVX_LEGS_CHORDWISE><<<grid, kCollSlices * kCollThreads, 0, stream>>>(A);
       break;
     default:
-      collapsed_kernel<FVX_LEGS_HORSESHOE><<<grid, kCollThreads, 0, stream>>>(A);
+      collapsed_kernel<FVX_LEGS_HORSESHOE><<<grid, kCollSlices * kCollThreads, 0, stream>>>(A);
       break;
   }
   FVX_LAUNCH_CHECK();
@@ -399,7 +475,9 @@ int segments_expanded_launch(const double* points, int64_t n_points, const doubl
   A.counts = counts;
   A.use_tma = 0;
   const int64_t gx = (n_vort + kExpThreads - 1) / kExpThreads;
-  const int64_t want = 4LL * device_sm_count();
+  // eight CTAs per SM: 501 points x 1,003 horseshoes take 125, 95, 87 and 97 us with
+  // 4, 6, 8 and 12 (fewer leave the FP32 pipe waiting, more repeat the prologue)
+  const int64_t want = 8LL * device_sm_count();
   int64_t gy = gx >= want ? 1 : (want + gx - 1) / gx;
   if (gy > n_points) gy = n_points;
   int ppc = static_cast<int>((n_points + gy - 1) / gy);
@@ -407,7 +485,7 @@ int segments_expanded_launch(const double* points, int64_t n_points, const doubl
   gy = (n_points + ppc - 1) / ppc;
   FVX_ARG_CHECK(gy <= 65535, "too many target points for one expanded launch");
   dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
-  size_t smem = sizeof(double) * 3 * ppc;
+  size_t smem = sizeof(x3::F3) * 3 * ppc;
   switch (leg_set) {
     case FVX_LEGS_RING:
       expanded_kernel<FVX_LEGS_RING><<<grid, kExpThreads, smem, stream>>>(A, ppc);

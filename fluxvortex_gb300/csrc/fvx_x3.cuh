@@ -35,6 +35,8 @@ struct F3 {
 };
 
 #if defined(__CUDA_ARCH__)
+FVX_X3 float rcp_seed(float x) { return __frcp_rn(x); }
+FVX_X3 uint64_t words(double x) { return (uint64_t)__double_as_longlong(x); }
 FVX_X3 float add(float a, float b) { return __fadd_rn(a, b); }
 FVX_X3 float sub(float a, float b) { return __fsub_rn(a, b); }
 FVX_X3 float mul(float a, float b) { return __fmul_rn(a, b); }
@@ -47,7 +49,9 @@ FVX_X3 int to_int(float x) { return __float2int_rn(x); }
 FVX_X3 int to_int_down(float x) { return __float2int_rd(x); }
 FVX_X3 float round_int(float x) { return rintf(x); }
 #else
-// the host's forms (compiled without contraction): the tests' oracle runs them
+// the host's forms (compiled without contraction): the tests run them
+FVX_X3 float rcp_seed(float x) { return 1.0f / x; }
+FVX_X3 uint64_t words(double x) { uint64_t w; memcpy(&w, &x, 8); return w; }
 FVX_X3 float add(float a, float b) { return a + b; }
 FVX_X3 float sub(float a, float b) { return a - b; }
 FVX_X3 float mul(float a, float b) { return a * b; }
@@ -96,6 +100,20 @@ FVX_X3 F3 split(double x) {
   return r;
 }
 
+// The same for a positive FP64 number of 2^-60 .. 2^60 by integer operations: the
+// leading 24 bits, the next 15 and the last 14.
+FVX_X3 F3 split_positive(double x) {
+  const uint64_t w = words(x);
+  const uint32_t hi = (uint32_t)(w >> 32), lo = (uint32_t)w;
+  const uint32_t b = ((hi << 3) | (lo >> 29)) - ((uint32_t)(1023 - 127) << 23);
+  const uint32_t e = b & 0x7f800000u;  // 2^exponent
+  F3 r;
+  r.h = from_bits(b);
+  r.m = mul((float)(int)((lo >> 14) & 0x7fffu), from_bits(e - (38u << 23)));
+  r.l = mul((float)(int)(lo & 0x3fffu), from_bits(e - (52u << 23)));
+  return r;
+}
+
 // h >= m >= l (in magnitude, loosely) -> without overlap
 FVX_X3 F3 renorm(float h, float m, float l) {
   F3 r;
@@ -103,6 +121,22 @@ FVX_X3 F3 renorm(float h, float m, float l) {
   r.h = fast_two_sum(h, m, e);
   r.m = fast_two_sum(e, l, r.l);
   return r;
+}
+
+// split() of any FP64 number, off the FP64 pipe where its magnitude allows
+FVX_X3 F3 split_fast(double x) {
+  const uint64_t w = words(x);
+  const uint32_t e = (uint32_t)(w >> 52) & 2047u;
+  if (e - (1023u - 60u) < 120u) {
+    F3 r = split_positive(from_words((uint32_t)(w >> 32) & 0x7fffffffu, (uint32_t)w));
+    const uint32_t sign = (uint32_t)(w >> 32) & 0x80000000u;
+    r.h = from_bits(bits(r.h) ^ sign);
+    r.m = from_bits(bits(r.m) ^ sign);
+    r.l = from_bits(bits(r.l) ^ sign);
+    return renorm(r.h, r.m, r.l);
+  }
+  if ((w << 1) == 0) return F3{0.0f, 0.0f, 0.0f};
+  return split(x);
 }
 
 // Three floats -> the FP64 number nearest to their sum, by integer operations:
@@ -239,7 +273,10 @@ FVX_X3 F3 scale_float(const F3& a, float t) {
   const float v = two_sum(e0, m, e2);
   return F3{h, v, add(fma_(a.l, t, e1), e2)};
 }
-// q^-1 and q^-5/2
+// q^-1/2, q^-1 and q^-5/2
+FVX_X3 F3 power_m1_2(const Root& R) {
+  return power_series(F3{R.t, 0.0f, 0.0f}, R, 0.5f, 0.375f, 0.3125f);
+}
 FVX_X3 F3 power_m1(const Root& R) { return power_series(F3{R.p, R.pe, 0.0f}, R, 1.0f, 1.0f, 1.0f); }
 FVX_X3 F3 power_m5_2(const Root& R) {
   float e0, e1, e2;
@@ -248,6 +285,22 @@ FVX_X3 F3 power_m5_2(const Root& R) {
   const float v = two_sum(e0, m, e2);
   const F3 t4{h, v, add(fma_(R.pe, R.pe, e1), e2)};
   return power_series(scale_float(t4, R.t), R, 2.5f, 4.375f, 6.5625f);
+}
+
+// a / d for an FP64 d of 2^-60 .. 2^60: with y = 1/d's float and E = 1 - d y, a / d =
+// a y (1 + E + E^2 + ..), |E| < 2^-23
+FVX_X3 F3 quotient(const F3& a, double d) {
+  const F3 q = split_positive(d);
+  const float y = rcp_seed(q.h);
+  float re, ve, ea, cl;
+  const float r = two_prod(q.h, y, re);
+  const float v = two_prod(q.m, y, ve);
+  const float e = two_sum(sub(1.0f, r), -add(re, v), ea);
+  // re + v rounds: what it loses (below 2^-24 of 2^-24) joins the low part
+  const float s = add(re, v), back = sub(v, sub(s, re));
+  const float l = sub(ea, add(add(back, ve), mul(q.l, y)));
+  const float ch = fast_two_sum(e, fma_(e, e, l), cl);
+  return scale1p(scale_float(a, y), ch, cl);
 }
 
 // Staged constants of a source: Winckelmans s2 = sigma^2, k = 1.5 sigma^2;
