@@ -66,6 +66,7 @@ SIGNATURES = {
     "fvx_mlp_forward": (I32, [P, I32, P, P, P, P, P, P]),
     "fvx_mlp_gemm": (I32, [P, I32, I32, P, I32, I32, P, I32, I32, I32, I32, I32, I32, P]),
     "fvx_mlp_loss_grad": (I32, [I32, P, P, P, P, P, P, P]),
+    "fvx_mlp_gradients": (I32, [P, P, P, I32, P, P, P, P, P, P, P]),
     "fvx_mlp_silu_back": (I32, [I32, I32, P, P, P, P, P]),
     "fvx_mlp_colsum": (I32, [I32, I32, P, P, P]),
     "fvx_mlp_adam": (I32, [I32, P, P, P, P, P, F, F, F, F, I32, P]),

@@ -16,10 +16,13 @@
 //     warpgroups form the inputs of every tile from the (target leaf, source
 //     cell) pair lists and reduce its outputs, scaled back to physical
 //     local-expansion coefficients, into the leaves' expansions;
-//   * training: a generic tile GEMM C = op(A) op(B)^T on tcgen05 (operands
-//     staged transposed as needed by the threads, split over K with FP32
-//     atomics) for dW = dZ^T H and dH = dZ W, plus element-wise kernels for
-//     the loss gradient, the SiLU backward with bias gradients, and Adam.
+//   * training: gradients_kernel takes 128 rows at a time through forward, loss
+//     and backward in tensor and shared memory; and the same as separate steps
+//     for hosts that put their own loop together: a generic tile GEMM C = op(A)
+//     op(B)^T on tcgen05 (operands staged transposed as needed by the threads,
+//     split over K with FP32 atomics) for dW = dZ^T H and dH = dZ W, element-wise
+//     kernels for the loss gradient and the SiLU backward with bias gradients;
+//     and Adam.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -1306,6 +1309,264 @@ __global__ void colsum_kernel(int rows, int cols, const float* __restrict__ G, f
   atomicAdd(db + c, acc);
 }
 
+// ---- loss and gradients of a batch in one kernel ----------------------------------
+// A CTA takes 128 rows at a time through forward, loss and backward.  The hidden
+// accumulators stay in tensor memory until the backward pass needs them for
+// SiLU', the activations in shared memory, where the weight gradients read them
+// by columns (dW = dZ^T H: K runs along the rows of both tiles) and the input
+// gradients read the forward's own weight tiles by columns (dH = dZ W).  Each
+// dZ replaces the activation tile that its layer's weight gradient has just
+// used.  Same operations and roundings per row as mlp_fwd_kernel<false>,
+// loss_grad_kernel, silu_back_kernel and the GEMMs; weight gradients are summed
+// per 128 rows in tensor memory, then by FP32 atomics.
+// Chain per tile: four forward and three backward MMA steps with their
+// epilogues, 512 threads (a warp: 32 rows x 32 columns).  A gradient pass over
+// 8,192 rows takes 45 us, one fill and this kernel; as sixteen launches, with
+// activations, pre-activations and their gradients through memory, 172 us.
+constexpr int kGradThreads = 512;
+// tensor memory columns: the hidden layers' accumulators at 128 l, then scratch
+constexpr uint32_t kGradScratch = 384;
+
+struct GradSmem {
+  __nv_bfloat16 w1[H * IN], w2[H * H], w3[H * H], w4[OUT * H];
+  __nv_bfloat16 x[128 * IN];
+  __nv_bfloat16 h[3][128 * H];  // activations, then dZ of the layer above's gradient
+  __nv_bfloat16 dy[128 * OUT];
+  float bias[BN], db[BN];
+  double loss[4];
+  uint64_t bar;
+  uint32_t tmem;
+};
+static_assert(sizeof(GradSmem) <= 227 * 1024, "one CTA's tiles must fit shared memory");
+
+struct GradArgs {
+  const __nv_bfloat16* X;
+  const float* T;
+  const float* wrow;
+  const __nv_bfloat16* W;
+  const float* bias;
+  float* Y;
+  float* gw;
+  float* gb;
+  float* loss;
+  int rows, wide;  // wide: gw's rows take 16-byte atomics
+};
+
+// Column sums over the warp's 32 rows of 32 columns: lane c ends with column c's.
+__device__ __forceinline__ float column_sums(float (&x)[32]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) {
+    const bool upper = (lane & off) != 0;
+#pragma unroll
+    for (int j = 0; j < off; ++j) {
+      const float send = upper ? x[j] : x[j + off];
+      const float keep = upper ? x[j + off] : x[j];
+      x[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  return x[0];
+}
+
+__device__ __forceinline__ void load32(uint32_t taddr, float (&v)[32]) {
+  tc::tmem_ld16(taddr, v);
+  tc::tmem_ld16(taddr + 16, v + 16);
+}
+
+// 32 columns of one row as BF16 into a K-major tile of `cols` columns
+__device__ __forceinline__ void store32(__nv_bfloat16* tile, int cols, int row, int c0,
+                                        const float (&v)[32]) {
+  char* base = reinterpret_cast<char*>(tile);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    __align__(16) __nv_bfloat162 b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b[i] = __floats2bfloat162_rn(v[8 * q + 2 * i], v[8 * q + 2 * i + 1]);
+    *reinterpret_cast<uint4*>(base + tc::kmajor_offset(row, c0 + 8 * q, cols)) =
+        *reinterpret_cast<const uint4*>(b);
+  }
+}
+
+// gw[m][n0 ..] += 32 (or n_in - n0) columns of row m
+__device__ __forceinline__ void add_row(float* g, int n, const float (&v)[32], bool wide) {
+  if (wide) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (4 * q < n)
+        atomicAdd(reinterpret_cast<float4*>(g) + q,
+                  make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < n) atomicAdd(g + i, v[i]);
+  }
+}
+
+__global__ void __launch_bounds__(kGradThreads, 1) gradients_kernel(GradArgs A) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  GradSmem& S = *reinterpret_cast<GradSmem*>(smem_raw);
+  if (threadIdx.x < 32) tc::tmem_alloc(&S.tmem, 512);
+  if (threadIdx.x == 0) {
+    mbar_init(&S.bar, 1);
+    fence_mbar_init();
+  }
+  stage_kmajor(S.w1, A.W + W1o, H, IN);
+  stage_kmajor(S.w2, A.W + W2o, H, H);
+  stage_kmajor(S.w3, A.W + W3o, H, H);
+  stage_kmajor(S.w4, A.W + W4o, OUT, H);
+  for (int i = threadIdx.x; i < BN; i += kGradThreads) {
+    S.bias[i] = A.bias[i];
+    S.db[i] = 0.f;
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = S.tmem;
+  const int lane = threadIdx.x & 31, quarter = (threadIdx.x >> 5) & 3;
+  const int lr = 32 * quarter + lane;          // row of the tile = lane of tensor memory
+  const int c0 = 32 * (threadIdx.x >> 7);      // this warp's 32 columns of 128
+  const uint32_t tl = tmem + (static_cast<uint32_t>(32 * quarter) << 16);
+  const uint32_t scratch = tl + kGradScratch;
+  uint32_t ph = 0;
+  bool ok = true;
+  // shared-memory writes visible to the tensor core, tensor memory reads done
+  auto handoff = [&]() {
+    tc::fence_smem_to_async();
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+  };
+  auto commit = [&]() {
+    if (threadIdx.x == 0) tc::mma_commit(&S.bar);
+  };
+  auto wait = [&]() { return __syncthreads_and(wait_mma(&S.bar, ph)) != 0; };
+  const uint32_t id128 = tc::idesc_bf16(128, H), id32 = tc::idesc_bf16(128, OUT),
+                 id48 = tc::idesc_bf16(128, IN);
+  const __nv_bfloat16* wl[3] = {S.w1, S.w2, S.w3};
+  const int ntiles = (A.rows + 127) / 128;
+  double loss = 0.0;
+  for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    const int row = tile * 128 + lr;
+    const bool in = row < A.rows;
+    for (int e = threadIdx.x; e < 128 * (IN / 8); e += kGradThreads) {
+      const int r = e / (IN / 8), k8 = e % (IN / 8);
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (tile * 128 + r < A.rows)
+        v = *reinterpret_cast<const uint4*>(A.X + static_cast<int64_t>(tile * 128 + r) * IN +
+                                            8 * k8);
+      *reinterpret_cast<uint4*>(reinterpret_cast<char*>(S.x) + tc::kmajor_offset(r, 8 * k8, IN)) =
+          v;
+    }
+    // ---- forward
+#pragma unroll 1
+    for (int l = 0; l < 3 && ok; ++l) {
+      handoff();
+      if (threadIdx.x == 0)
+        tc::gemm_issue_ops(tmem + 128 * l, l == 0 ? S.x : S.h[l - 1], l == 0 ? IN : H, wl[l],
+                           l == 0 ? IN : H, l == 0 ? IN : H, id128);
+      commit();
+      ok = wait();
+      if (!ok) break;
+      float v[32];
+      load32(tl + 128 * l + c0, v);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = silu(v[i] + S.bias[H * l + c0 + i]);
+      store32(S.h[l], H, lr, c0, v);
+    }
+    if (!ok) break;
+    handoff();
+    if (threadIdx.x == 0) tc::gemm_issue_ops(tmem + kGradScratch, S.h[2], H, S.w4, H, H, id32);
+    commit();
+    if (!(ok = wait())) break;
+    // ---- loss: the first four warps, one per 32 rows
+    if (threadIdx.x < 128) {
+      float v[32];
+      load32(scratch, v);
+      const float wr = in && A.wrow ? A.wrow[row] : 1.f;
+      const float* t = A.T + static_cast<int64_t>(row) * OUT;
+      float* y = A.Y + static_cast<int64_t>(row) * OUT;
+      float part[2] = {0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < OUT; ++c) {
+        const float yc = v[c] + S.bias[B4o + c];
+        float g = 0.f;
+        if (in) {
+          y[c] = yc;
+          if (c < NOUT) {
+            const float e = yc - t[c];
+            part[c & 1] += wr * e * e;
+            g = 2.f * wr * e / (static_cast<float>(A.rows) * NOUT);
+          }
+        }
+        v[c] = g;
+      }
+      loss += static_cast<double>(part[0]) + static_cast<double>(part[1]);
+      store32(S.dy, OUT, lr, 0, v);
+      const float s = column_sums(v);
+      atomicAdd(&S.db[B4o + lane], s);
+    }
+    // ---- output layer's weight gradient, transposed: H3^T dY (128 x 32)
+    handoff();
+    if (threadIdx.x == 0)
+      tc::gemm_issue_ops(tmem + kGradScratch, S.h[2], H, S.dy, OUT, 128,
+                         id32 | tc::kAColumns | tc::kBColumns);
+    commit();
+    if (!(ok = wait())) break;
+    if (threadIdx.x < 128) {
+      float v[32];
+      load32(scratch, v);
+      float* g = A.gw + W4o + lr;  // row lr: input feature; column: output
+#pragma unroll
+      for (int c = 0; c < NOUT; ++c) atomicAdd(g + c * H, v[c]);
+    }
+    // ---- dH3 = dY W4, then dZ3; per hidden layer its weight gradient and the next dH
+    handoff();
+    if (threadIdx.x == 0)
+      tc::gemm_issue_ops(tmem + kGradScratch, S.dy, OUT, S.w4, H, OUT, id128 | tc::kBColumns);
+    commit();
+    if (!(ok = wait())) break;
+#pragma unroll 1
+    for (int l = 2; l >= 0; --l) {
+      float z[32], g[32];
+      load32(tl + 128 * l + c0, z);
+      load32(scratch + c0, g);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) g[i] *= silu_grad(z[i] + S.bias[H * l + c0 + i]);
+      store32(S.h[l], H, lr, c0, g);  // dZ; the layer above has used h[l]
+      const float s = column_sums(g);
+      atomicAdd(&S.db[H * l + c0 + lane], s);
+      handoff();
+      // dW_l over this tile's rows into the accumulator that SiLU' is done with;
+      // dH of the layer below into scratch
+      const int n_in = l > 0 ? H : IN;
+      if (threadIdx.x == 0) {
+        tc::gemm_issue_ops(tmem + 128 * l, S.h[l], H, l > 0 ? S.h[l - 1] : S.x, n_in, 128,
+                           (l > 0 ? id128 : id48) | tc::kAColumns | tc::kBColumns);
+        if (l > 0)
+          tc::gemm_issue_ops(tmem + kGradScratch, S.h[l], H, wl[l], H, H, id128 | tc::kBColumns);
+      }
+      commit();
+      if (!(ok = wait())) break;
+      if (c0 < n_in) {
+        load32(tl + 128 * l + c0, z);
+        const int off = l == 0 ? W1o : (l == 1 ? W2o : W3o);
+        add_row(A.gw + off + lr * n_in + c0, min(32, n_in - c0), z, A.wide != 0);
+      }
+    }
+  }
+  if (!ok && threadIdx.x == 0) flag_status(kStatusTimeout);
+  // the loss in FP64 up to one FP32 addition per CTA
+  for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+  if (lane == 0 && threadIdx.x < 128) S.loss[quarter] = loss;
+  tc::fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x == 0)
+    atomicAdd(A.loss, static_cast<float>((S.loss[0] + S.loss[1]) + (S.loss[2] + S.loss[3])));
+  for (int i = threadIdx.x; i < BN; i += kGradThreads)
+    if (S.db[i] != 0.f) atomicAdd(A.gb + i, S.db[i]);
+  if (threadIdx.x < 32) tc::tmem_dealloc(tmem, 512);
+}
+
 // Adam on FP32 master weights; refreshes the BF16 copy.
 __global__ void adam_kernel(int n, float* __restrict__ w, const float* __restrict__ g,
                             float* __restrict__ m, float* __restrict__ v,
@@ -1517,6 +1778,25 @@ int fvx_mlp_gemm(const void* A, int lda, int tA, const void* B, int ldb, int tB,
       static_cast<const __nv_bfloat16*>(A), lda, tA, wide(A, lda, tA),
       static_cast<const __nv_bfloat16*>(B), ldb, tB, wide(B, ldb, tB), C, ldc, wide_c, M, N, K,
       kchunk, accumulate);
+  FVX_LAUNCH_CHECK();
+  return FVX_OK;
+}
+
+int fvx_mlp_gradients(const void* X, const float* T, const float* row_weight, int rows,
+                      const void* W, const float* bias, float* Y, float* gw, float* gb,
+                      float* loss, void* stream) {
+  using namespace fvx::mlp;
+  FVX_ARG_CHECK(rows > 0 && X && T && W && bias && Y && gw && gb && loss, "bad arguments");
+  FVX_ARG_CHECK(fvx::aligned16(X) && fvx::aligned16(W), "X and W need 16-byte alignment");
+  FVX_CUDA_TRY(cudaFuncSetAttribute(gradients_kernel,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(sizeof(GradSmem))));
+  const GradArgs A{static_cast<const __nv_bfloat16*>(X), T, row_weight,
+                   static_cast<const __nv_bfloat16*>(W), bias, Y, gw, gb, loss, rows,
+                   fvx::aligned16(gw) ? 1 : 0};
+  const int ntiles = (rows + 127) / 128;
+  const int grid = ntiles < fvx::device_sm_count() ? ntiles : fvx::device_sm_count();
+  gradients_kernel<<<grid, kGradThreads, sizeof(GradSmem), static_cast<cudaStream_t>(stream)>>>(A);
   FVX_LAUNCH_CHECK();
   return FVX_OK;
 }

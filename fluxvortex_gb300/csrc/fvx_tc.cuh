@@ -51,6 +51,12 @@ __host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
          | (static_cast<uint32_t>(M >> 4) << 24);   // M / 16
 }
 
+// The same tile read the other way: as an operand whose M (or N) runs along the
+// tile's columns and whose K along its rows ("MN-major").  A core matrix holds 8
+// x 8 elements either way; MN advances by 128 B per core matrix, K by the 8-row
+// groups' stride.  Selected per operand in the instruction descriptor.
+constexpr uint32_t kAColumns = 1u << 15, kBColumns = 1u << 16;
+
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                    smem_u32(slot)),
@@ -145,6 +151,24 @@ __device__ __forceinline__ void gemm_issue(uint32_t d_tmem, const void* A, const
              (accumulate || kk > 0) ? 1u : 0u);
   }
   mma_commit(bar);
+}
+
+// Issues the K/16 MMAs of D[128 x N] = op(A) op(B)^T from one thread (no commit).
+// A tile of `cols` columns is read by rows (K along its columns) or, with the
+// flag in `idesc`, by columns (K along its rows).
+__device__ __forceinline__ void gemm_issue_ops(uint32_t d_tmem, const void* A, int a_cols,
+                                               const void* B, int b_cols, int K, uint32_t idesc) {
+  const uint32_t a0 = smem_u32(A), b0 = smem_u32(B);
+  const uint32_t ag = static_cast<uint32_t>(a_cols >> 3) * 128u,
+                 bg = static_cast<uint32_t>(b_cols >> 3) * 128u;  // 8-row group strides
+  const bool ac = (idesc & kAColumns) != 0, bc = (idesc & kBColumns) != 0;
+  for (int kk = 0; kk < K / 16; ++kk) {
+    // two core matrices along K
+    const uint32_t ao = static_cast<uint32_t>(kk) * (ac ? 2u * ag : 256u),
+                   bo = static_cast<uint32_t>(kk) * (bc ? 2u * bg : 256u);
+    mma_bf16(d_tmem, smem_desc(a0 + ao, ac ? ag : 128u, ac ? 128u : ag),
+             smem_desc(b0 + bo, bc ? bg : 128u, bc ? 128u : bg), idesc, kk > 0 ? 1u : 0u);
+  }
 }
 
 }  // namespace tc

@@ -79,11 +79,11 @@ class FarFieldMLP:
         self.vw = torch.zeros_like(self.w32)
         self.mb = torch.zeros_like(self.b)
         self.vb = torch.zeros_like(self.b)
-        self.gw = torch.zeros_like(self.w32)
-        self.gb = torch.zeros_like(self.b)
+        # gradients and loss side by side: one fill clears them
+        self._grads = torch.zeros(NW + NB + 1, dtype=torch.float32, device=self.device)
+        self.gw, self.gb, self.loss = self._grads.split([NW, NB, 1])
         self.step_count = 0
         self.lib = _capi.load()
-        self._bufs = {}
         self.meta = {}
 
     # ---- persistence ---------------------------------------------------------------
@@ -124,62 +124,19 @@ class FarFieldMLP:
         return (Y, Z, Hs) if store else Y
 
     # ---- training ----------------------------------------------------------------
-    def _gemm(self, A, lda, tA, B, ldb, tB, C, ldc, M, N, K, split_k, accumulate):
-        _capi.check(self.lib.fvx_mlp_gemm(A, lda, tA, B, ldb, tB, C, ldc, M, N, K, split_k,
-                                          accumulate, self._stream()))
-
-    def _buffers(self, rows):
-        bufs = self._bufs.get(rows)
-        if bufs is None:
-            dev = self.device
-            bufs = dict(
-                dY=torch.empty((rows, OUT), dtype=torch.bfloat16, device=dev),
-                dY32=torch.empty((rows, OUT), dtype=torch.float32, device=dev),
-                dH=torch.empty((rows, HID), dtype=torch.float32, device=dev),
-                dZ=torch.empty((rows, HID), dtype=torch.bfloat16, device=dev),
-                loss=torch.zeros(1, dtype=torch.float32, device=dev))
-            self._bufs = {rows: bufs}
-        return bufs
-
     def gradients(self, X, T, weights=None):
         """Loss sum(w_r (Y - T)^2) over the 30 used outputs (device scalar; w_r = 1
         without row weights) and the gradients of the mean loss into self.gw /
         self.gb."""
         rows = X.shape[0]
-        Y, Z, Hs = self.forward(X, store=True)
-        bf = self._buffers(rows)
-        self.gw.zero_()
-        self.gb.zero_()
-        bf["loss"].zero_()
-        st = self._stream()
-        lib = self.lib
-        _capi.check(lib.fvx_mlp_loss_grad(rows, Y.data_ptr(), T.data_ptr(),
-                                          None if weights is None else weights.data_ptr(),
-                                          bf["dY"].data_ptr(), bf["dY32"].data_ptr(),
-                                          bf["loss"].data_ptr(), st))
-        split = max(1, rows // 256)      # two 128-row chunks per CTA
-        gw, wb = self.gw.data_ptr(), self.wb.data_ptr()
-        es_w, es_b = self.gw.element_size(), self.wb.element_size()
-        # output layer
-        self._gemm(bf["dY"].data_ptr(), OUT, 1, Hs[2].data_ptr(), HID, 1,
-                   gw + W_OFFSETS[3] * es_w, HID, OUT, HID, rows, split, 1)
-        _capi.check(lib.fvx_mlp_colsum(rows, OUT, bf["dY32"].data_ptr(),
-                                       self.gb.data_ptr() + B_OFFSETS[3] * 4, st))
-        self._gemm(bf["dY"].data_ptr(), OUT, 0, wb + W_OFFSETS[3] * es_b, HID, 1,
-                   bf["dH"].data_ptr(), HID, rows, HID, OUT, 1, 0)
-        # hidden layers, last to first
-        for l in (2, 1, 0):
-            n_in = HID if l > 0 else IN
-            _capi.check(lib.fvx_mlp_silu_back(rows, HID, bf["dH"].data_ptr(), Z[l].data_ptr(),
-                                              bf["dZ"].data_ptr(),
-                                              self.gb.data_ptr() + B_OFFSETS[l] * 4, st))
-            inp = Hs[l - 1].data_ptr() if l > 0 else X.data_ptr()
-            self._gemm(bf["dZ"].data_ptr(), HID, 1, inp, n_in, 1, gw + W_OFFSETS[l] * es_w,
-                       n_in, HID, n_in, rows, split, 1)
-            if l > 0:
-                self._gemm(bf["dZ"].data_ptr(), HID, 0, wb + W_OFFSETS[l] * es_b, n_in, 1,
-                           bf["dH"].data_ptr(), HID, rows, HID, HID, 1, 0)
-        return bf["loss"], Y
+        assert X.dtype == torch.bfloat16 and X.shape[1] == IN and X.is_contiguous()
+        Y = torch.empty((rows, OUT), dtype=torch.float32, device=self.device)
+        self._grads.zero_()
+        _capi.check(self.lib.fvx_mlp_gradients(
+            X.data_ptr(), T.data_ptr(), None if weights is None else weights.data_ptr(), rows,
+            self.wb.data_ptr(), self.b.data_ptr(), Y.data_ptr(), self.gw.data_ptr(),
+            self.gb.data_ptr(), self.loss.data_ptr(), self._stream()))
+        return self.loss, Y
 
     def adam(self, lr, b1=0.9, b2=0.999, eps=1e-8):
         self.step_count += 1

@@ -502,6 +502,12 @@ int fvx_flutter_sweep(const FlutterParams* params, const FlutterState* state, in
  * fvx_mlp_loss_grad: weighted mean-square loss over the 30 used outputs:
  *   loss += sum w_r (Y - T)^2 (device scalar), dY = 2 w_r (Y - T) / (30 rows)
  *   in BF16 and FP32; row_weight (w_r, FP32 [rows]) may be NULL (w_r = 1).
+ * fvx_mlp_gradients: forward, loss and backward of a batch in one kernel (the
+ *   forward with stores, fvx_mlp_loss_grad, fvx_mlp_silu_back, fvx_mlp_colsum
+ *   and the GEMMs of a training step, nothing stored between): Y as
+ *   fvx_mlp_forward with stores, loss +=, and the packed weight and bias
+ *   gradients of the mean loss added to gw and gb.  X (16-byte aligned) and T
+ *   (FP32 [rows][32]) row by row, W and bias as in fvx_mlp_forward.
  * fvx_mlp_silu_back: dZ = dH SiLU'(Z) (BF16 out), db[c] += sum_r dZ[r][c].
  * fvx_mlp_colsum: db[c] += sum_r G[r][c].
  * fvx_mlp_adam: Adam step `step` (1-based) on FP32 master weights w with
@@ -514,6 +520,9 @@ int fvx_mlp_gemm(const void* A, int lda, int tA, const void* B, int ldb, int tB,
                  int ldc, int M, int N, int K, int split_k, int accumulate, void* stream);
 int fvx_mlp_loss_grad(int rows, const float* Y, const float* T, const float* row_weight, void* dY,
                       float* dY32, float* loss, void* stream);
+int fvx_mlp_gradients(const void* X, const float* T, const float* row_weight, int rows,
+                      const void* W, const float* bias, float* Y, float* gw, float* gb,
+                      float* loss, void* stream);
 int fvx_mlp_silu_back(int rows, int cols, const float* dH, const float* Z, void* dZ, float* db,
                       void* stream);
 int fvx_mlp_colsum(int rows, int cols, const float* G, float* db, void* stream);
