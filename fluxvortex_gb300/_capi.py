@@ -119,6 +119,8 @@ def library_path() -> str:
 def load(build_if_missing: bool = True):
     """Loads (building first if needed) and returns the ctypes library."""
     global _lib
+    if _lib is not None:       # set once, complete
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
@@ -145,6 +147,9 @@ def check(status: int) -> None:
 
 def context(device: int = 0) -> int:
     """Process-wide host-call context for `device` (created on first use)."""
+    h = _contexts.get(device)
+    if h is not None:
+        return h
     lib = load()
     with _lock:
         h = _contexts.get(device)

@@ -22,6 +22,8 @@ count singular cases into it.
 """
 from __future__ import annotations
 
+import contextlib
+
 import numpy as np
 
 from . import _capi
@@ -36,17 +38,25 @@ __all__ = [
 ]
 
 
+_F64, _I64 = np.dtype(np.float64), np.dtype(np.int64)
+
+
 def _is_cuda_tensor(x) -> bool:
     return getattr(x, "is_cuda", False) and hasattr(x, "data_ptr")
 
 
 def _host_f64(a, shape_tail):
+    # (an array that already is what the kernel takes passes unchanged)
+    if type(a) is np.ndarray and a.dtype is _F64 and a.flags.c_contiguous:
+        if a.shape[1:] == shape_tail and a.ndim == 1 + len(shape_tail):
+            return a
     a = np.ascontiguousarray(a, dtype=np.float64)
     return a.reshape((-1,) + shape_tail) if shape_tail else a.reshape(-1)
 
 
 def _ptr(a):
-    return None if a is None else a.ctypes.data
+    # (the attribute ndarray.ctypes builds an object on each access)
+    return None if a is None else a.__array_interface__["data"][0]
 
 
 def _segments_host(expanded, leg_set, points, br, fr, fl, bl, strengths, r_c0s, counts, ages, nu):
@@ -57,14 +67,19 @@ def _segments_host(expanded, leg_set, points, br, fr, fl, bl, strengths, r_c0s, 
     rc = _host_f64(r_c0s, ())
     a = None if ages is None else _host_f64(ages, ())
     N, M = P.shape[0], s.shape[0]
-    if any(c.shape[0] != M for c in C) or rc.shape[0] != M or (a is not None and a.shape[0] != M):
+    if not (C[0].shape[0] == C[1].shape[0] == C[2].shape[0] == C[3].shape[0] == rc.shape[0] == M
+            and (a is None or a.shape[0] == M)):
         raise ValueError("vortex arrays must all have strengths.shape[0] rows")
-    out = np.empty((N, M, 3) if expanded else (N, 3), dtype=np.float64)
-    cnt = np.zeros(4, dtype=np.int64)
+    out = np.empty((N, M, 3) if expanded else (N, 3))
+    # the library adds to int64 counters in place
+    direct = (type(counts) is np.ndarray and counts.dtype is _I64 and counts.size >= 4
+              and counts.flags.c_contiguous and counts.flags.writeable)
+    cnt = counts if direct else np.zeros(4, dtype=np.int64)
     fn = lib.fvx_host_segments_expanded if expanded else lib.fvx_host_segments_collapsed
-    _capi.check(fn(_capi.context(0), _ptr(P), N, *[_ptr(c) for c in C], _ptr(s), _ptr(rc),
-                   _ptr(a), float(nu), M, leg_set, _ptr(out), _ptr(cnt)))
-    _add_counts(counts, cnt)
+    _capi.check(fn(_capi.context(0), _ptr(P), N, *map(_ptr, C), _ptr(s), _ptr(rc), _ptr(a),
+                   float(nu), M, leg_set, _ptr(out), _ptr(cnt)))
+    if not direct:
+        _add_counts(counts, cnt)
     return out
 
 
@@ -82,35 +97,45 @@ def _segments_device(expanded, leg_set, points, br, fr, fl, bl, strengths, r_c0s
     import torch
     lib = _capi.load()
     dev = points.device
+    f64 = torch.float64
 
-    def f64(x, tail):
-        t = torch.as_tensor(x, device=dev, dtype=torch.float64).contiguous()
+    def rows(x, tail):
+        # (an array that already is what the kernel takes passes unchanged)
+        if (torch.is_tensor(x) and x.dtype is f64 and x.device == dev and x.is_contiguous()
+                and x.dim() == 1 + len(tail) and (not tail or x.shape[1] == tail[0])):
+            return x
+        t = torch.as_tensor(x, device=dev, dtype=f64).contiguous()
         return t.reshape((-1,) + tail) if tail else t.reshape(-1)
 
-    P = f64(points, (3,))
-    C = [f64(x, (3,)) for x in (br, fr, fl, bl)]
-    s = f64(strengths, ())
-    rc = f64(r_c0s, ())
-    a = None if ages is None else f64(ages, ())
+    P = rows(points, (3,))
+    C = [rows(x, (3,)) for x in (br, fr, fl, bl)]
+    s = rows(strengths, ())
+    rc = rows(r_c0s, ())
+    a = None if ages is None else rows(ages, ())
     N, M = P.shape[0], s.shape[0]
     stream = torch.cuda.current_stream(dev).cuda_stream
-    out = torch.empty((N, M, 3) if expanded else (N, 3), device=dev, dtype=torch.float64)
-    dcnt = torch.zeros(4, device=dev, dtype=torch.int64)
+    out = torch.empty((N, M, 3) if expanded else (N, 3), device=dev, dtype=f64)
+    # the kernel adds to int64 counters on this device in place
+    direct = (_is_cuda_tensor(counts) and counts.dtype is torch.int64 and counts.device == dev
+              and counts.is_contiguous() and counts.numel() >= 4)
+    dcnt = counts if direct else torch.zeros(4, device=dev, dtype=torch.int64)
     ap = None if a is None else a.data_ptr()
-    with torch.cuda.device(dev):
+    ptrs = [c.data_ptr() for c in C]
+    switch = (contextlib.nullcontext() if dev.index is None
+              or dev.index == torch.cuda.current_device() else torch.cuda.device(dev))
+    with switch:
         if expanded:
-            st = lib.fvx_segments_expanded(P.data_ptr(), N, *[c.data_ptr() for c in C],
-                                           s.data_ptr(), rc.data_ptr(), ap, float(nu), M, leg_set,
-                                           out.data_ptr(), dcnt.data_ptr(), stream)
+            st = lib.fvx_segments_expanded(P.data_ptr(), N, *ptrs, s.data_ptr(), rc.data_ptr(), ap,
+                                           float(nu), M, leg_set, out.data_ptr(),
+                                           dcnt.data_ptr(), stream)
         else:
             nbytes = lib.fvx_segments_collapsed_scratch_bytes(N, M, leg_set)
             scratch = torch.empty(max(nbytes, 1), device=dev, dtype=torch.uint8)
-            st = lib.fvx_segments_collapsed(P.data_ptr(), N, *[c.data_ptr() for c in C],
-                                            s.data_ptr(), rc.data_ptr(), ap, float(nu), M, leg_set,
-                                            out.data_ptr(), dcnt.data_ptr(), scratch.data_ptr(),
-                                            nbytes, stream)
+            st = lib.fvx_segments_collapsed(P.data_ptr(), N, *ptrs, s.data_ptr(), rc.data_ptr(),
+                                            ap, float(nu), M, leg_set, out.data_ptr(),
+                                            dcnt.data_ptr(), scratch.data_ptr(), nbytes, stream)
     _capi.check(st)
-    if counts is not None:
+    if counts is not None and not direct:
         if _is_cuda_tensor(counts):
             counts.view(-1)[:4] += dcnt.to(counts.dtype)
         else:

@@ -67,6 +67,14 @@ struct JudgeSampleView {
   float h[2];                // target size of each list
 };
 
+// Collapsed line-vortex sweep on page-locked host memory (fvx_segments.cu): the
+// inputs are read where they are, and the result and the skip counts written
+// here.
+struct SegmentsHostIO {
+  double* out;
+  int64_t* counts;
+};
+
 // Thread-local error message of the last failing C-ABI call.
 void set_last_error(const char* fmt, ...);
 

@@ -25,7 +25,7 @@ namespace fvx {
 int segments_collapsed_launch(const double*, int64_t, const double*, const double*,
                               const double*, const double*, const double*, const double*,
                               const double*, double, int64_t, int, double*, int64_t*, void*,
-                              size_t, cudaStream_t);
+                              size_t, const SegmentsHostIO*, cudaStream_t);
 size_t segments_collapsed_scratch(int64_t, int64_t);
 
 namespace {
@@ -89,6 +89,6 @@ extern "C" int fvx_segments_collapsed_noalloc(const double* points, int64_t n_po
   if (rc != FVX_OK) return rc;
   return fvx::segments_collapsed_launch(points, n_points, br, fr, fl, bl, strengths, r_c0s, ages,
                                         nu, n_vortices, leg_set, out, singularity_counts,
-                                        scratch, fvx::kScratchBytes,
+                                        scratch, fvx::kScratchBytes, nullptr,
                                         static_cast<cudaStream_t>(stream));
 }

@@ -79,7 +79,7 @@ int device_smem_optin() {
 int segments_collapsed_launch(const double*, int64_t, const double*, const double*,
                               const double*, const double*, const double*, const double*,
                               const double*, double, int64_t, int, double*, int64_t*, void*,
-                              size_t, cudaStream_t);
+                              size_t, const SegmentsHostIO*, cudaStream_t);
 size_t segments_collapsed_scratch(int64_t, int64_t);
 int segments_expanded_launch(const double*, int64_t, const double*, const double*,
                              const double*, const double*, const double*, const double*,
@@ -99,6 +99,8 @@ struct fvx_context {
   size_t dcap = 0;
   void* hbuf = nullptr;
   size_t hcap = 0;
+  int64_t* counters = nullptr;   // skip counts of the calls that copy nothing
+  bool counters_clear = false;   // all four zero (each such call leaves them so)
   std::mutex mu;
 };
 
@@ -140,14 +142,18 @@ int ensure(fvx_context* c, size_t dbytes, size_t hbytes) {
   return FVX_OK;
 }
 
-// Copies the packed inputs to the device workspace (one transfer).
-int upload(fvx_context* c, const Packer& pk) {
+void stage(fvx_context* c, const Packer& pk) {
   char* h = static_cast<char*>(c->hbuf);
   size_t off = 0;
   for (auto& it : pk.items) {
     if (it.first && it.second) std::memcpy(h + off, it.first, it.second);
     off = round_up(off + it.second);
   }
+}
+
+// Copies the packed inputs to the device workspace (one transfer).
+int upload(fvx_context* c, const Packer& pk) {
+  stage(c, pk);
   if (pk.total)
     FVX_CUDA_TRY(cudaMemcpyAsync(c->dbuf, c->hbuf, pk.total, cudaMemcpyHostToDevice, c->stream));
   return FVX_OK;
@@ -169,6 +175,13 @@ struct DevGuard {
     if (prev >= 0 && cudaGetDevice(&cur) == cudaSuccess && cur != prev) cudaSetDevice(prev);
   }
 };
+
+// Inputs up to this many bytes are read by the kernel from the pinned buffer
+// over the coherent link, and the results written to it: no transfer and no fill
+// then stand before and after the two kernels.  Whole call, copied against read
+// in place: 200 points x 100 rings (16 KB) 62 and 54 us, 100 x 500 (61 KB) 75 and
+// 65, 1,000 x 1,000 (141 KB) 203 and 197, 1,000 x 2,000 (258 KB) 329 and 332.
+constexpr size_t kDirectBytes = size_t(256) << 10;
 
 int host_segments(fvx_context* c, bool expanded, const double* points, int64_t n_points,
                   const double* br, const double* fr, const double* fl, const double* bl,
@@ -196,6 +209,30 @@ int host_segments(fvx_context* c, bool expanded, const double* points, int64_t n
   const size_t out_bytes = round_up(out_elems * sizeof(double));
   const size_t cnt_bytes = round_up(4 * sizeof(int64_t));
   const size_t scratch = expanded ? 0 : round_up(fvx::segments_collapsed_scratch(n_points, n_vort));
+  if (!expanded && scratch > 0 && in_bytes <= kDirectBytes) {
+    int rc = ensure(c, out_bytes + scratch, in_bytes + out_bytes + cnt_bytes);
+    if (rc) return rc;
+    if (c->counters == nullptr) FVX_CUDA_TRY(cudaMalloc(&c->counters, 4 * sizeof(int64_t)));
+    if (!c->counters_clear)
+      FVX_CUDA_TRY(cudaMemsetAsync(c->counters, 0, 4 * sizeof(int64_t), c->stream));
+    c->counters_clear = false;
+    stage(c, pk);
+    char* h = static_cast<char*>(c->hbuf);
+    auto in = [&](size_t off) { return reinterpret_cast<const double*>(h + off); };
+    const fvx::SegmentsHostIO io{reinterpret_cast<double*>(h + in_bytes),
+                                 reinterpret_cast<int64_t*>(h + in_bytes + out_bytes)};
+    rc = fvx::segments_collapsed_launch(
+        in(o_p), n_points, in(o_c[0]), in(o_c[1]), in(o_c[2]), in(o_c[3]), in(o_s), in(o_r),
+        ages ? in(o_a) : nullptr, nu, n_vort, leg_set, dptr<double>(c, 0), c->counters,
+        dptr<char>(c, out_bytes), scratch, &io, c->stream);
+    if (rc) return rc;
+    FVX_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    c->counters_clear = true;
+    std::memcpy(out, io.out, out_elems * sizeof(double));
+    if (counts)
+      for (int k = 0; k < 4; ++k) counts[k] += io.counts[k];
+    return FVX_OK;
+  }
   const size_t o_out = in_bytes, o_cnt = o_out + out_bytes, o_scr = o_cnt + cnt_bytes;
   int rc = ensure(c, o_scr + scratch, in_bytes > out_bytes + cnt_bytes ? in_bytes : out_bytes + cnt_bytes);
   if (rc) return rc;
@@ -214,7 +251,7 @@ int host_segments(fvx_context* c, bool expanded, const double* points, int64_t n
                                         dptr<double>(c, o_s), dptr<double>(c, o_r),
                                         ages ? dptr<double>(c, o_a) : nullptr, nu, n_vort,
                                         leg_set, dptr<double>(c, o_out), dptr<int64_t>(c, o_cnt),
-                                        dptr<char>(c, o_scr), scratch, c->stream);
+                                        dptr<char>(c, o_scr), scratch, nullptr, c->stream);
   if (rc) return rc;
   // output and counters are adjacent: one device-to-host transfer
   FVX_CUDA_TRY(cudaMemcpyAsync(c->hbuf, dptr<char>(c, o_out), out_bytes + cnt_bytes,
@@ -269,6 +306,7 @@ void fvx_context_destroy(fvx_context* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->dbuf) cudaFree(c->dbuf);
     if (c->hbuf) cudaFreeHost(c->hbuf);
+    if (c->counters) cudaFree(c->counters);
     if (c->stream) cudaStreamDestroy(c->stream);
   }
   delete c;

@@ -134,6 +134,23 @@ __device__ __forceinline__ int64_t div_small(int64_t a, int64_t b) {
   return ((a | b) >> 32) == 0 ? static_cast<uint32_t>(a) / static_cast<uint32_t>(b) : a / b;
 }
 
+// The whole tile by plain loads, every element in flight at once (array after
+// array, the copies above wait for seven loads in a row; over the link to host
+// memory that is 10 us).
+__device__ void load_tile(const SegArgs& A, RawTile& raw, int64_t v0, int n) {
+  const int words = (A.ages ? 15 : 14) * n;
+  for (int e = threadIdx.x; e < words; e += blockDim.x) {
+    if (e < 12 * n) {
+      const int c = e / (3 * n), k = e - 3 * n * c;
+      raw.c[c][k] = A.corner[c][3 * v0 + k];
+    } else {
+      const int f = e / n - 12, k = e - n * (f + 12);
+      (f == 0 ? raw.strength : (f == 1 ? raw.rc0 : raw.age))[k] =
+          (f == 0 ? A.strengths : (f == 1 ? A.rc0s : A.ages))[v0 + k];
+    }
+  }
+}
+
 template <int LEGS>
 __global__ void __launch_bounds__(kCollSlices* kCollThreads) collapsed_kernel(SegArgs A) {
   __shared__ __align__(128) RawTile raw[2];
@@ -190,7 +207,10 @@ __global__ void __launch_bounds__(kCollSlices* kCollThreads) collapsed_kernel(Se
         return;
       }
       phase[buf] ^= 1u;
-      tail_tile(A, raw[buf], v0, n);
+      if (A.use_tma)
+        tail_tile(A, raw[buf], v0, n);
+      else
+        load_tile(A, raw[buf], v0, n);
       __syncthreads();
       for (int k = threadIdx.x; k < n; k += kCollSlices * kCollThreads) {
         prep_vortex<LEGS>(rec[k], &raw[buf].c[0][3 * k], &raw[buf].c[1][3 * k],
@@ -226,14 +246,20 @@ __global__ void __launch_bounds__(kCollSlices* kCollThreads) collapsed_kernel(Se
   flush_counts(cnt, A.counts);
 }
 
-// out[v] += the partial sums of value v = 3 row + component, in a fixed order:
+// dst[v] = out[v] + the partial sums of value v = 3 row + component, in a fixed order:
 // kReduceLanes lanes per value take the block's CTAs in turn, then a shuffle
 // tree.  (One thread per value waits for one load after another: 12 us for 200
 // points split 50 ways.)
 constexpr int kReduceLanes = 8;
 
+// dst_counts, if not null, receives the skip counts, which start again at zero.
 __global__ void reduce_runs_kernel(const double* __restrict__ partial, int64_t n_points, Runs R,
-                                   double* __restrict__ out) {
+                                   const double* out, double* dst, int64_t* counts,
+                                   int64_t* dst_counts) {
+  if (dst_counts != nullptr && blockIdx.x == 0 && threadIdx.x < 4) {
+    dst_counts[threadIdx.x] = counts[threadIdx.x];
+    counts[threadIdx.x] = 0;
+  }
   const int64_t v =
       (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kReduceLanes;
   const int lane = threadIdx.x % kReduceLanes;
@@ -250,7 +276,7 @@ __global__ void reduce_runs_kernel(const double* __restrict__ partial, int64_t n
 #pragma unroll
   for (int off = kReduceLanes / 2; off >= 1; off >>= 1)
     s += __shfl_down_sync(0xffffffffu, s, off, kReduceLanes);
-  if (active && lane == 0) out[v] += s;
+  if (active && lane == 0) dst[v] = out[v] + s;
 }
 
 // The general path of one (point, vortex) pair of an expanded call.
@@ -372,12 +398,16 @@ int check_legs(int leg_set) {
 }  // namespace
 
 // Internal launcher shared by the device, host and scratch-free entry points.
+// host: the inputs are in page-locked host memory, read as they are, and the
+// result (out being device memory) and the skip counts go to host->out and
+// host->counts there, the device's counters restarting at zero; asked for only
+// where segments_collapsed_scratch is not 0.
 int segments_collapsed_launch(const double* points, int64_t n_points, const double* br,
                               const double* fr, const double* fl, const double* bl,
                               const double* strengths, const double* r_c0s, const double* ages,
                               double nu, int64_t n_vort, int leg_set, double* out,
                               int64_t* counts, void* scratch, size_t scratch_bytes,
-                              cudaStream_t stream) {
+                              const SegmentsHostIO* host, cudaStream_t stream) {
   FVX_ARG_CHECK(check_legs(leg_set), "unknown leg set %d", leg_set);
   FVX_ARG_CHECK(n_points >= 0 && n_vort >= 0, "negative size");
   if (n_points == 0) return FVX_OK;
@@ -417,7 +447,7 @@ int segments_collapsed_launch(const double* points, int64_t n_points, const doub
   A.out = out;
   A.partial = static_cast<double*>(scratch);
   A.counts = counts;
-  A.use_tma = aligned16(br) && aligned16(fr) && aligned16(fl) && aligned16(bl) &&
+  A.use_tma = host == nullptr && aligned16(br) && aligned16(fr) && aligned16(fl) && aligned16(bl) &&
               aligned16(strengths) && aligned16(r_c0s) && (!ages || aligned16(ages));
   const unsigned grid = static_cast<unsigned>(ctas);
   switch (leg_set) {
@@ -435,7 +465,8 @@ int segments_collapsed_launch(const double* points, int64_t n_points, const doub
   if (splits > 1) {
     const int64_t lanes = 3 * n_points * kReduceLanes;
     reduce_runs_kernel<<<static_cast<unsigned>((lanes + 255) / 256), 256, 0, stream>>>(
-        A.partial, n_points, R, out);
+        A.partial, n_points, R, out, host ? host->out : out, counts,
+        host ? host->counts : nullptr);
     FVX_LAUNCH_CHECK();
   }
   return FVX_OK;
@@ -517,7 +548,7 @@ int fvx_segments_collapsed(const double* points, int64_t n_points, const double*
                            void* stream) {
   return fvx::segments_collapsed_launch(points, n_points, br, fr, fl, bl, strengths, r_c0s,
                                         ages, nu, n_vortices, leg_set, out, singularity_counts,
-                                        scratch, scratch_bytes,
+                                        scratch, scratch_bytes, nullptr,
                                         static_cast<cudaStream_t>(stream));
 }
 
