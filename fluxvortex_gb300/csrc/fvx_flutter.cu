@@ -25,7 +25,7 @@
 // amplifies a rounding difference anywhere upstream.  64 airspeeds, 20 chords,
 // mixed precision: 104.3 ms with the loads' bound rings on one warp, both CTAs
 // forming the whole AIC, one thread searching the pivots and converting rows,
-// and eleven FP64 operations and conversions per particle; 37.5 ms so.
+// and eleven FP64 operations and conversions per particle; 31.1 ms so.
 // Reference: src/fluxvortex/aeroelastic_solver.py:68-221 and beam_fe.py:231-351
 // around PteraSoftware's ring-vortex UVLM; the PteraSoftware-free model is
 // described in fluxvortex_gb300/flutter.py.
@@ -49,11 +49,16 @@ constexpr double kC = -0.07957747154594767;  // -1/(4 pi): particle strength sca
 constexpr int kLegItems = 256;  // (point, ring) pairs per pass of the loads' leg terms
 constexpr int kLegStride = 17;  // doubles per pair: 4 legs of (c4, r3), one of padding
 
-// A wake ring for the mixed-precision sweep: corners in FP64 and as the sum of
-// two floats, and the leg constants rounded once here instead of per point.
+// An FP64 number as three floats, exactly (24 + 24 + 5 bits).
+struct Parts {
+  float h, l, r;
+};
+
+// A wake ring for the mixed-precision sweep: corners in FP64 and in parts
+// (split_f32), and the leg constants rounded once here instead of per point.
 struct RingF32 {
   double c[4][3];
-  float hi[4][3], lo[4][3];
+  Parts p[4][3];
   float c2[4], tol[4];
   float c1;
   int valid;
@@ -76,10 +81,14 @@ struct Smem {
   double W[kMaxRows + 1][kMaxNS + 1][3];
   double wgam[kMaxRows][kMaxNS], wage[kMaxRows];
   double d[kMaxDof], v[kMaxDof], a[kMaxDof], F[kMaxDof], feff[kMaxDof], gd[kMaxDof];
-  double tile[kTile][8];  // staged particles: x y z | a' (C-scaled) | sigma^2, 2.5 sigma^2
-  // mixed precision: x y z as two floats each, a', sigma^2, 2.5 sigma^2
-  __align__(16) float tile_hi[kTile][4], tile_lo[kTile][4], tile_a[kTile][4];
+  // two tiles of staged particles: x y z | a' (C-scaled) | sigma^2, 2.5 sigma^2
+  double tile[2 * kTile][8];
+  // mixed precision: the parts of x y z with sigma^2 and 2.5 sigma^2, and a'
+  __align__(16) float tile_h[2 * kTile][4], tile_l[2 * kTile][4], tile_r[2 * kTile][4],
+      tile_a[2 * kTile][4];
+  double newmark[6];  // a0 .. a5 of the Newmark step
   double legs[kLegItems * kLegStride];
+  double udiag_inv[kMaxP];  // reciprocals of U's diagonal
   int perm[kMaxP];
   int lu_ok;
   double red[8];
@@ -87,29 +96,37 @@ struct Smem {
 
 static_assert(sizeof(Smem) <= 227 * 1024, "the environment's state must fit shared memory");
 
-// float(x - y) of FP64 x and y, each given as hi + lo as well (hi = float(x),
-// lo = float(x - hi)): the float of the rounded FP64 difference, bit for bit,
-// without the FP64 pipe (one subtraction and one conversion cost it about 130
-// FP32 issue slots).  hi and lo differ from x by 2^-48 |x| at most; the exact
-// difference of the his (two_sum of Knuth) plus that of the los is within
-// 2^-44 (|x| + |y|) of x - y, FP64's own rounding included.  Where adding and
+__device__ __forceinline__ Parts split_f32(double x) {
+  Parts p;
+  p.h = static_cast<float>(x);
+  const double y = x - static_cast<double>(p.h);
+  p.l = static_cast<float>(y);
+  p.r = static_cast<float>(y - static_cast<double>(p.l));
+  return p;
+}
+
+// float(x - y) of FP64 x and y in parts: the float of the rounded FP64
+// difference, bit for bit, without the FP64 pipe (one subtraction and one
+// conversion cost it about 130 FP32 issue slots).  x - y is h + l exactly, h the
+// leading parts' rounded difference and l the error of that (Knuth's two_sum)
+// plus the differences of the others; l rounds four times, by 2^-24 of at most
+// |e| + |a| + |b| each, and FP64's own rounding is 2^-53 |h|.  Where adding and
 // taking off that bound rounds to the same float, that float is the answer;
-// else (2^-20 |x| / |x - y| of the pairs) `same` is cleared and the caller
-// takes the FP64 way.
-__device__ __forceinline__ float diff_f32(float xh, float xl, float yh, float yl, bool& same) {
-  const float h = xh - yh;
-  const float bb = h - xh;
-  const float e = (xh - (h - bb)) - (yh + bb);
-  const float l = e + (xl - yl);
-  const float t = fabsf(xh) + fabsf(yh);
-  const float r0 = h + fmaf(t, -5.684341886080802e-14f, l);  // 2^-44
-  const float r1 = h + fmaf(t, 5.684341886080802e-14f, l);
+// else (about 2^-20 of the pairs) `same` is cleared and the caller takes the
+// FP64 way.  Equal coordinates (particles on a point's span station) give zero
+// bounds and a zero.
+__device__ __forceinline__ float diff_f32(const Parts& x, const Parts& y, bool& same) {
+  const float h = x.h - y.h;
+  const float bb = h - x.h;
+  const float e = (x.h - (h - bb)) - (y.h + bb);
+  const float a = x.l - y.l, b = x.r - y.r;
+  const float l = e + (a + b);
+  const float w = fmaf(fabsf(h), 2.220446049250313e-16f,                            // 2^-52
+                       (fabsf(e) + (fabsf(a) + fabsf(b))) * 2.384185791015625e-07f);  // 2^-22
+  const float r0 = h + (l - w);
+  const float r1 = h + (l + w);
   same = same && r0 == r1;
   return r0;
-}
-__device__ __forceinline__ void split_f32(double x, float& hi, float& lo) {
-  hi = static_cast<float>(x);
-  lo = static_cast<float>(x - static_cast<double>(hi));
 }
 
 // Deformed vertices and their velocities from the beam state in S.d / S.v.
@@ -148,15 +165,24 @@ __device__ __forceinline__ void quarter(const double (*V)[3], int nc, int ns, in
   }
 }
 
+// (geometry on the first warps, ring records on the next)
 __device__ void build_lattice(Smem& S, const FlutterParams& p) {
-  const int P = p.nc * p.ns, s1 = p.ns + 1;
-  for (int k = threadIdx.x; k < P; k += blockDim.x) {
+  const int P = p.nc * p.ns, s1 = p.ns + 1, w = (P + 31) & ~31;
+  for (int t = threadIdx.x; t < 2 * w; t += blockDim.x) {
+    const int k = t < w ? t : t - w;
+    if (k >= P) continue;
     const int i = k / p.ns, j = k % p.ns;
-    double fl[3], fr[3], br[3], bl[3], vfl[3], vfr[3];
+    double fl[3], fr[3];
     quarter(S.verts, p.nc, p.ns, i, j, fl);
     quarter(S.verts, p.nc, p.ns, i, j + 1, fr);
-    quarter(S.verts, p.nc, p.ns, i + 1, j + 1, br);
-    quarter(S.verts, p.nc, p.ns, i + 1, j, bl);
+    if (t >= w) {
+      double br[3], bl[3];
+      quarter(S.verts, p.nc, p.ns, i + 1, j + 1, br);
+      quarter(S.verts, p.nc, p.ns, i + 1, j, bl);
+      seg::prep_vortex<FVX_LEGS_RING, true>(S.bound[k], br, fr, fl, bl, 1.0, p.rc0, 0.0, p.nu);
+      continue;
+    }
+    double vfl[3], vfr[3];
     quarter(S.vvel, p.nc, p.ns, i, j, vfl);
     quarter(S.vvel, p.nc, p.ns, i, j + 1, vfr);
     const double* v00 = S.verts[i * s1 + j];
@@ -189,7 +215,6 @@ __device__ void build_lattice(Smem& S, const FlutterParams& p) {
     S.normal[k][1] = cy / nrm;
     S.normal[k][2] = cz / nrm;
     S.area[k] = 0.5 * nrm;
-    seg::prep_vortex<FVX_LEGS_RING, true>(S.bound[k], br, fr, fl, bl, 1.0, p.rc0, 0.0, p.nu);
   }
 }
 
@@ -289,7 +314,7 @@ __device__ __forceinline__ void prep_ring_f32(RingF32& Q, const double* br, cons
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       Q.c[c][k] = R.c[c][k];
-      split_f32(R.c[c][k], Q.hi[c][k], Q.lo[c][k]);
+      Q.p[c][k] = split_f32(R.c[c][k]);
     }
     Q.c2[c] = static_cast<float>(R.c2[c]);
     Q.tol[c] = static_cast<float>(R.tol[c]);
@@ -298,10 +323,10 @@ __device__ __forceinline__ void prep_ring_f32(RingF32& Q, const double* br, cons
   Q.valid = R.valid;
 }
 
-// A target point of the wake induction, in FP64 and as two floats.
+// A target point of the wake induction, in FP64 and in parts.
 struct Point {
   double p[3];
-  float hi[3], lo[3];
+  Parts s[3];
 };
 
 // One wake ring at a point in FP32 on the FP64 offsets' floats (the
@@ -314,7 +339,7 @@ __device__ __forceinline__ void ring_velocity_f32(const RingF32& R, const Point&
   for (int c = 0; c < 4; ++c)
 #pragma unroll
     for (int k = 0; k < 3; ++k)
-      d[c][k] = diff_f32(R.hi[c][k], R.lo[c][k], P.hi[k], P.lo[k], same);
+      d[c][k] = diff_f32(R.p[c][k], P.s[k], same);
   if (!same) {
 #pragma unroll
     for (int c = 0; c < 4; ++c)
@@ -368,7 +393,7 @@ __device__ void wake_induction(Smem& S, const FlutterParams& p, const FlutterSta
     if constexpr (F32) {
       for (int k = 0; k < 3; ++k) {
         pt.p[k] = q[k];
-        split_f32(q[k], pt.hi[k], pt.lo[k]);
+        pt.s[k] = split_f32(q[k]);
       }
     }
   }
@@ -394,11 +419,13 @@ __device__ void wake_induction(Smem& S, const FlutterParams& p, const FlutterSta
   const double* pa = st.palp + static_cast<int64_t>(env) * Pm * 3;
   const double* ps = st.psig + static_cast<int64_t>(env) * Pm;
   float hx = 0.f, hy = 0.f, hz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
-  for (int t0 = crank * kTile; t0 < count; t0 += kTile * CL) {
-    const int nt = min(kTile, count - t0);
+  // this CTA's tiles, two at a time: a thread per particle stages them
+  for (int t0 = crank * kTile; t0 < count; t0 += 2 * kTile * CL) {
     __syncthreads();
-    for (int e = threadIdx.x; e < nt; e += blockDim.x) {
-      const int q = (head + t0 + e) % Pm;
+    for (int e = threadIdx.x; e < 2 * kTile; e += blockDim.x) {
+      const int at = t0 + (e / kTile) * kTile * CL + e % kTile;
+      if (at >= count) continue;
+      const int q = (head + at) % Pm;
       const double s = ps[q];
       S.tile[e][0] = pp[3 * q];
       S.tile[e][1] = pp[3 * q + 1];
@@ -406,11 +433,14 @@ __device__ void wake_induction(Smem& S, const FlutterParams& p, const FlutterSta
       if constexpr (F32) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          split_f32(S.tile[e][k], S.tile_hi[e][k], S.tile_lo[e][k]);
+          const Parts w = split_f32(S.tile[e][k]);
+          S.tile_h[e][k] = w.h;
+          S.tile_l[e][k] = w.l;
+          S.tile_r[e][k] = w.r;
           S.tile_a[e][k] = static_cast<float>(kC * pa[3 * q + k]);
         }
-        S.tile_hi[e][3] = static_cast<float>(s * s);
-        S.tile_lo[e][3] = static_cast<float>(2.5 * s * s);
+        S.tile_h[e][3] = static_cast<float>(s * s);
+        S.tile_l[e][3] = static_cast<float>(2.5 * s * s);
       } else {
         S.tile[e][3] = kC * pa[3 * q];
         S.tile[e][4] = kC * pa[3 * q + 1];
@@ -421,46 +451,77 @@ __device__ void wake_induction(Smem& S, const FlutterParams& p, const FlutterSta
     }
     __syncthreads();
     if (!active) continue;
-    for (int e = sl; e < nt; e += slices) {
-      const double* s = S.tile[e];
+    for (int h = 0; h < 2; ++h) {
+      const int nt = min(kTile, count - t0 - h * kTile * CL);
+      const int e1 = h * kTile + nt;
       if constexpr (F32) {
-        // FP32 pair arithmetic on the FP64 offset's float, compensated sums
-        const float4 sh = *reinterpret_cast<const float4*>(S.tile_hi[e]);
-        const float4 sl4 = *reinterpret_cast<const float4*>(S.tile_lo[e]);
-        const float4 av = *reinterpret_cast<const float4*>(S.tile_a[e]);
-        bool same = true;
-        float dx = diff_f32(pt.hi[0], pt.lo[0], sh.x, sl4.x, same);
-        float dy = diff_f32(pt.hi[1], pt.lo[1], sh.y, sl4.y, same);
-        float dz = diff_f32(pt.hi[2], pt.lo[2], sh.z, sl4.z, same);
-        if (!same) {
-          dx = static_cast<float>(px - s[0]);
-          dy = static_cast<float>(py - s[1]);
-          dz = static_cast<float>(pz - s[2]);
+        // FP32 pair arithmetic on the FP64 offset's float, compensated sums;
+        // two particles side by side (two warps per quarter leave a single
+        // particle's chain exposed), added in order
+        for (int e = h * kTile + sl; e < e1; e += 2 * slices) {
+          const int pair_n = e + slices < e1 ? 2 : 1;
+          float d[2][3], s2[2], k2[2], al[2][3], u[2][3];
+          bool same = true;
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            const int em = m < pair_n ? e + m * slices : e;
+            const float4 sh = *reinterpret_cast<const float4*>(S.tile_h[em]);
+            const float4 so = *reinterpret_cast<const float4*>(S.tile_l[em]);
+            const float4 sr = *reinterpret_cast<const float4*>(S.tile_r[em]);
+            const float4 av = *reinterpret_cast<const float4*>(S.tile_a[em]);
+            d[m][0] = diff_f32(pt.s[0], Parts{sh.x, so.x, sr.x}, same);
+            d[m][1] = diff_f32(pt.s[1], Parts{sh.y, so.y, sr.y}, same);
+            d[m][2] = diff_f32(pt.s[2], Parts{sh.z, so.z, sr.z}, same);
+            s2[m] = sh.w;
+            k2[m] = so.w;
+            al[m][0] = av.x;
+            al[m][1] = av.y;
+            al[m][2] = av.z;
+          }
+          if (!same) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+              const double* s = S.tile[m < pair_n ? e + m * slices : e];
+#pragma unroll
+              for (int c = 0; c < 3; ++c) d[m][c] = static_cast<float>(pt.p[c] - s[c]);
+            }
+          }
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            const float r2 = d[m][0] * d[m][0] + d[m][1] * d[m][1] + d[m][2] * d[m][2];
+            float f, fpr;
+            pair::core_f32<FVX_KERNEL_WINCKELMANS, false>(r2, s2[m], k2[m], f, fpr);
+            const float ex = f * d[m][0], ey = f * d[m][1], ez = f * d[m][2];
+            u[m][0] = ey * al[m][2] - ez * al[m][1];
+            u[m][1] = ez * al[m][0] - ex * al[m][2];
+            u[m][2] = ex * al[m][1] - ey * al[m][0];
+          }
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            if (m >= pair_n) break;
+            float t = hx + u[m][0];
+            lx += (hx - t) + u[m][0];
+            hx = t;
+            t = hy + u[m][1];
+            ly += (hy - t) + u[m][1];
+            hy = t;
+            t = hz + u[m][2];
+            lz += (hz - t) + u[m][2];
+            hz = t;
+          }
         }
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        float f, fpr;
-        pair::core_f32<FVX_KERNEL_WINCKELMANS, false>(r2, sh.w, sl4.w, f, fpr);
-        const float ax = av.x, ay = av.y, az = av.z;
-        const float ex = f * dx, ey = f * dy, ez = f * dz;
-        const float ux = ey * az - ez * ay, uy = ez * ax - ex * az, uz = ex * ay - ey * ax;
-        float t = hx + ux;
-        lx += (hx - t) + ux;
-        hx = t;
-        t = hy + uy;
-        ly += (hy - t) + uy;
-        hy = t;
-        t = hz + uz;
-        lz += (hz - t) + uz;
-        hz = t;
       } else {
-        const double dx = px - s[0], dy = py - s[1], dz = pz - s[2];
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        double f, fpr;
-        pair::core_f64<FVX_KERNEL_WINCKELMANS, false>(r2, s[6], s[7], f, fpr);
-        const double ex = f * dx, ey = f * dy, ez = f * dz;
-        vx += ey * s[5] - ez * s[4];
-        vy += ez * s[3] - ex * s[5];
-        vz += ex * s[4] - ey * s[3];
+        for (int e = h * kTile + sl; e < e1; e += slices) {
+          const double* s = S.tile[e];
+          const double dx = px - s[0], dy = py - s[1], dz = pz - s[2];
+          const double r2 = dx * dx + dy * dy + dz * dz;
+          double f, fpr;
+          pair::core_f64<FVX_KERNEL_WINCKELMANS, false>(r2, s[6], s[7], f, fpr);
+          const double ex = f * dx, ey = f * dy, ez = f * dz;
+          vx += ey * s[5] - ez * s[4];
+          vy += ez * s[3] - ex * s[5];
+          vz += ex * s[4] - ey * s[3];
+        }
       }
     }
   }
@@ -582,12 +643,27 @@ __device__ bool lu_solve(Smem& S, int P) {
       const double u0 = j0 <= P ? S.A[pp][j0] : 0.0;
       const double u1 = j1 <= P ? S.A[pp][j1] : 0.0;
       const double u2 = j2 <= P ? S.A[pp][j2] : 0.0;
-      for (int i = k + 1 + warp; i < P; i += nw) {
-        const double l = __shfl_sync(0xffffffffu, i < 32 ? m0 : m1, i & 31);
-        const int r = __shfl_sync(0xffffffffu, i < 32 ? p0 : p1, i & 31);
-        if (j0 <= P) S.A[r][j0] -= l * u0;
-        if (j1 <= P) S.A[r][j1] -= l * u1;
-        if (j2 <= P) S.A[r][j2] -= l * u2;
+      // four rows at a time, loads first: a row's store would hold up the next
+      // row's loads
+      for (int i0 = k + 1 + warp; i0 < P; i0 += 4 * nw) {
+        double l[4], a0[4], a1[4], a2[4];
+        double* row[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const int i = min(i0 + m * nw, P - 1);
+          l[m] = __shfl_sync(0xffffffffu, i < 32 ? m0 : m1, i & 31);
+          row[m] = S.A[__shfl_sync(0xffffffffu, i < 32 ? p0 : p1, i & 31)];
+          a0[m] = j0 <= P ? row[m][j0] : 0.0;
+          a1[m] = j1 <= P ? row[m][j1] : 0.0;
+          a2[m] = j2 <= P ? row[m][j2] : 0.0;
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          if (i0 + m * nw >= P) break;
+          if (j0 <= P) row[m][j0] = a0[m] - l[m] * u0;
+          if (j1 <= P) row[m][j1] = a1[m] - l[m] * u1;
+          if (j2 <= P) row[m][j2] = a2[m] - l[m] * u2;
+        }
       }
       asm volatile("bar.sync 1, %0;" ::"r"(32 * nw) : "memory");
     }
@@ -596,15 +672,27 @@ __device__ bool lu_solve(Smem& S, int P) {
       if (lane + 32 < P) S.perm[lane + 32] = p1;
       if (lane == 0) S.lu_ok = ok;
       __syncwarp();
-      // back substitution, each row's terms in order: one thread's chain
+      // back substitution, each row's terms in order: one thread's chain.  The
+      // diagonals' correctly rounded reciprocals are formed side by side first;
+      // q = s r and one step q + (s - q d) r is then the correctly rounded s / d
+      // (Markstein, 1990), at a third of a division's latency.
+      if (lane < P) S.udiag_inv[lane] = 1.0 / S.A[p0][lane];
+      if (lane + 32 < P) S.udiag_inv[lane + 32] = 1.0 / S.A[p1][lane + 32];
+      __syncwarp();
       if (ok && lane == 0) {
         for (int i = P - 1; i >= 0; --i) {
           const double* row = S.A[S.perm[i]];
           double s = row[P];
-          const double diag = row[i];
+          const double diag = row[i], r = S.udiag_inv[i];
 #pragma unroll 4
           for (int j = i + 1; j < P; ++j) s -= row[j] * S.gam[j];
-          S.gam[i] = s / diag;
+          const double q = s * r;
+          const double rem = fma(-q, diag, s);
+          // (a quotient or remainder at the ends of the range: the division)
+          const int h = __double2hiint(q) & 0x7ff00000;
+          S.gam[i] = h > (200 << 20) && h < (1800 << 20) && fabs(diag) < 1e200 && fabs(diag) > 1e-200
+                         ? fma(rem, r, q)
+                         : s / diag;
         }
       }
     }
@@ -649,6 +737,15 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
     S.wgam[k / p.ns][k % p.ns] = st.wgam[env * (p.n_keep + 1) * p.ns + k];
   for (int k = threadIdx.x; k < R; k += blockDim.x) S.wage[k] = st.wage[env * (p.n_keep + 1) + k];
   for (int k = threadIdx.x; k < P; k += blockDim.x) S.gprev[k] = st.gprev[env * P + k];
+  if (threadIdx.x == 0) {
+    const double b = p.beta, g = p.gamma;
+    S.newmark[0] = 1.0 / (b * dt * dt);
+    S.newmark[1] = 1.0 / (b * dt);
+    S.newmark[2] = 1.0 / (2.0 * b) - 1.0;
+    S.newmark[3] = g / (b * dt);
+    S.newmark[4] = g / b - 1.0;
+    S.newmark[5] = dt * (g / (2.0 * b) - 1.0);
+  }
   int has_prev = st.has_prev[env];
   int head = st.phead[env], count = st.pcount[env];
   __syncthreads();
@@ -669,7 +766,7 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
       build_lattice(S, p);
     }
     // the wake's rings on the threads after the lattice's warps
-    const int t0 = (P + 31) & ~31;
+    const int t0 = (2 * ((P + 31) & ~31)) % blockDim.x;
     for (int k = threadIdx.x >= t0 ? threadIdx.x - t0 : threadIdx.x + blockDim.x - t0;
          k < R * p.ns; k += blockDim.x) {
       const int r = k / p.ns, j = k % p.ns;
@@ -815,9 +912,9 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
       S.F[k] = f;
     }
     // 7. Newmark: F_eff = F + M (a0 d + a1 v + a2 a) + C (a3 d + a4 v + a5 a)
-    const double b = p.beta, g = p.gamma;
-    const double a0 = 1.0 / (b * dt * dt), a1 = 1.0 / (b * dt), a2 = 1.0 / (2.0 * b) - 1.0;
-    const double a3 = g / (b * dt), a4 = g / b - 1.0, a5 = dt * (g / (2.0 * b) - 1.0);
+    const double g = p.gamma;
+    const double a0 = S.newmark[0], a1 = S.newmark[1], a2 = S.newmark[2], a3 = S.newmark[3],
+                 a4 = S.newmark[4], a5 = S.newmark[5];
     double* xm = torque + kMaxNS;
     double* xc = xm + kMaxDof;
     for (int c = threadIdx.x; c < nf && couple; c += blockDim.x) {
@@ -878,20 +975,21 @@ __global__ void __launch_bounds__(512) sweep_kernel(FlutterParams p, FlutterStat
       pp[3 * q + 1] += uy * dt;
       pp[3 * q + 2] += uz * dt;
     }
-    // shift rows down by one (new row 0), from the back so nothing is overwritten early
-    for (int r = R; r >= 0; --r) {
-      for (int k = threadIdx.x; k < s1; k += blockDim.x) {
-        S.W[r + 1][k][0] = S.W[r][k][0] + ux * dt;
-        S.W[r + 1][k][1] = S.W[r][k][1] + uy * dt;
-        S.W[r + 1][k][2] = S.W[r][k][2] + uz * dt;
+    // shift rows down by one (new row 0), from the back so nothing is overwritten
+    // early: a thread per coordinate of a column, strip or age
+    for (int k = threadIdx.x; k < 3 * s1 + p.ns + 1; k += blockDim.x) {
+      if (k < 3 * s1) {
+        const int j = k / 3, c = k % 3;
+        const double step_c = (c == 0 ? ux : (c == 1 ? uy : uz)) * dt;
+        for (int r = R; r >= 0; --r) S.W[r + 1][j][c] = S.W[r][j][c] + step_c;
+      } else if (k < 3 * s1 + p.ns) {
+        const int j = k - 3 * s1;
+        for (int r = R - 1; r >= 0; --r) S.wgam[r + 1][j] = S.wgam[r][j];
+      } else {
+        for (int r = R - 1; r >= 0; --r) S.wage[r + 1] = S.wage[r] + dt;
       }
-      __syncthreads();
     }
-    for (int r = R - 1; r >= 0; --r) {
-      for (int k = threadIdx.x; k < p.ns; k += blockDim.x) S.wgam[r + 1][k] = S.wgam[r][k];
-      if (threadIdx.x == 0) S.wage[r + 1] = S.wage[r] + dt;
-      __syncthreads();
-    }
+    __syncthreads();
     for (int k = threadIdx.x; k < s1; k += blockDim.x) {
       if (ref)
         trailing_edge_reference(S, p, S.W[0][k], k);

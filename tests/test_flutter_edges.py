@@ -1,6 +1,6 @@
 """The flutter kernel at the edges of its splits: panel counts on both sides of
 a warp and of the cluster's row shares, threads below three per point, particle
-stores smaller than one step's edges; and the mixed-precision offset (two floats
+stores smaller than one step's edges; and the mixed-precision offset (three floats
 per coordinate) against the rounded FP64 difference it stands for."""
 import numpy as np
 import pytest
@@ -29,36 +29,43 @@ def test_shapes_match_oracle(cuda, nc, ns, threads, envs, store):
 
 
 def _split(x):
-    hi = x.astype(np.float32)
-    return hi, (x - hi.astype(np.float64)).astype(np.float32)
+    h = x.astype(np.float32)
+    y = x - h.astype(np.float64)
+    lo = y.astype(np.float32)
+    return h, lo, (y - lo.astype(np.float64)).astype(np.float32)
 
 
-@pytest.mark.parametrize("kind", ["apart", "near", "ties", "equal"])
-def test_two_float_difference_is_the_rounded_fp64_difference(kind):
+@pytest.mark.parametrize("kind", ["apart", "near", "ties", "floats", "equal"])
+def test_difference_in_parts_is_the_rounded_fp64_difference(kind):
     """The kernel's diff_f32 restated in NumPy: wherever it does not send the
     pair to the FP64 way, its float is that of the FP64 difference."""
     rng = np.random.default_rng(17)
     n = 400000
+    f32, f64 = np.float32, np.float64
     x = rng.uniform(-20, 20, n)
     y = rng.uniform(-20, 20, n)
     if kind == "near":
         y = x + rng.standard_normal(n) * 2.0 ** -rng.integers(0, 50, n)
     elif kind == "ties":
-        f = (x - y).astype(np.float32)
-        mid = 0.5 * (f.astype(np.float64) + np.nextafter(f, np.float32(np.inf)))
+        f = (x - y).astype(f32)
+        mid = 0.5 * (f.astype(f64) + np.nextafter(f, f32(np.inf)))
         y = np.nextafter(x - mid, np.where(rng.random(n) < 0.5, np.inf, -np.inf))
+    elif kind == "floats":
+        x = x.astype(f32).astype(f64)
+        y = x * (1.0 + 2.0 ** -rng.integers(8, 52, n).astype(f64))
     elif kind == "equal":
-        x = x.astype(np.float32).astype(np.float64)
-        y = x * (1.0 + 2.0 ** -rng.integers(8, 52, n).astype(np.float64))
-    (xh, xl), (yh, yl) = _split(x), _split(y)
+        y = x.copy()
+    (xh, xl, xr), (yh, yl, yr) = _split(x), _split(y)
     h = xh - yh
     bb = h - xh
-    low = ((xh - (h - bb)) - (yh + bb)) + (xl - yl)
-    t = (np.abs(xh) + np.abs(yh)).astype(np.float64) * 2.0 ** -44   # fma: one rounding
-    r0 = h + (low.astype(np.float64) - t).astype(np.float32)
-    r1 = h + (low.astype(np.float64) + t).astype(np.float32)
-    ref = (x - y).astype(np.float32)
+    e = (xh - (h - bb)) - (yh + bb)
+    a, b = xl - yl, xr - yr
+    low = e + (a + b)
+    t = (np.abs(e) + (np.abs(a) + np.abs(b))) * f32(2.0 ** -22)
+    w = (np.abs(h).astype(f64) * 2.0 ** -52 + t.astype(f64)).astype(f32)   # fma: one rounding
+    r0, r1 = h + (low - w), h + (low + w)
+    ref = (x - y).astype(f32)
     same = r0 == r1
     assert np.array_equal(r0[same], ref[same])
-    if kind == "apart":
+    if kind in ("apart", "equal"):
         assert same.mean() > 0.9999
