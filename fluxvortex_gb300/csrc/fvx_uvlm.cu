@@ -25,6 +25,8 @@
 // the host only sequences launches.
 #include <cooperative_groups.h>
 
+#include <utility>
+
 #include "fvx_common.cuh"
 #include "fvx_segment_math.cuh"
 
@@ -411,50 +413,125 @@ __global__ void __launch_bounds__(kLuThreads) lu_solve_kernel(int P, int T, doub
 // The same solve on a cluster of kLuCtas CTAs (systems with P <= kLuClusterMaxP):
 // one SM's FP64 pipe bounds the single-CTA form, so the columns are dealt out
 // cyclically (column j to CTA j mod kLuCtas, kept whole in its shared memory).
-// Step k: the owner of column k searches its pivot, swaps and forms the
-// multipliers in its own shared memory; after one cluster barrier every CTA
-// reads them (distributed shared memory), swaps rows k and piv in its
-// columns, updates its copy of the right-hand side and its trailing columns.
-// The multipliers alternate between two buffers, so one barrier per step
-// suffices (the owner of step k + 2 writes only after every CTA has passed
-// step k + 1's barrier, i.e. finished step k).  Every element sees the same
-// operations in the same order as the single-CTA form, so the factors and the
-// solution are the same.  The upper triangle is then gathered, packed, into
-// CTA 0, which back-substitutes.
+// What a step costs is its chain -- pivot, reciprocal, multipliers, their way to
+// the other CTAs -- so that is all that stands between two steps: the owner of
+// column k + 1 brings that column up to date first, finds its pivot by integer
+// comparisons (one warp), forms the multipliers, writes them into every CTA's
+// shared memory and arrives at the cluster barrier; everybody's other columns
+// follow while the barrier fills.  Rows are permuted by index; every element sees
+// the operations of the single-CTA form in its order, so the factors and the
+// solution are the same.  The multipliers
+// go round three buffers: step k + 3's writer has passed barrier k + 2, at which
+// every thread arrived after its last use of step k's.
+// 120 unknowns: 199 us, 1.7 us a step (3.2 us while every step's pivot, swap,
+// division and the reading back of the multipliers stood in the chain); the
+// replayed solve takes 51 us (125 us with two barriers a column).
 namespace cg = cooperative_groups;
 constexpr int kLuCtas = 8;
 constexpr int kLuClusterThreads = 256;
 constexpr int kLuClusterMaxP = 192;  // packed U, P (P + 1) / 2 doubles, in CTA 0
-static_assert(kLuClusterThreads >= kLuClusterMaxP, "the replayed solve takes one row per thread");
+static_assert(kLuClusterThreads >= kLuClusterMaxP, "one row per thread");
 
-// doubles of one system's factorisation workspace: multipliers P x P, pivots
-// P, packed U P (P + 1) / 2
+// doubles of one system's factorisation workspace: multipliers P x P (row k:
+// step k's, by the rows' places in A), the permutation P (the row of A that
+// became row i), packed U P (P + 1) / 2
 __host__ __device__ constexpr int64_t lu_workspace_doubles(int P) {
   return static_cast<int64_t>(P) * P + P + static_cast<int64_t>(P) * (P + 1) / 2;
 }
 
-// Back substitution with the packed upper triangle (column j's rows 0..j at
-// j (j + 1) / 2), x in place; every thread of the CTA takes part.
-__device__ __forceinline__ void back_substitute(int P, const double* s_u, double* s_x, int tid,
-                                                int NT) {
-  for (int k = P - 1; k >= 0; --k) {
-    const int base = k * (k + 1) / 2;
-    const double xk = s_x[k] / s_u[base + k];
-    for (int r = tid; r < k; r += NT) s_x[r] -= s_u[base + r] * xk;
+__device__ __forceinline__ int packed_u(int j) { return j * (j + 1) / 2; }  // column j's row 0
+
+// s / d from the correctly rounded reciprocal r of d: q = s r and one step
+// q + (s - q d) r is the correctly rounded quotient (Markstein, 1990), at a third
+// of a division's latency and 3 of its 7 FP64 operations.  Quotients and divisors
+// at the ends of the range (zeros, infinities and NaNs among them) are divided.
+__device__ __forceinline__ double quotient(double s, double d, double r) {
+  const double q = s * r;
+  const int h = __double2hiint(q) & 0x7ff00000, hd = __double2hiint(d) & 0x7ff00000;
+  const bool mid = h > (200 << 20) && h < (1800 << 20) && hd > (400 << 20) && hd < (1600 << 20);
+  return mid ? fma(fma(-q, d, s), r, q) : s / d;
+}
+
+// Back substitution with the packed upper triangle, x in place, by the whole
+// CTA, 32 columns at a time from the last: a warp solves their triangle with
+// its rows in registers, then a thread per row above subtracts their share.
+// Every row sees its columns in descending order, as in the single-CTA form.
+__device__ void back_substitute(int P, const double* s_u, double* s_x, int tid) {
+  const int lane = tid & 31;
+  for (int k0 = (P - 1) / 32 * 32; k0 >= 0; k0 -= 32) {
+    const int n = min(32, P - k0);
+    if (tid < 32) {
+      double u[32];
+      double x = 0.0, d = 1.0;
+      if (lane < n) {
+        d = s_u[packed_u(k0 + lane) + k0 + lane];
+        x = s_x[k0 + lane];
+      }
+      const double r = 1.0 / d;
+#pragma unroll
+      for (int c = 0; c < 32; ++c)
+        u[c] = c < n && lane < c ? s_u[packed_u(k0 + c) + k0 + lane] : 0.0;
+#pragma unroll
+      for (int c = 31; c >= 0; --c) {
+        if (c >= n) continue;
+        if (lane == c) x = quotient(x, d, r);
+        const double xc = __shfl_sync(0xffffffffu, x, c);
+        if (lane < c) x -= u[c] * xc;
+      }
+      if (lane < n) s_x[k0 + lane] = x;
+    }
     __syncthreads();
-    if (tid == 0) s_x[k] = xk;
+    if (tid < k0) {
+      double x = s_x[tid];
+      for (int c = n - 1; c >= 0; --c) x -= s_u[packed_u(k0 + c) + tid] * s_x[k0 + c];
+      s_x[tid] = x;
+    }
     __syncthreads();
   }
 }
 
+// The pivot of a column among logical rows k..P-1 (perm[i]: where row i is):
+// largest magnitude, first row on ties, by integer comparisons of the words
+// (NaNs count as zero); one warp, every lane returns the row, or P if all are zero.
+__device__ __forceinline__ int lu_warp_pivot(const double* col, const int* perm, int k, int P) {
+  constexpr int kRows = kLuClusterMaxP / 32;
+  const int lane = threadIdx.x & 31;
+  unsigned h[kRows], l[kRows];
+  unsigned hm = 0;
+#pragma unroll
+  for (int m = 0; m < kRows; ++m) {
+    const int i = k + lane + 32 * m;
+    h[m] = l[m] = 0;
+    if (i < P) {
+      const double v = col[perm[i]];
+      h[m] = __double2hiint(v) & 0x7fffffff;
+      l[m] = __double2loint(v);
+      if (h[m] > 0x7ff00000u || (h[m] == 0x7ff00000u && l[m] != 0)) h[m] = l[m] = 0;
+    }
+    hm = max(hm, h[m]);
+  }
+  hm = __reduce_max_sync(0xffffffffu, hm);
+  unsigned lm = 0;
+#pragma unroll
+  for (int m = 0; m < kRows; ++m)
+    if (h[m] == hm) lm = max(lm, l[m]);
+  lm = __reduce_max_sync(0xffffffffu, lm);
+  if ((hm | lm) == 0) return P;
+  int piv = P;
+#pragma unroll
+  for (int m = kRows - 1; m >= 0; --m)
+    if (k + lane + 32 * m < P && h[m] == hm && l[m] == lm) piv = k + lane + 32 * m;
+  return __reduce_min_sync(0xffffffffu, piv);
+}
+
 // Dynamic shared memory per CTA: panel[ceil(P/kLuCtas)][P] (column-major),
-// s_l[2][P], s_x[P], packed U[P (P + 1) / 2] (used in CTA 0).
-// FACTOR: the factorisation alone, no right-hand side: step k's multipliers
-// (as formed at step k), its pivot and the packed upper triangle go to the
-// workspace W (lu_workspace), from which lu_solve_factored_kernel replays the
-// same elimination on a right-hand side later (same operations, same order:
-// the same solution bit for bit), so the factorisation can run while the
-// right-hand side is still being formed.
+// l[3][P], x[P], packed U[P (P + 1) / 2] (x and U used in CTA 0).
+// FACTOR: the factorisation alone, no right-hand side: the multipliers, the
+// permutation and the packed upper triangle go to the workspace W
+// (lu_workspace_doubles), from which lu_solve_factored_kernel replays the same
+// elimination on a right-hand side later (same operations, same order: the same
+// solution bit for bit), so the factorisation can run while the right-hand
+// side is still being formed.
 template <bool FACTOR>
 __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThreads)
     lu_cluster_kernel(int P, double* __restrict__ A, double* __restrict__ b,
@@ -465,8 +542,6 @@ __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThre
   const int sys = blockIdx.x / kLuCtas;
   double* a = A + static_cast<int64_t>(sys) * P * P;
   double* xg = FACTOR ? nullptr : b + static_cast<int64_t>(sys) * P;
-  // workspace of this system: multipliers L[k][r] (row k: step k's, r > k),
-  // pivots (as doubles), packed U
   double* wl = FACTOR ? W + static_cast<int64_t>(sys) * lu_workspace_doubles(P) : nullptr;
   double* wp = FACTOR ? wl + static_cast<int64_t>(P) * P : nullptr;
   double* wu = FACTOR ? wp + P : nullptr;
@@ -474,132 +549,118 @@ __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThre
   const int ncol = rank < P ? (P - rank + kLuCtas - 1) / kLuCtas : 0;
   double* panel = lc_smem;
   double* s_l = panel + static_cast<size_t>(ncmax) * P;
-  double* s_x = s_l + 2 * P;
+  double* s_x = s_l + 3 * P;
   double* s_u = s_x + P;
-  __shared__ double s_wv[kLuClusterThreads / 32];
-  __shared__ int s_wi[kLuClusterThreads / 32];
-  __shared__ int s_piv[2];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ int s_perm[kLuClusterMaxP];
+  __shared__ int s_piv[3];
+  __shared__ double s_rcp;
+  const int tid = threadIdx.x;
   constexpr int NT = kLuClusterThreads;
   for (int e = tid; e < ncol * P; e += NT) {
     const int q = e / P, r = e - q * P;
     panel[q * P + r] = a[static_cast<int64_t>(r) * P + rank + kLuCtas * q];
   }
-  if (!FACTOR)
+  for (int r = tid; r < P; r += NT) s_perm[r] = r;
+  if (!FACTOR && rank == 0)
     for (int r = tid; r < P; r += NT) s_x[r] = xg[r];
-  __syncthreads();
-  for (int k = 0; k < P; ++k) {
-    const int o = k % kLuCtas, par = k & 1;
-    double* l_own = s_l + par * P;
-    if (rank == o) {
-      double* col = panel + (k / kLuCtas) * P;
-      double best = -1.0;
-      int bi = P;
-      for (int r = k + tid; r < P; r += NT) {
-        const double v = fabs(col[r]);
-        if (v > best) {
-          best = v;
-          bi = r;
-        }
-      }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const double v2 = __shfl_down_sync(0xffffffffu, best, off);
-        const int i2 = __shfl_down_sync(0xffffffffu, bi, off);
-        if (v2 > best || (v2 == best && i2 < bi)) {
-          best = v2;
-          bi = i2;
-        }
-      }
-      if (lane == 0) {
-        s_wv[warp] = best;
-        s_wi[warp] = bi;
-      }
-      __syncthreads();
+  cl.sync();  // every CTA runs: its shared memory may be written
+
+  // pivot and multipliers of column k (this CTA's, up to date) into every CTA
+  auto prepare = [&](int k) {
+    const double* col = panel + (k / kLuCtas) * P;
+    const int par = k % 3;
+    if (tid < 32) {
+      int piv = lu_warp_pivot(col, s_perm, k, P);
+      if (tid == 0 && piv == P) flag_status(kStatusNonFinite);
+      if (piv == P) piv = k;
+      if (tid < kLuCtas) *cl.map_shared_rank(s_piv + par, tid) = piv;
       if (tid == 0) {
-        best = s_wv[0];
-        bi = s_wi[0];
-        for (int w = 1; w < NT / 32; ++w)
-          if (s_wv[w] > best || (s_wv[w] == best && s_wi[w] < bi)) {
-            best = s_wv[w];
-            bi = s_wi[w];
-          }
-        if (!(best > 0.0)) flag_status(kStatusNonFinite);
-        s_piv[par] = bi;
-        if (bi != k && bi < P) {
-          const double t = col[k];
-          col[k] = col[bi];
-          col[bi] = t;
-        }
+        s_piv[par] = piv;
+        s_rcp = 1.0 / col[s_perm[piv]];
       }
+    }
+    __syncthreads();
+    const int piv = s_piv[par];
+    const double akk = col[s_perm[piv]];  // row k once swapped
+    const int i = k + 1 + tid;
+    if (i < P) {
+      const int r = s_perm[i == piv ? k : i];
+      const double l = quotient(col[r], akk, s_rcp);
+#pragma unroll
+      for (int c = 0; c < kLuCtas; ++c) cl.map_shared_rank(s_l + par * P, c)[r] = l;
+      if (FACTOR) wl[static_cast<int64_t>(k) * P + r] = l;
+    }
+  };
+
+  if (rank == 0) prepare(0);
+  auto token = cl.barrier_arrive();
+  for (int k = 0; k < P; ++k) {
+    cl.barrier_wait(std::move(token));
+    const double* l = s_l + (k % 3) * P;
+    if (tid == 0) {
+      const int piv = s_piv[k % 3], t = s_perm[k];
+      s_perm[k] = s_perm[piv];
+      s_perm[piv] = t;
+    }
+    __syncthreads();  // the permutation, and the last step's updates
+    const int top = s_perm[k];
+    const int i = k + 1 + tid;
+    const int r = i < P ? s_perm[i] : 0;
+    // the next column first, its pivot and multipliers
+    const bool own = k + 1 < P && (k + 1) % kLuCtas == rank;
+    if (own) {
+      double* col = panel + ((k + 1) / kLuCtas) * P;
+      if (i < P) col[r] -= l[r] * col[top];
       __syncthreads();
-      const double akk = col[k];
-      for (int r = k + 1 + tid; r < P; r += NT) l_own[r] = col[r] / akk;
-      if (FACTOR) {
-        for (int r = k + 1 + tid; r < P; r += NT) wl[static_cast<int64_t>(k) * P + r] = l_own[r];
-        if (tid == 0) wp[k] = static_cast<double>(s_piv[par]);
+      prepare(k + 1);
+    }
+    token = cl.barrier_arrive();
+    // then this CTA's other columns j > k + 1 (and the right-hand side)
+    const int first = k + 1 - rank + (own ? 1 : 0);  // least j - rank
+    const int q0 = first > 0 ? (first + kLuCtas - 1) / kLuCtas : 0;
+    if (i < P) {
+      const double lr = l[r];
+      if (!FACTOR && rank == 0) s_x[r] -= lr * s_x[top];
+      for (int q = q0; q < ncol; ++q) {
+        double* col = panel + q * P;
+        col[r] -= lr * col[top];
       }
     }
-    cl.sync();
-    const double* l_src = cl.map_shared_rank(l_own, o);
-    const int piv = *cl.map_shared_rank(s_piv + par, o);
-    if (rank != o)
-      for (int r = k + 1 + tid; r < P; r += NT) l_own[r] = l_src[r];
-    // rows k and piv in this CTA's columns j > k (the owner's column k is done)
-    const int q0 = (k + 1 - rank + kLuCtas - 1) / kLuCtas > 0 ? (k + 1 - rank + kLuCtas - 1) / kLuCtas
-                                                             : 0;  // first q with j > k
-    if (piv != k && piv < P)
-      for (int q = q0 + tid; q < ncol; q += NT) {
-        double* c = panel + q * P;
-        const double t = c[k];
-        c[k] = c[piv];
-        c[piv] = t;
-      }
-    if (!FACTOR && tid == 0 && piv != k && piv < P) {
-      const double t = s_x[k];
-      s_x[k] = s_x[piv];
-      s_x[piv] = t;
-    }
-    __syncthreads();
-    if (!FACTOR) {
-      const double xk = s_x[k];
-      for (int r = k + 1 + tid; r < P; r += NT) s_x[r] -= l_own[r] * xk;
-    }
-    // trailing update of this CTA's columns j > k, rows r > k
-    const int nq = ncol - q0, nr = P - k - 1;
-    for (int e = tid; e < nq * nr; e += NT) {
-      const int qq = e / nr, r = k + 1 + (e - qq * nr);
-      double* c = panel + (q0 + qq) * P;
-      c[r] -= l_own[r] * c[k];
-    }
-    __syncthreads();
   }
-  // gather the upper triangle, packed by columns, into CTA 0
-  double* u0 = cl.map_shared_rank(s_u, 0);
+  cl.barrier_wait(std::move(token));
+  __syncthreads();
+  // the upper triangle, packed by columns, into the workspace or CTA 0
+  double* u0 = FACTOR ? wu : cl.map_shared_rank(s_u, 0);
   for (int q = 0; q < ncol; ++q) {
     const int j = rank + kLuCtas * q;
-    const int base = j * (j + 1) / 2;
-    for (int r = tid; r <= j; r += NT) u0[base + r] = panel[q * P + r];
+    for (int i = tid; i <= j; i += NT) u0[packed_u(j) + i] = panel[q * P + s_perm[i]];
+  }
+  if (FACTOR) {
+    if (rank == 0)
+      for (int i = tid; i < P; i += NT) wp[i] = static_cast<double>(s_perm[i]);
+    return;
   }
   cl.sync();
-  if (rank == 0) {
-    if (FACTOR) {
-      for (int e = tid; e < P * (P + 1) / 2; e += NT) wu[e] = s_u[e];
-      return;
-    }
-    back_substitute(P, s_u, s_x, tid, NT);
-    for (int r = tid; r < P; r += NT) xg[r] = s_x[r];
-  }
+  if (rank != 0) return;
+  // the right-hand side in the rows' final order
+  double x = 0.0;
+  if (tid < P) x = s_x[s_perm[tid]];
+  __syncthreads();
+  if (tid < P) s_x[tid] = x;
+  __syncthreads();
+  back_substitute(P, s_u, s_x, tid);
+  for (int i = tid; i < P; i += NT) xg[i] = s_x[i];
 }
 
 // The solve of a factorisation left by lu_cluster_kernel<true> in W: the
-// fused kernel's right-hand-side operations replayed in its order (the pivot
-// swap and the multipliers of step k, k = 0..P-1, then the back
-// substitution), one CTA per system.  Dynamic shared memory: s_x[P], packed
-// U[P (P + 1) / 2], the pivots[P].
+// fused kernel's operations on the right-hand side, in its order, one CTA per
+// system.  Forward 32 columns at a time: a warp runs through their triangle with
+// its multipliers in registers, then a thread per row below subtracts their
+// share; then the back substitution.  Dynamic shared memory: x[P], packed U.
 __global__ void __launch_bounds__(kLuClusterThreads)
     lu_solve_factored_kernel(int P, const double* __restrict__ W, double* __restrict__ b) {
   extern __shared__ double sf_smem[];
+  __shared__ int s_perm[kLuClusterMaxP];
   const int sys = blockIdx.x;
   const double* wl = W + static_cast<int64_t>(sys) * lu_workspace_doubles(P);
   const double* wp = wl + static_cast<int64_t>(P) * P;
@@ -607,36 +668,38 @@ __global__ void __launch_bounds__(kLuClusterThreads)
   double* xg = b + static_cast<int64_t>(sys) * P;
   double* s_x = sf_smem;
   double* s_u = s_x + P;
-  double* s_p = s_u + P * (P + 1) / 2;  // pivots
-  const int tid = threadIdx.x;
-  constexpr int NT = kLuClusterThreads;  // >= P: one row per thread and step
-  for (int r = tid; r < P; r += NT) {
-    s_x[r] = xg[r];
-    s_p[r] = wp[r];
-  }
-  for (int e = tid; e < P * (P + 1) / 2; e += NT) s_u[e] = wu[e];
+  const int tid = threadIdx.x, lane = tid & 31;
+  constexpr int NT = kLuClusterThreads;  // >= P: one row per thread
+  for (int i = tid; i < P; i += NT) s_perm[i] = static_cast<int>(wp[i]);
+  for (int e = tid; e < packed_u(P); e += NT) s_u[e] = wu[e];
   __syncthreads();
-  // step k updates row k + 1 + tid with step k's multiplier for that row; the
-  // next step's multiplier is loaded while this step's barrier waits
-  double lcur = 1 + tid < P ? wl[1 + tid] : 0.0;
-  for (int k = 0; k < P; ++k) {
-    const int piv = static_cast<int>(s_p[k]);
-    if (tid == 0 && piv != k && piv < P) {
-      const double t = s_x[k];
-      s_x[k] = s_x[piv];
-      s_x[piv] = t;
+  const int row = tid < P ? s_perm[tid] : 0;
+  double x = tid < P ? xg[row] : 0.0;
+  __syncthreads();  // (every row is read before any is written)
+  for (int k0 = 0; k0 < P; k0 += 32) {
+    const int n = min(32, P - k0);
+    // this row's multipliers of the block's columns
+    double l[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c)
+      l[c] = c < n && tid < P && tid > k0 + c ? wl[static_cast<int64_t>(k0 + c) * P + row] : 0.0;
+    if ((tid >> 5) == (k0 >> 5)) {
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        const double xc = __shfl_sync(0xffffffffu, x, c);
+        if (c < n && lane > c) x -= l[c] * xc;
+      }
+      if (lane < n) s_x[k0 + lane] = x;
     }
     __syncthreads();
-    const double xk = s_x[k];
-    const int rn = k + 2 + tid;
-    const double lnext = rn < P ? wl[static_cast<int64_t>(k + 1) * P + rn] : 0.0;
-    const int r = k + 1 + tid;
-    if (r < P) s_x[r] -= lcur * xk;
-    lcur = lnext;
+    if (tid >= k0 + 32 && tid < P) {
+#pragma unroll
+      for (int c = 0; c < 32; ++c) x -= l[c] * s_x[k0 + c];
+    }
     __syncthreads();
   }
-  back_substitute(P, s_u, s_x, tid, NT);
-  for (int r = tid; r < P; r += NT) xg[r] = s_x[r];
+  back_substitute(P, s_u, s_x, tid);
+  for (int i = tid; i < P; i += NT) xg[i] = s_x[i];
 }
 
 struct LoadsArgs {
@@ -1038,7 +1101,7 @@ int fvx_lu_solve_batched(int n_systems, int P, double* A, double* b, void* strea
   if (P <= fvx::kLuClusterMaxP) {
     const int ncmax = (P + fvx::kLuCtas - 1) / fvx::kLuCtas;
     const size_t smem =
-        8 * (static_cast<size_t>(ncmax) * P + 3 * static_cast<size_t>(P) + P * (P + 1) / 2);
+        8 * (static_cast<size_t>(ncmax) * P + 4 * static_cast<size_t>(P) + P * (P + 1) / 2);
     FVX_CUDA_TRY(cudaFuncSetAttribute(fvx::lu_cluster_kernel<false>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(smem)));
@@ -1071,7 +1134,7 @@ int fvx_lu_factor_batched(int n_systems, int P, double* A, double* work, void* s
                 "bad factor arguments (P must be 1..%d)", fvx::kLuClusterMaxP);
   const int ncmax = (P + fvx::kLuCtas - 1) / fvx::kLuCtas;
   const size_t smem =
-      8 * (static_cast<size_t>(ncmax) * P + 3 * static_cast<size_t>(P) + P * (P + 1) / 2);
+      8 * (static_cast<size_t>(ncmax) * P + 4 * static_cast<size_t>(P));
   FVX_CUDA_TRY(cudaFuncSetAttribute(fvx::lu_cluster_kernel<true>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(smem)));
@@ -1085,7 +1148,7 @@ int fvx_lu_solve_factored_batched(int n_systems, int P, const double* work, doub
                                   void* stream) {
   FVX_ARG_CHECK(n_systems >= 1 && P >= 1 && P <= fvx::kLuClusterMaxP && work && b,
                 "bad solve arguments (P must be 1..%d)", fvx::kLuClusterMaxP);
-  const size_t smem = 8 * (2 * static_cast<size_t>(P) + static_cast<size_t>(P) * (P + 1) / 2);
+  const size_t smem = 8 * (static_cast<size_t>(P) + static_cast<size_t>(P) * (P + 1) / 2);
   FVX_CUDA_TRY(cudaFuncSetAttribute(fvx::lu_solve_factored_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(smem)));
