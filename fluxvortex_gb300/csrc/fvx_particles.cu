@@ -22,20 +22,23 @@
 // (fvx_x3.cuh) and only the vector part stays in FP64; tiles with values outside
 // that arithmetic's range take the FP64 core (core_f64).
 //
-// Layout and tiling: a CTA owns 128 (FP64) or 256-512 (FP32, two or four per
-// thread) targets held in registers.  Source tiles of 128 particles (AoS pos, alpha,
+// Layout and tiling: a CTA owns 128 (FP64) or 256 (FP32, two per thread) targets
+// held in registers.  Source tiles of 128 particles (AoS pos, alpha,
 // sigma exactly as the caller stores them) are staged by 1-D TMA bulk copies
 // (cp.async.bulk) into a double-buffered raw area, then converted by all
 // threads into a compute tile (alpha pre-scaled by C, sigma^2 and the core's
-// second constant precomputed; FP32 positions re-centred on the CTA's first
-// target in FP64 before rounding).  Every thread then sweeps the tile reading
+// second constant precomputed; FP32 positions re-centred in FP64 on the first
+// of the target's block of 256 or 512 before rounding).  Every thread then sweeps the tile reading
 // shared memory by broadcast.  FP32 sums are kept per tile and folded into a
 // two-sum (hi, lo) pair per component.  When targets alone cannot fill the
 // SMs the source range is split over gridDim.y; partial sums go to scratch
 // and a second kernel adds them in fixed order.
+#include <cfloat>
+
 #include "fvx_common.cuh"
 #include "fvx_core_table.cuh"
 #include "fvx_pair_math.cuh"
+#include "fvx_x2.cuh"
 #include "fvx_x3.cuh"
 
 namespace fvx {
@@ -62,11 +65,13 @@ struct SrcTile {
   float4 a[kSrcTile];  // C*alpha_x, C*alpha_y, C*alpha_z, k2
 };
 
-// Targets per thread: more register blocking for the 3-component modes.
+// FP32 sweeps: two targets per thread, the halves of f32x2 registers.  (Four took
+// half the shared-memory loads but 96-106 registers and half as many CTAs:
+// 32,768 particles 918 us against 841 for the velocity, 1,340 against 1,222 for the
+// stretching.)  Blocks of `origin` targets share a re-centring origin.
+constexpr int kTargetsF32 = 2 * kThreads;
 template <int MODE>
-struct Blocking {
-  static constexpr int tpt = ModeInfo<MODE>::ncomp <= 3 ? 4 : 2;
-};
+constexpr int kOrigin = kThreads * (ModeInfo<MODE>::ncomp <= 3 ? 4 : 2);
 
 struct PairArgs {
   const double* tgt;
@@ -113,10 +118,89 @@ __device__ __forceinline__ void two_sum_fold(T& hi, T& lo, T p) {
   lo += err;
 }
 
+// One source against a thread's pair of targets (Winckelmans): core_f32 and
+// accumulate in paired arithmetic, each product and sum with the scalar form's
+// roundings, so the sums are the scalar loop's bit for bit.  The FP32 pipe bounds
+// the loop (25 operations a pair for the velocity, 36 for the stretching); scalar
+// instructions fill the issue slots before the pipe (79 % issue, 72 % of the
+// pipe), paired ones take half of them.  32,768 particles: velocity
+// 1,184 -> 839 us, stretching 1,538 -> 1,197 us (85 % of the pipe).
+// NORMAL: q = r^2 + s^2 is a normal number whatever r (core_f32's rsqrtf scales
+// its argument in case it is not: three of a pair's forty instructions).
+template <int MODE, bool NORMAL>
+__device__ __forceinline__ void pair_x2(const float4 pv, const float4 av, const uint64_t (&t)[3],
+                                        const uint64_t (&g)[3],
+                                        uint64_t (&acc)[ModeInfo<MODE>::ncomp]) {
+  const uint64_t a[3] = {x2::dup(av.x), x2::dup(av.y), x2::dup(av.z)};
+  const uint64_t na[3] = {x2::dup(-av.x), x2::dup(-av.y), x2::dup(-av.z)};
+  const uint64_t s2 = x2::dup(pv.w);
+  const uint64_t d[3] = {x2::sub(t[0], x2::dup(pv.x)), x2::sub(t[1], x2::dup(pv.y)),
+                         x2::sub(t[2], x2::dup(pv.z))};
+  const uint64_t r2 = x2::fma(d[2], d[2], x2::fma(d[0], d[0], x2::mul(d[1], d[1])));
+  float qa, qb;
+  x2::unpack(x2::add(r2, s2), qa, qb);
+  const uint64_t T = NORMAL ? x2::pack(rsqrt_ftz(qa), rsqrt_ftz(qb))
+                            : x2::pack(rsqrtf(qa), rsqrtf(qb));
+  const uint64_t T2 = x2::mul(T, T);
+  const uint64_t T5 = x2::mul(x2::mul(T2, T2), T);
+  const uint64_t f = x2::mul(x2::add(r2, x2::dup(av.w)), T5);
+  uint64_t fpr = 0;
+  if constexpr (ModeInfo<MODE>::need_fpr)
+    fpr = x2::mul(
+        x2::mul(x2::fma(x2::dup(-10.5f), s2, x2::mul(x2::dup(-3.0f), r2)), T2), T5);
+  // (v x a)_c = v_i a_j - v_j a_i, (c, i, j) cyclic
+  auto cross = [&](const uint64_t (&v)[3], int c) {
+    const int i = (c + 1) % 3, j = (c + 2) % 3;
+    return x2::fma(v[i], a[j], x2::mul(v[j], na[i]));
+  };
+  auto dot = [&](const uint64_t (&v)[3]) {
+    return x2::fma(d[2], v[2], x2::fma(d[0], v[0], x2::mul(d[1], v[1])));
+  };
+  if constexpr (MODE == FVX_PAIR_VELOCITY || MODE == FVX_PAIR_VELOCITY_STRETCH) {
+    const uint64_t e[3] = {x2::mul(f, d[0]), x2::mul(f, d[1]), x2::mul(f, d[2])};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) acc[c] = x2::add(acc[c], cross(e, c));
+  }
+  if constexpr (MODE == FVX_PAIR_STRETCH || MODE == FVX_PAIR_VELOCITY_STRETCH) {
+    constexpr int o = MODE == FVX_PAIR_STRETCH ? 0 : 3;
+    const uint64_t w = x2::mul(fpr, dot(g));
+    uint64_t v[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[c] = x2::fma(f, g[c], x2::mul(w, d[c]));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) acc[o + c] = x2::add(acc[o + c], cross(v, c));
+  }
+  if constexpr (MODE == FVX_PAIR_JACOBIAN) {
+    const uint64_t q[3] = {x2::mul(fpr, cross(d, 0)), x2::mul(fpr, cross(d, 1)),
+                           x2::mul(fpr, cross(d, 2))};
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        uint64_t& o = acc[3 * i + j];
+        if (i == j) {
+          o = x2::fma(q[i], d[i], o);
+        } else {  // + f a_l where (i, j, l) is cyclic, - f a_l otherwise
+          const int l = 3 - i - j;
+          o = x2::add(o, x2::fma(q[i], d[j], x2::mul(f, (j - i + 3) % 3 == 1 ? a[l] : na[l])));
+        }
+      }
+  }
+  if constexpr (MODE == FVX_PAIR_VORTICITY) {
+    const uint64_t u = x2::mul(fpr, dot(a));
+    const uint64_t v = x2::fma(fpr, r2, x2::add(f, f));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) acc[c] = x2::add(acc[c], x2::fma(d[c], u, x2::mul(na[c], v)));
+  }
+}
+
+// (the stated minimum of one CTA per SM leaves ptxas its registers: 839 and 1,197 us
+// at 32,768 particles; 873 and 1,207 with the default's 64)
 template <int MODE, int KERNEL>
-__global__ void __launch_bounds__(kThreads) pairs_f32_kernel(PairArgs A) {
+__global__ void __launch_bounds__(kThreads, 1) pairs_f32_kernel(PairArgs A) {
   using T = float;
-  constexpr int TPT = Blocking<MODE>::tpt;  // targets per thread
+  constexpr int TPT = kTargetsF32 / kThreads;  // targets per thread
+  constexpr bool PAIRED = KERNEL == FVX_KERNEL_WINCKELMANS;
   constexpr int NC = ModeInfo<MODE>::ncomp;
   constexpr bool NEED_FPR = ModeInfo<MODE>::need_fpr;
   constexpr bool NEED_TG = ModeInfo<MODE>::need_tg;
@@ -125,9 +209,9 @@ __global__ void __launch_bounds__(kThreads) pairs_f32_kernel(PairArgs A) {
   __shared__ __align__(16) SrcTile tile;
   __shared__ __align__(8) uint64_t bar[2];
 
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * (kThreads * TPT);
-  // Re-centring origin: the CTA's first target.
-  const double ox = A.tgt[3 * base + 0], oy = A.tgt[3 * base + 1], oz = A.tgt[3 * base + 2];
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kTargetsF32;
+  const int64_t ob = base / kOrigin<MODE> * kOrigin<MODE>;
+  const double ox = A.tgt[3 * ob + 0], oy = A.tgt[3 * ob + 1], oz = A.tgt[3 * ob + 2];
   T tx[TPT], ty[TPT], tz[TPT], gx[TPT], gy[TPT], gz[TPT];
   bool act[TPT];
 #pragma unroll
@@ -169,6 +253,8 @@ __global__ void __launch_bounds__(kThreads) pairs_f32_kernel(PairArgs A) {
   for (int j = 0; j < TPT; ++j)
 #pragma unroll
     for (int c = 0; c < NC; ++c) hi[j][c] = lo[j][c] = T(0);
+  const uint64_t t2[3] = {x2::pack(tx[0], tx[1]), x2::pack(ty[0], ty[1]), x2::pack(tz[0], tz[1])};
+  const uint64_t g2[3] = {x2::pack(gx[0], gx[1]), x2::pack(gy[0], gy[1]), x2::pack(gz[0], gz[1])};
 
   uint32_t phase[2] = {0u, 0u};
   bool ok = true;
@@ -192,6 +278,7 @@ __global__ void __launch_bounds__(kThreads) pairs_f32_kernel(PairArgs A) {
     phase[buf] ^= 1u;
     tail_src(A, raw[buf], j0, n);
     __syncthreads();
+    bool subnormal = false;
     for (int k = threadIdx.x; k < n; k += kThreads) {
       const double sg = raw[buf].sigma[k];
       float4 pv, av;
@@ -205,26 +292,44 @@ __global__ void __launch_bounds__(kThreads) pairs_f32_kernel(PairArgs A) {
       av.w = static_cast<T>(KERNEL == FVX_KERNEL_WINCKELMANS ? 2.5 * sg * sg : 1.0 / sg);
       tile.p[k] = pv;
       tile.a[k] = av;
+      if (PAIRED) subnormal |= !(pv.w >= FLT_MIN);  // (or NaN)
     }
-    __syncthreads();
+    bool normal = false;
+    if constexpr (PAIRED)
+      normal = !__syncthreads_or(subnormal);
+    else
+      __syncthreads();
     T part[TPT][NC];
+    if constexpr (PAIRED) {
+      uint64_t part2[NC];
 #pragma unroll
-    for (int j = 0; j < TPT; ++j)
+      for (int c = 0; c < NC; ++c) part2[c] = 0ull;
+      if (normal) {
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) pair_x2<MODE, true>(tile.p[k], tile.a[k], t2, g2, part2);
+      } else {
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) pair_x2<MODE, false>(tile.p[k], tile.a[k], t2, g2, part2);
+      }
 #pragma unroll
-      for (int c = 0; c < NC; ++c) part[j][c] = T(0);
+      for (int c = 0; c < NC; ++c) x2::unpack(part2[c], part[0][c], part[1][c]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < TPT; ++j)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) part[j][c] = T(0);
 #pragma unroll 2
-    for (int k = 0; k < n; ++k) {
-      const float4 pv = tile.p[k];
-      const float4 av = tile.a[k];
-      const T sx = pv.x, sy = pv.y, sz = pv.z, s2 = pv.w;
-      const T ax = av.x, ay = av.y, az = av.z, k2 = av.w;
+      for (int k = 0; k < n; ++k) {
+        const float4 pv = tile.p[k], av = tile.a[k];
 #pragma unroll
-      for (int j = 0; j < TPT; ++j) {
-        const T dx = tx[j] - sx, dy = ty[j] - sy, dz = tz[j] - sz;
-        const T r2 = dx * dx + dy * dy + dz * dz;
-        T f, fpr = T(0);
-        core_f32<KERNEL, NEED_FPR>(r2, s2, k2, f, fpr);
-        accumulate<MODE, T>(part[j], dx, dy, dz, r2, ax, ay, az, f, fpr, gx[j], gy[j], gz[j]);
+        for (int j = 0; j < TPT; ++j) {
+          const T dx = tx[j] - pv.x, dy = ty[j] - pv.y, dz = tz[j] - pv.z;
+          const T r2 = dx * dx + dy * dy + dz * dz;
+          T f, fpr = T(0);
+          core_f32<KERNEL, NEED_FPR>(r2, pv.w, av.w, f, fpr);
+          accumulate<MODE, T>(part[j], dx, dy, dz, r2, av.x, av.y, av.z, f, fpr, gx[j], gy[j],
+                              gz[j]);
+        }
       }
     }
 #pragma unroll
@@ -612,14 +717,15 @@ int mode_ncomp(int mode) {
 
 int mode_na(int mode) { return mode == FVX_PAIR_VELOCITY_STRETCH ? 3 : mode_ncomp(mode); }
 
+// Targets of one row of the split rule's grid.
 int targets_per_cta(int mode, int precision) {
   if (precision != FVX_PREC_F32C) return kThreads;
   return kThreads * (mode_ncomp(mode) <= 3 ? 4 : 2);
 }
 
-// Splits of the source range for six resident CTAs per SM (80 registers x 128
-// threads), of at least two source tiles: few targets (the panel points against
-// every particle) split the sources that far.
+// Splits of the source range for six CTAs of a row's targets per SM, of at least
+// two source tiles: few targets (the panel points against every particle) split
+// the sources that far.
 int splits_f32(int64_t gx, int64_t n_src, int64_t* chunk) {
   const int64_t want = 6LL * device_sm_count();
   int64_t s = gx >= want ? 1 : (want + gx - 1) / gx;
@@ -673,6 +779,7 @@ int pair_splits(int mode, int precision, int64_t n_tgt, int64_t n_src, int64_t* 
 template <int MODE, int KERNEL>
 void launch_mode(int precision, dim3 grid, cudaStream_t stream, const PairArgs& A) {
   if (precision == FVX_PREC_F32C) {
+    grid.x = static_cast<unsigned>((A.n_tgt + kTargetsF32 - 1) / kTargetsF32);
     pairs_f32_kernel<MODE, KERNEL><<<grid, kThreads, 0, stream>>>(A);
     return;
   }

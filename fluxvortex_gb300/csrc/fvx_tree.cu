@@ -31,6 +31,7 @@
 
 #include "fvx_common.cuh"
 #include "fvx_pair_math.cuh"
+#include "fvx_x2.cuh"
 
 namespace fvx {
 namespace tree {
@@ -1184,39 +1185,6 @@ __device__ __forceinline__ void m2p(float* acc, const float* R, float rx, float 
     }
   }
 }
-
-// ---- paired FP32 (f32x2) arithmetic: two targets per instruction -------------
-namespace x2 {
-__device__ __forceinline__ uint64_t pack(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t dup(float a) { return pack(a, a); }
-__device__ __forceinline__ void unpack(uint64_t v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t sub(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-}  // namespace x2
 
 // The packed near tile: kNearTile staged sources, one per row, in planes of
 // 16-byte words (plane w of row k at w * kNearTile + k), so that a warp
