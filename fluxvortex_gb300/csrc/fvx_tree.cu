@@ -14,10 +14,9 @@
 //   bbox -> host picks the grid (tree_params.grid_params: root cube of 2^L
 //   leaves of size c 2^k, c in {1, 5/4, 3/2, 7/4}, aligned to the leaf size) -> 30-bit Morton keys -> stable LSD radix
 //   sort (4 x 8-bit digits, per-block histograms, warp-match ranking) ->
-//   leaf cells = runs of equal keys, coarser levels = runs of equal key >> 3
-//   among the finer level's cells -> sorted FP32 particle records relative to
-//   their leaf centre -> leaf moments (one warp per leaf) -> M2M shifts up the
-//   levels -> interaction lists per target leaf (depth-first traversal, exact
+//   cells of all levels = runs of equal key prefixes -> sorted FP32 particle
+//   records relative to their leaf centre -> leaf moments (one warp per leaf)
+//   and M2M shifts up the levels -> interaction lists per target leaf (depth-first traversal, exact
 //   acceptance test |dc|^2 > 3/4 (h_T + h_S)^2 / theta^2 in FP64) -> eval.
 // Because cell centres are exact binary fractions, centre differences are
 // exact in FP32 and pair offsets are (c_T - c_S) + (o_t - o_s) with small
@@ -309,18 +308,7 @@ int sort_pairs_u32(uint32_t* keys, int* idx, uint32_t* keys_tmp, int* idx_tmp, i
 namespace tree {
 
 // ---- cells ----------------------------------------------------------------------
-// flag[i] = 1 where the level key (key >> shift) changes
-__global__ void flags_kernel(const uint32_t* __restrict__ keys, const int* __restrict__ n_ptr,
-                             int n_cap, int shift, int* __restrict__ flag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = n_ptr ? *n_ptr : n_cap;
-  if (i >= n_cap) return;
-  if (i >= n) {
-    flag[i] = 0;
-    return;
-  }
-  flag[i] = (i == 0 || (keys[i] >> shift) != (keys[i - 1] >> shift)) ? 1 : 0;
-}
+constexpr int kMaxLevels = 11;
 
 struct Level {
   int* start;     // first sorted particle of each cell
@@ -330,63 +318,157 @@ struct Level {
   int* child_hi;  // one past the last child
 };
 
-// leaf cells from the particle flags (cid = inclusive scan of flags)
-__global__ void leaf_cells_kernel(const uint32_t* __restrict__ keys, int n,
-                                  const int* __restrict__ flag, const int* __restrict__ cid,
-                                  Level lv, int* __restrict__ n_cells) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int c = cid[i] - 1;
-  if (flag[i]) {
-    lv.start[c] = i;
-    lv.key[c] = keys[i];
+// The cells of all levels, as arrays over the levels' concatenated capacities
+// (level l's at base[l]).
+struct Cells {
+  int* start;
+  int* count;
+  uint32_t* key;
+  int* child_lo;
+  int* child_hi;
+  int* parent;   // level-local id of the parent (levels 1..L)
+  int* arrived;  // children whose moments are done (zero between sweeps)
+  int base[kMaxLevels + 1];
+  int L;
+};
+
+// A sorted particle starts a new cell on every level from some level on: that level
+// follows from the highest bit in which its key and its predecessor's differ, so
+// one pass over the particles counts and one pass fills the cells of all levels
+// (a launch per array and level, with a device-wide scan each, took 42 launches
+// and 0.14 ms at 131,072 particles; these four take 27 us).
+__device__ __forceinline__ int first_level(const uint32_t* __restrict__ keys, int i, int L) {
+  if (i == 0) return 0;
+  const uint32_t d = keys[i] ^ keys[i - 1];
+  return d ? max(L - (31 - __clz(d)) / 3, 0) : L + 1;
+}
+
+// Cells started in each block of kSortItems particles, per level: table[l][block].
+__global__ void __launch_bounds__(256) level_hist_kernel(const uint32_t* __restrict__ keys, int n,
+                                                         int L, int nblk,
+                                                         int* __restrict__ table) {
+  __shared__ int h[kMaxLevels + 1];
+  if (threadIdx.x <= kMaxLevels) h[threadIdx.x] = 0;
+  __syncthreads();
+  for (int k = threadIdx.x; k < kSortItems; k += 256) {
+    const int i = blockIdx.x * kSortItems + k;
+    const int lv = i < n ? first_level(keys, i, L) : L + 1;
+    for (int l = 0; l <= L; ++l) {
+      const unsigned m = __ballot_sync(0xffffffffu, lv <= l);
+      if ((threadIdx.x & 31) == 0 && m) atomicAdd(&h[l], __popc(m));
+    }
   }
-  if (i == n - 1) *n_cells = c + 1;
+  __syncthreads();
+  if (threadIdx.x <= L) table[threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];
 }
 
-__global__ void cell_counts_kernel(Level lv, const int* __restrict__ n_cells, int n_total) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nc = *n_cells;
-  if (c >= nc) return;
-  const int end = c + 1 < nc ? lv.start[c + 1] : n_total;
-  lv.count[c] = end - lv.start[c];
-}
-
-// parent flags over the children cells of level l+1 (keys >> 3)
-__global__ void parent_flags_kernel(Level child, const int* __restrict__ n_child, int cap,
-                                    int* __restrict__ flag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cap) return;
-  const int n = *n_child;
-  if (i >= n) {
-    flag[i] = 0;
-    return;
+// Inclusive sum over the CTA (a multiple of 32 threads, at most 1024).
+__device__ __forceinline__ int block_inclusive(int v, int* s_warp, int& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
   }
-  flag[i] = (i == 0 || (child.key[i] >> 3) != (child.key[i - 1] >> 3)) ? 1 : 0;
-}
-
-__global__ void parent_cells_kernel(Level child, const int* __restrict__ n_child,
-                                    const int* __restrict__ flag, const int* __restrict__ pid,
-                                    Level par, int* __restrict__ n_par) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = *n_child;
-  if (i >= n) return;
-  const int p = pid[i] - 1;
-  if (flag[i]) {
-    par.start[p] = child.start[i];
-    par.key[p] = child.key[i] >> 3;
-    par.child_lo[p] = i;
+  if (lane == 31) s_warp[warp] = v;
+  __syncthreads();
+  int w = lane < nw ? s_warp[lane] : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, w, o);
+    if (lane >= o) w += u;
   }
-  if (i == n - 1 || flag[i + 1]) par.child_hi[p] = i + 1;
-  if (i == n - 1) *n_par = p + 1;
+  total = __shfl_sync(0xffffffffu, w, nw - 1);
+  const int before = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
+  __syncthreads();  // s_warp may be written again
+  return warp ? v + before : v;
 }
 
-// parent particle count = (last child's end) - (first child's start)
-__global__ void parent_counts_kernel(Level child, Level par, const int* __restrict__ n_par) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= *n_par) return;
-  const int lc = par.child_hi[p] - 1;
-  par.count[p] = child.start[lc] + child.count[lc] - par.start[p];
+// A CTA per level: exclusive sums of its row of the table, in place, and the
+// level's cell count.
+__global__ void __launch_bounds__(1024) level_scan_kernel(int nblk, int* __restrict__ table,
+                                                          int* __restrict__ n_cells) {
+  __shared__ int s_warp[32];
+  int* row = table + static_cast<int64_t>(blockIdx.x) * nblk;
+  int run = 0;
+  for (int b0 = 0; b0 < nblk; b0 += 1024) {
+    const int b = b0 + threadIdx.x;
+    const int v = b < nblk ? row[b] : 0;
+    int total;
+    const int incl = block_inclusive(v, s_warp, total);
+    if (b < nblk) row[b] = run + incl - v;
+    run += total;
+  }
+  if (threadIdx.x == 0) n_cells[blockIdx.x] = run;
+}
+
+// Starts, keys, parents and first children of the cells that start in the block,
+// and each particle's leaf (cid, counted from 1).
+__global__ void __launch_bounds__(256) level_cells_kernel(const uint32_t* __restrict__ keys, int n,
+                                                          int nblk, const int* __restrict__ table,
+                                                          Cells C, int* __restrict__ cid) {
+  constexpr int kIters = kSortItems / 256, kSegs = 8 * kIters;  // segments of 32 particles
+  static_assert(kSegs == 32, "a lane per segment");
+  __shared__ int s_seg[kMaxLevels][kSegs];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, L = C.L;
+  const int i0 = blockIdx.x * kSortItems;
+  int lv[kIters];
+#pragma unroll
+  for (int it = 0; it < kIters; ++it) {
+    const int i = i0 + it * 256 + threadIdx.x;
+    lv[it] = i < n ? first_level(keys, i, L) : L + 1;
+    for (int l = 0; l <= L; ++l) {
+      const unsigned m = __ballot_sync(0xffffffffu, lv[it] <= l);
+      if (lane == 0) s_seg[l][it * 8 + warp] = __popc(m);
+    }
+  }
+  __syncthreads();
+  for (int l = warp; l <= L; l += 8) {
+    const int v = s_seg[l][lane];
+    int w = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
+    }
+    s_seg[l][lane] = table[l * nblk + blockIdx.x] + w - v;
+  }
+  __syncthreads();
+  const unsigned upto = lane == 31 ? 0xffffffffu : (2u << lane) - 1u;
+#pragma unroll
+  for (int it = 0; it < kIters; ++it) {
+    const int i = i0 + it * 256 + threadIdx.x;
+    const uint32_t key = i < n ? keys[i] : 0u;
+    int up = -1;  // this particle's cell one level up
+    for (int l = 0; l <= L; ++l) {
+      const unsigned m = __ballot_sync(0xffffffffu, lv[it] <= l);
+      const int r = s_seg[l][it * 8 + warp] + __popc(m & upto) - 1;
+      if (lv[it] <= l) {
+        const int c = C.base[l] + r;
+        C.start[c] = i;
+        C.key[c] = key >> (3 * (L - l));
+        C.parent[c] = up;
+        if (l > 0 && lv[it] < l) C.child_lo[C.base[l - 1] + up] = r;
+      }
+      up = r;
+    }
+    if (i < n) cid[i] = up + 1;
+  }
+}
+
+// What the next cell's entries give: particle counts and last children.
+__global__ void level_finish_kernel(Cells C, int n, const int* __restrict__ n_cells) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int l = 0; l <= C.L; ++l) {
+    const int nc = n_cells[l], b = C.base[l];
+    const int nch = l < C.L ? n_cells[l + 1] : 0;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += stride) {
+      const bool last = c + 1 == nc;
+      C.count[b + c] = (last ? n : C.start[b + c + 1]) - C.start[b + c];
+      if (l < C.L) C.child_hi[b + c] = last ? nch : C.child_lo[b + c + 1];
+      C.arrived[b + c] = 0;
+    }
+  }
 }
 
 // ---- sorted particle records -----------------------------------------------------
@@ -439,17 +521,23 @@ __device__ __forceinline__ int m2i(int j, int k) {
   return a == 0 ? b : (a == 1 ? 2 + b : 5);
 }
 
-// one warp per leaf, moments of the C-scaled strengths about the leaf centre
-__global__ void leaf_moments_kernel(Level lv, const int* __restrict__ n_leaves, float hl,
-                                    const float4* __restrict__ sp, const float4* __restrict__ sa,
-                                    float* __restrict__ rec) {
+// One warp per leaf: moments of the C-scaled strengths about the leaf centre.  The
+// warp whose leaf completes its parent's children goes on with the parent (a
+// lane per moment, the children in order, each shifted by s = c_child -
+// c_parent, exact), and so up the levels: one launch, at 131,072 particles 34 us
+// (96 us with a launch per level and a thread per cell).  The sums round as a
+// thread's running through its cell's moments in turn.
+// Nothing waits: a warp that finds children missing ends.
+__global__ void moments_kernel(Cells C, int nleaf, float hl, const float4* __restrict__ sp,
+                               const float4* __restrict__ sa, float* __restrict__ recs) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp >= *n_leaves) return;
+  if (warp >= nleaf) return;
+  const int leaf = C.base[C.L] + warp;
   float m[30];
 #pragma unroll
   for (int q = 0; q < 30; ++q) m[q] = 0.f;
-  const int s = lv.start[warp], e = s + lv.count[warp];
+  const int s = C.start[leaf], e = s + C.count[leaf];
   for (int i = s + lane; i < e; i += 32) {
     const float4 p = sp[i];
     const float4 a = sa[i];
@@ -471,8 +559,8 @@ __global__ void leaf_moments_kernel(Level lv, const int* __restrict__ n_leaves, 
   for (int q = 0; q < 30; ++q)
     for (int o = 16; o > 0; o >>= 1) m[q] += __shfl_xor_sync(0xffffffffu, m[q], o);
   if (lane == 0) {
-    float* r = rec + static_cast<int64_t>(warp) * kRecFloats;
-    const float3 c = cell_center_rel(lv.key[warp], hl);
+    float* r = recs + static_cast<int64_t>(leaf) * kRecFloats;
+    const float3 c = cell_center_rel(C.key[leaf], hl);
     r[0] = c.x;
     r[1] = c.y;
     r[2] = c.z;
@@ -485,44 +573,57 @@ __global__ void leaf_moments_kernel(Level lv, const int* __restrict__ n_leaves, 
     for (int q = 0; q < 18; ++q) r[19 + q] = m[12 + q];
     r[37] = r[38] = r[39] = 0.f;
   }
-}
-
-// parent moments from children (shift by s = c_child - c_parent, exact)
-__global__ void m2m_kernel(Level par, const int* __restrict__ n_par, float hl,
-                           const float* __restrict__ child_rec, float* __restrict__ par_rec) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= *n_par) return;
-  const float3 cp = cell_center_rel(par.key[p], hl);
-  float M0[3] = {0, 0, 0}, M1[9], M2[18];
-  for (int q = 0; q < 9; ++q) M1[q] = 0.f;
-  for (int q = 0; q < 18; ++q) M2[q] = 0.f;
-  for (int c = par.child_lo[p]; c < par.child_hi[p]; ++c) {
-    const float* r = child_rec + static_cast<int64_t>(c) * kRecFloats;
-    const float s[3] = {r[0] - cp.x, r[1] - cp.y, r[2] - cp.z};
-    for (int m = 0; m < 3; ++m) {
-      const float m0 = r[4 + m];
-      M0[m] += m0;
-      for (int j = 0; j < 3; ++j) M1[3 * m + j] += r[10 + 3 * m + j] + m0 * s[j];
-      for (int j = 0; j < 3; ++j)
-        for (int k = j; k < 3; ++k) {
-          const int u = m2i(j, k);
-          M2[6 * m + u] += r[19 + 6 * m + u] + r[10 + 3 * m + j] * s[k] +
-                           r[10 + 3 * m + k] * s[j] + m0 * s[j] * s[k];
-        }
+  // lane q holds moment q: M0 (3), M1 (3 x 3), M2 (3 x 6: xx xy xz yy yz zz)
+  const int q = min(lane, 29);
+  const int mm = q < 3 ? q : q < 12 ? (q - 3) / 3 : (q - 12) / 6;
+  const int u = q < 12 ? 0 : (q - 12) % 6;
+  const int j = q < 3 ? 0 : q < 12 ? (q - 3) % 3 : u < 3 ? 0 : u < 5 ? 1 : 2;
+  const int k = q < 12 ? 0 : u < 3 ? u : u < 5 ? u - 2 : 2;
+  const int own = q < 3 ? 4 + q : 7 + q;
+  int cell = warp;
+  for (int l = C.L; l > 0; --l) {
+    __threadfence();  // this cell's record before its arrival
+    __syncwarp();
+    const int p = C.parent[C.base[l] + cell], gp = C.base[l - 1] + p;
+    const int lo = C.child_lo[gp], hi = C.child_hi[gp];
+    int before = 0;
+    if (lane == 0) before = atomicAdd(C.arrived + gp, 1);
+    before = __shfl_sync(0xffffffffu, before, 0);
+    if (before != hi - lo - 1) return;
+    if (lane == 0) C.arrived[gp] = 0;
+    __threadfence();
+    hl *= 2.0f;
+    const float3 cp = cell_center_rel(C.key[gp], hl);
+    const float cj = j == 0 ? cp.x : j == 1 ? cp.y : cp.z;
+    const float ck = k == 0 ? cp.x : k == 1 ? cp.y : cp.z;
+    float acc = 0.0f;
+#pragma unroll 4
+    for (int c = lo; c < hi; ++c) {
+      const float* r = recs + static_cast<int64_t>(C.base[l] + c) * kRecFloats;
+      float v = __ldcg(r + own);
+      const float sj = __ldcg(r + j) - cj, sk = __ldcg(r + k) - ck;
+      const float m0 = __ldcg(r + 4 + mm);
+      const float mj = __ldcg(r + 10 + 3 * mm + j), mk = __ldcg(r + 10 + 3 * mm + k);
+      const float ms = __fmul_rn(m0, sj);
+      if (q >= 12)
+        v = fmaf(ms, sk, fmaf(mk, sj, fmaf(mj, sk, v)));
+      else if (q >= 3)
+        v = __fadd_rn(v, ms);
+      acc += v;
     }
+    const float xx = __shfl_sync(0xffffffffu, acc, 12 + 6 * min(lane, 2));
+    const float yy = __shfl_sync(0xffffffffu, acc, 15 + 6 * min(lane, 2));
+    const float zz = __shfl_sync(0xffffffffu, acc, 17 + 6 * min(lane, 2));
+    float* r = recs + static_cast<int64_t>(gp) * kRecFloats;
+    if (lane < 30) r[own] = acc;
+    if (lane < 3) {
+      r[7 + lane] = xx + yy + zz;
+      r[lane] = lane == 0 ? cp.x : lane == 1 ? cp.y : cp.z;
+      r[37 + lane] = 0.0f;
+    }
+    if (lane == 3) r[3] = hl;
+    cell = p;
   }
-  float* r = par_rec + static_cast<int64_t>(p) * kRecFloats;
-  r[0] = cp.x;
-  r[1] = cp.y;
-  r[2] = cp.z;
-  r[3] = hl;
-  for (int m = 0; m < 3; ++m) {
-    r[4 + m] = M0[m];
-    r[7 + m] = M2[6 * m + 0] + M2[6 * m + 3] + M2[6 * m + 5];
-  }
-  for (int q = 0; q < 9; ++q) r[10 + q] = M1[q];
-  for (int q = 0; q < 18; ++q) r[19 + q] = M2[q];
-  r[37] = r[38] = r[39] = 0.f;
 }
 
 // ---- interaction lists --------------------------------------------------------------
@@ -695,14 +796,6 @@ __global__ void order_keys_kernel(int nleaf, const int* __restrict__ near_cnt,
   const long long w = static_cast<long long>(near_cnt[t]) * leaf_count[t];
   keys[t] = 0xFFFFu - static_cast<uint32_t>(w < 0xFFFF ? w : 0xFFFF);
   idx[t] = t;
-}
-
-// leaf -> its parent's level-local index, from the parents' child ranges
-__global__ void leaf_parents_kernel(TreeView T, int* __restrict__ leaf_parent) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= T.ncell[T.L - 1]) return;
-  const int gP = T.base[T.L - 1] + p;
-  for (int c = T.child_lo[gP]; c < T.child_hi[gP]; ++c) leaf_parent[c] = p;
 }
 
 template <bool FILL>
@@ -2318,7 +2411,7 @@ int judge_sums_launch(const JudgeSampleView& S, const uint32_t* leaf_key, const 
 
 struct fvx_tree {
   int device = 0;
-  fvx::DevBuf keys0, keys1, idx0, idx1, table, scan_tmp, flags, cid, levels, counts, rec, sp, sa,
+  fvx::DevBuf keys0, keys1, idx0, idx1, table, scan_tmp, cid, levels, counts, rec, sp, sa,
       sg, lists_meta, near_list, far_list, bbox;
   int64_t stats[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around the last evaluation launch
@@ -2523,6 +2616,19 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
     v.child_hi = lvb + 4 * total_cells + base[l];
     return v;
   };
+  auto cells = [&]() {
+    Cells C;
+    C.start = lvb;
+    C.count = lvb + total_cells;
+    C.key = reinterpret_cast<uint32_t*>(lvb + 2 * total_cells);
+    C.child_lo = lvb + 3 * total_cells;
+    C.child_hi = lvb + 4 * total_cells;
+    C.parent = lvb + 5 * total_cells;
+    C.arrived = lvb + 6 * total_cells;
+    for (int l = 0; l <= L + 1; ++l) C.base[l] = base[l];
+    C.L = L;
+    return C;
+  };
   if (reuse) {
     L = ST.L;
     total_cells = ST.total_cells;
@@ -2573,8 +2679,7 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
       (rc = grow(T->idx0, 4 * size_t(n))) || (rc = grow(T->idx1, 4 * size_t(n))) ||
       (rc = grow(T->table, 4 * size_t(256) * nblk * 2)) ||
       (rc = grow(T->scan_tmp, 4 * size_t(2 * kScanBlock))) ||
-      (rc = grow(T->flags, 4 * size_t(n))) || (rc = grow(T->cid, 4 * size_t(n))) ||
-      (rc = grow(T->levels, 4 * size_t(total_cells) * 5)) ||
+      (rc = grow(T->cid, 4 * size_t(n))) || (rc = grow(T->levels, 4 * size_t(total_cells) * 7)) ||
       (rc = grow(T->counts, 4 * 16)) ||
       (rc = grow(T->rec, 4 * size_t(total_cells) * kRecFloats)) ||
       (rc = grow(T->sp, 16 * size_t(n))) || (rc = grow(T->sa, 16 * size_t(n))) ||
@@ -2606,40 +2711,23 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   }
   const uint32_t* keys = ka;  // sorted
   perm = ia;
-  // 3. cells: leaves from particles, parents from children
+  // 3. cells of all levels
   lvb = P<int>(T->levels);
   int* ncells_d = P<int>(T->counts);
-  int* flag = P<int>(T->flags);
-  int* cid = P<int>(T->cid);
-  flags_kernel<<<(n + 255) / 256, 256, 0, s>>>(keys, nullptr, n, 0, flag);
+  const Cells C = cells();
+  level_hist_kernel<<<nblk, 256, 0, s>>>(keys, n, L, nblk, table);
   FVX_LAUNCH_CHECK();
-  if ((rc = scan_ints(flag, n, cid, 1, P<int>(T->scan_tmp), s))) return rc;
-  Level leaves = level(L);
-  leaf_cells_kernel<<<(n + 255) / 256, 256, 0, s>>>(keys, n, flag, cid, leaves, ncells_d + L);
+  level_scan_kernel<<<L + 1, 1024, 0, s>>>(nblk, table, ncells_d);
   FVX_LAUNCH_CHECK();
-  cell_counts_kernel<<<(n + 255) / 256, 256, 0, s>>>(leaves, ncells_d + L, n);
+  level_cells_kernel<<<nblk, 256, 0, s>>>(keys, n, nblk, table, C, P<int>(T->cid));
   FVX_LAUNCH_CHECK();
-  // parent levels reuse flag (as flags) and the scan buffer; the leaf ids of
-  // the particles (cid) are kept for the gather
-  int* pflag = reinterpret_cast<int*>(kb);  // the sort's free pair
-  int* pid = ib;
-  for (int l = L - 1; l >= 0; --l) {
-    Level ch = level(l + 1), par = level(l);
-    const int cc = cap[l + 1];
-    parent_flags_kernel<<<(cc + 255) / 256, 256, 0, s>>>(ch, ncells_d + l + 1, cc, pflag);
-    FVX_LAUNCH_CHECK();
-    if ((rc = scan_ints(pflag, cc, pid, 1, P<int>(T->scan_tmp), s))) return rc;
-    parent_cells_kernel<<<(cc + 255) / 256, 256, 0, s>>>(ch, ncells_d + l + 1, pflag, pid, par,
-                                                         ncells_d + l);
-    FVX_LAUNCH_CHECK();
-    parent_counts_kernel<<<(cap[l] + 255) / 256, 256, 0, s>>>(ch, par, ncells_d + l);
-    FVX_LAUNCH_CHECK();
-  }
+  level_finish_kernel<<<static_cast<int>(std::min<int64_t>((n + 255) / 256, 4 * device_sm_count())),
+                        256, 0, s>>>(C, n, ncells_d);
+  FVX_LAUNCH_CHECK();
   FVX_CUDA_TRY(cudaMemcpyAsync(ncells, ncells_d, sizeof(int) * (L + 1), cudaMemcpyDeviceToHost, s));
   FVX_CUDA_TRY(cudaStreamSynchronize(s));
   nleaf = ncells[L];
   }
-  int* ncells_d = P<int>(T->counts);
   int* cid = P<int>(T->cid);
   Level leaves = level(L);
   // 4. sorted FP32 records
@@ -2652,18 +2740,11 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
     launch_gather<FVX_KERNEL_GAUSSIANERF>(n, perm, cid, leaves.key, g, pos, alpha, sigma,
                                           need_tg ? tgt_gamma : nullptr, sp, sa, sg, s);
   FVX_LAUNCH_CHECK();
-  // 5. moments: leaves, then M2M up the levels
+  // 5. moments: leaves and up the levels
   float* rec = P<float>(T->rec);
-  leaf_moments_kernel<<<(nleaf * 32 + 255) / 256, 256, 0, s>>>(
-      leaves, ncells_d + L, static_cast<float>(h), sp, sa, rec + int64_t(base[L]) * kRecFloats);
+  moments_kernel<<<(nleaf * 32 + 255) / 256, 256, 0, s>>>(cells(), nleaf, static_cast<float>(h), sp,
+                                                          sa, rec);
   FVX_LAUNCH_CHECK();
-  for (int l = L - 1; l >= 0; --l) {
-    const float hl = static_cast<float>(h * static_cast<double>(1 << (L - l)));
-    m2m_kernel<<<(ncells[l] + 127) / 128, 128, 0, s>>>(
-        level(l), ncells_d + l, hl, rec + int64_t(base[l + 1]) * kRecFloats,
-        rec + int64_t(base[l]) * kRecFloats);
-    FVX_LAUNCH_CHECK();
-  }
   // 6. interaction lists
   TreeView V;
   V.L = L;
@@ -2703,7 +2784,7 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   const int npar = dual ? ncells[L - 1] : 0;
   if ((rc = grow(T->lists_meta, 4 * size_t(nleaf) * 4 + 64))) return rc;
   if (learned && (rc = grow(T->lrn_meta, 4 * size_t(nleaf) * 2 + 64))) return rc;
-  if (dual && (rc = grow(T->dual_meta, 4 * (2 * size_t(npar) + size_t(nleaf)) + 64))) return rc;
+  if (dual && (rc = grow(T->dual_meta, 4 * 2 * size_t(npar) + 64))) return rc;
   LearnedLists LL{nullptr, nullptr, nullptr, nullptr, 0};
   if (learned) {
     LL.cnt = P<int>(T->lrn_meta);
@@ -2716,7 +2797,7 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   unsigned* ovf = reinterpret_cast<unsigned*>(far_off + nleaf);  // + 2 x u64 work counters
   int* par_cnt = dual ? P<int>(T->dual_meta) : nullptr;
   int* par_off = dual ? par_cnt + npar : nullptr;
-  int* leaf_parent = dual ? par_off + npar : nullptr;
+  const int* leaf_parent = dual ? cells().parent + base[L] : nullptr;
   int64_t near_total = 0, far_total = 0, lrn_total = 0, par_total = 0;
   if (reuse) {
     near_total = ST.near_total;
@@ -2729,12 +2810,10 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   // local-expansion pairs are then compacted into flat lists ordered by
   // target.  A slot overflow falls back to the counting pass and exact lists.
   if (dual) {
-    // what every leaf's traversal reads: cell centres and its parent
+    // what every leaf's traversal reads: cell centres
     if ((rc = grow(T->cen, 16 * size_t(total_cells)))) return rc;
     V.cen = P<int4>(T->cen);
     cell_centres_kernel<<<(total_cells + 255) / 256, 256, 0, s>>>(V, total_cells, P<int4>(T->cen));
-    FVX_LAUNCH_CHECK();
-    leaf_parents_kernel<<<(npar + 127) / 128, 128, 0, s>>>(V, leaf_parent);
     FVX_LAUNCH_CHECK();
   }
   bool slotted = false;
@@ -3208,7 +3287,7 @@ void fvx_tree_destroy(fvx_tree* T) {
   if (T->ev2) cudaEventDestroy(T->ev2);
   if (T->ev3) cudaEventDestroy(T->ev3);
   fvx::DevBuf* bufs[] = {&T->keys0,   &T->keys1,     &T->idx0,     &T->idx1,     &T->table,
-                         &T->scan_tmp, &T->flags,   &T->cid,      &T->levels,   &T->counts,
+                         &T->scan_tmp, &T->cid,      &T->levels,   &T->counts,
                          &T->rec,     &T->sp,       &T->sa,       &T->sg,       &T->lists_meta,
                          &T->near_list, &T->far_list, &T->bbox,   &T->lrn_meta, &T->lrn_leaf,
                          &T->lrn_cell, &T->leaf_local, &T->judge_act, &T->judge_cls,
