@@ -35,7 +35,10 @@
 namespace fvx {
 namespace tree {
 
-constexpr int kScanBlock = 2048;   // elements per scan block (1024 threads x 2)
+constexpr int kScanThreads = 1024;
+constexpr int kScanItems = 8;      // elements per thread
+constexpr int kScanBlock = kScanThreads * kScanItems;
+constexpr int kScanOneCta = 65536;  // up to here one CTA scans an array
 constexpr int kSortItems = 1024;   // keys per radix-sort block (256 threads x 4)
 constexpr int kEvalThreads = 32;   // eval CTA (one warp); 1, 2 or 4 targets per thread
 constexpr int kFarTile = 32;       // far cells staged per tile
@@ -44,62 +47,137 @@ constexpr int kRecFloats = 40;     // far-cell record
 constexpr double kC = -0.07957747154594767;  // -1/(4 pi)
 
 // ---- scan: exclusive / inclusive prefix sums of int32 ------------------------
-__global__ void scan_block_kernel(const int* __restrict__ in, int n, int* __restrict__ out,
-                                  int* __restrict__ block_sums, int inclusive) {
-  __shared__ int s[kScanBlock];
-  const int base = blockIdx.x * kScanBlock;
-  for (int k = threadIdx.x; k < kScanBlock; k += blockDim.x) {
-    const int i = base + k;
-    s[k] = i < n ? in[i] : 0;
+// Inclusive sum over the CTA (a multiple of 32 threads, at most 1024).
+__device__ __forceinline__ int block_inclusive(int v, int* s_warp, int& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
   }
+  if (lane == 31) s_warp[warp] = v;
   __syncthreads();
-  // Hillis-Steele on kScanBlock elements with kScanBlock / 2 threads
-  for (int off = 1; off < kScanBlock; off <<= 1) {
-    int v0 = 0, v1 = 0;
-    const int k0 = threadIdx.x, k1 = threadIdx.x + blockDim.x;
-    if (k0 >= off) v0 = s[k0 - off];
-    if (k1 >= off) v1 = s[k1 - off];
-    __syncthreads();
-    s[k0] += v0;
-    s[k1] += v1;
-    __syncthreads();
+  int w = lane < nw ? s_warp[lane] : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, w, o);
+    if (lane >= o) w += u;
   }
-  for (int k = threadIdx.x; k < kScanBlock; k += blockDim.x) {
-    const int i = base + k;
-    if (i < n) out[i] = inclusive ? s[k] : s[k] - (i < n ? in[i] : 0);
-  }
-  if (threadIdx.x == 0 && block_sums) block_sums[blockIdx.x] = s[kScanBlock - 1];
+  total = __shfl_sync(0xffffffffu, w, nw - 1);
+  const int before = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
+  __syncthreads();  // s_warp may be written again
+  return warp ? v + before : v;
 }
 
-__global__ void scan_add_kernel(int* __restrict__ out, int n, const int* __restrict__ offs) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += offs[i / kScanBlock];
+// One CTA's scan of kScanBlock elements from base, `run` before them; returns their sum.
+// Each warp takes kScanItems runs of 32 (coalesced).
+__device__ __forceinline__ int scan_tile(const int* __restrict__ in, int n, int* __restrict__ out,
+                                         int base, int run, int inclusive, int* s_warp) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i0 = base + warp * 32 * kScanItems + lane;
+  int own[kScanItems], v[kScanItems];
+#pragma unroll
+  for (int e = 0; e < kScanItems; ++e) v[e] = own[e] = i0 + 32 * e < n ? in[i0 + 32 * e] : 0;
+  int sum = 0;  // of the warp's runs
+#pragma unroll
+  for (int e = 0; e < kScanItems; ++e) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v[e], o);
+      if (lane >= o) v[e] += u;
+    }
+    const int t = __shfl_sync(0xffffffffu, v[e], 31);
+    v[e] += sum;
+    sum += t;
+  }
+  int total;
+  const int before = block_inclusive(lane == 31 ? sum : 0, s_warp, total);
+  const int off = run + __shfl_sync(0xffffffffu, before, 31) - sum;
+#pragma unroll
+  for (int e = 0; e < kScanItems; ++e)
+    if (i0 + 32 * e < n) out[i0 + 32 * e] = off + v[e] - (inclusive ? 0 : own[e]);
+  return total;
 }
 
-// total of an inclusive scan -> *total
-__global__ void scan_total_kernel(const int* __restrict__ incl, int n, int* __restrict__ total) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *total = n > 0 ? incl[n - 1] : 0;
+// Up to four arrays of at most kScanOneCta elements, a CTA each, and their sums.
+struct ScanJobs {
+  const int* in[4];
+  int* out[4];
+  int n[4];
+  int* total;  // null, or one per job
+};
+__global__ void __launch_bounds__(kScanThreads) scan_jobs_kernel(ScanJobs J, int inclusive) {
+  __shared__ int s_warp[32];
+  const int j = blockIdx.x;
+  int run = 0;
+  for (int base = 0; base < J.n[j]; base += kScanBlock)
+    run += scan_tile(J.in[j], J.n[j], J.out[j], base, run, inclusive, s_warp);
+  if (J.total && threadIdx.x == 0) J.total[j] = run;
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(const int* __restrict__ in, int n,
+                                                                 int* __restrict__ sums) {
+  __shared__ int s_warp[32];
+  const int i0 = blockIdx.x * kScanBlock + threadIdx.x;
+  int v = 0, total;
+#pragma unroll
+  for (int e = 0; e < kScanItems; ++e)
+    if (i0 + e * kScanThreads < n) v += in[i0 + e * kScanThreads];
+  block_inclusive(v, s_warp, total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+// (every block adds up the sums of the blocks before it: at most 512)
+__global__ void __launch_bounds__(kScanThreads)
+    scan_blocks_kernel(const int* __restrict__ in, int n, int* __restrict__ out,
+                       const int* __restrict__ sums, int inclusive, int* __restrict__ total) {
+  __shared__ int s_warp[32];
+  int before;
+  block_inclusive(threadIdx.x < blockIdx.x ? sums[threadIdx.x] : 0, s_warp, before);
+  const int sum = scan_tile(in, n, out, blockIdx.x * kScanBlock, before, inclusive, s_warp);
+  if (total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = before + sum;
 }
 
 }  // namespace tree
 
-// Device-wide scan of n <= 2048*2048 ints (in -> out); tmp holds >= 2*2048 ints.
-int scan_ints(const int* in, int n, int* out, int inclusive, int* tmp, cudaStream_t s) {
+// Device-wide scans of n <= 2^22 ints each (in -> out); tmp holds >= 512 ints;
+// total: null, or where the arrays' sums go.  Arrays of at most kScanOneCta
+// elements share one launch, a CTA each: 32,768 elements take 10 us (12 in the
+// three launches of a scan by blocks, a scan of their sums and an addition, the
+// launches' gaps apart); longer ones take two launches.
+int scan_many(const tree::ScanJobs& J, int jobs, int inclusive, int* tmp, cudaStream_t s) {
   using namespace tree;
-  if (n <= 0) return FVX_OK;
-  const int nb = (n + kScanBlock - 1) / kScanBlock;
-  FVX_ARG_CHECK(nb <= kScanBlock, "scan of %d elements exceeds 2^22", n);
-  int* bsum = tmp;
-  int* bsum_ex = tmp + kScanBlock;
-  scan_block_kernel<<<nb, kScanBlock / 2, 0, s>>>(in, n, out, bsum, inclusive);
-  FVX_LAUNCH_CHECK();
-  if (nb > 1) {
-    scan_block_kernel<<<1, kScanBlock / 2, 0, s>>>(bsum, nb, bsum_ex, nullptr, 0);
+  bool one = true;
+  for (int j = 0; j < jobs; ++j) one &= J.n[j] <= kScanOneCta;
+  if (one) {
+    scan_jobs_kernel<<<jobs, kScanThreads, 0, s>>>(J, inclusive);
     FVX_LAUNCH_CHECK();
-    scan_add_kernel<<<(n + 255) / 256, 256, 0, s>>>(out, n, bsum_ex);
+    return FVX_OK;
+  }
+  for (int j = 0; j < jobs; ++j) {
+    const int nb = (J.n[j] + kScanBlock - 1) / kScanBlock;
+    FVX_ARG_CHECK(J.n[j] <= (1 << 22), "scan of %d elements exceeds 2^22", J.n[j]);
+    int* total = J.total ? J.total + j : nullptr;
+    if (nb == 0) {
+      if (total) FVX_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(int), s));
+      continue;
+    }
+    scan_sums_kernel<<<nb, kScanThreads, 0, s>>>(J.in[j], J.n[j], tmp);
+    FVX_LAUNCH_CHECK();
+    scan_blocks_kernel<<<nb, kScanThreads, 0, s>>>(J.in[j], J.n[j], J.out[j], tmp, inclusive,
+                                                   total);
     FVX_LAUNCH_CHECK();
   }
   return FVX_OK;
+}
+
+int scan_ints(const int* in, int n, int* out, int inclusive, int* tmp, cudaStream_t s) {
+  if (n <= 0) return FVX_OK;
+  tree::ScanJobs J{};
+  J.in[0] = in;
+  J.out[0] = out;
+  J.n[0] = n;
+  return scan_many(J, 1, inclusive, tmp, s);
 }
 
 namespace tree {
@@ -274,7 +352,7 @@ __global__ void __launch_bounds__(256) radix_scatter_kernel(
 
 // Stable LSD radix sort of (key, index) pairs by 32-bit keys, four 8-bit
 // passes: the pairs are read from (keys, idx) and returned there, (keys_tmp,
-// idx_tmp) hold n each, table sort_table_ints(n) ints, scan_tmp 2 x 2048 ints.
+// idx_tmp) hold n each, table sort_table_ints(n) ints, scan_tmp 512 ints.
 int sort_table_ints(int n) { return 256 * ((n + tree::kSortItems - 1) / tree::kSortItems) * 2; }
 
 // passes: 8-bit digits sorted (an even number: the result is back in (keys, idx))
@@ -360,28 +438,6 @@ __global__ void __launch_bounds__(256) level_hist_kernel(const uint32_t* __restr
   }
   __syncthreads();
   if (threadIdx.x <= L) table[threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];
-}
-
-// Inclusive sum over the CTA (a multiple of 32 threads, at most 1024).
-__device__ __forceinline__ int block_inclusive(int v, int* s_warp, int& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += u;
-  }
-  if (lane == 31) s_warp[warp] = v;
-  __syncthreads();
-  int w = lane < nw ? s_warp[lane] : 0;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, w, o);
-    if (lane >= o) w += u;
-  }
-  total = __shfl_sync(0xffffffffu, w, nw - 1);
-  const int before = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
-  __syncthreads();  // s_warp may be written again
-  return warp ? v + before : v;
 }
 
 // A CTA per level: exclusive sums of its row of the table, in place, and the
@@ -2411,6 +2467,7 @@ int judge_sums_launch(const JudgeSampleView& S, const uint32_t* leaf_key, const 
 
 struct fvx_tree {
   int device = 0;
+  int* host = nullptr;  // pinned words that the host reads back
   fvx::DevBuf keys0, keys1, idx0, idx1, table, scan_tmp, cid, levels, counts, rec, sp, sa,
       sg, lists_meta, near_list, far_list, bbox;
   int64_t stats[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -2654,12 +2711,14 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   bbox_final_kernel<<<1, kBboxFinalThreads, 0, s>>>(nbb, P<double>(T->bbox),
                                                     P<double>(T->bbox) + 7 * nbb);
   FVX_LAUNCH_CHECK();
+  // (one copy to pinned memory: the box, and the count right after it)
+  if (!T->host) FVX_CUDA_TRY(cudaMallocHost(&T->host, 64));
+  FVX_CUDA_TRY(cudaMemcpyAsync(T->host, P<double>(T->bbox) + 7 * nbb, 64, cudaMemcpyDeviceToHost, s));
+  FVX_CUDA_TRY(cudaStreamSynchronize(s));
   double lohi[7];
   unsigned nbad = 0;
-  FVX_CUDA_TRY(cudaMemcpyAsync(lohi, P<double>(T->bbox) + 7 * nbb, sizeof(lohi),
-                               cudaMemcpyDeviceToHost, s));
-  FVX_CUDA_TRY(cudaMemcpyAsync(&nbad, nonfinite, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  FVX_CUDA_TRY(cudaStreamSynchronize(s));
+  memcpy(lohi, T->host, sizeof(lohi));
+  memcpy(&nbad, T->host + 14, sizeof(nbad));
   // a non-finite position would otherwise collapse the grid (all keys in one
   // cell) and turn the sweep into an all-pairs sum on a few CTAs
   FVX_ARG_CHECK(nbad == 0, "treecode: %u particles with non-finite positions", nbad);
@@ -2678,9 +2737,9 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   if ((rc = grow(T->keys0, 4 * size_t(n))) || (rc = grow(T->keys1, 4 * size_t(n))) ||
       (rc = grow(T->idx0, 4 * size_t(n))) || (rc = grow(T->idx1, 4 * size_t(n))) ||
       (rc = grow(T->table, 4 * size_t(256) * nblk * 2)) ||
-      (rc = grow(T->scan_tmp, 4 * size_t(2 * kScanBlock))) ||
+      (rc = grow(T->scan_tmp, 4 * 512)) ||
       (rc = grow(T->cid, 4 * size_t(n))) || (rc = grow(T->levels, 4 * size_t(total_cells) * 7)) ||
-      (rc = grow(T->counts, 4 * 16)) ||
+      (rc = grow(T->counts, 4 * (kMaxLevels + 4))) ||
       (rc = grow(T->rec, 4 * size_t(total_cells) * kRecFloats)) ||
       (rc = grow(T->sp, 16 * size_t(n))) || (rc = grow(T->sa, 16 * size_t(n))) ||
       (rc = grow(T->sg, 16 * size_t(n))))
@@ -2724,8 +2783,9 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   level_finish_kernel<<<static_cast<int>(std::min<int64_t>((n + 255) / 256, 4 * device_sm_count())),
                         256, 0, s>>>(C, n, ncells_d);
   FVX_LAUNCH_CHECK();
-  FVX_CUDA_TRY(cudaMemcpyAsync(ncells, ncells_d, sizeof(int) * (L + 1), cudaMemcpyDeviceToHost, s));
+  FVX_CUDA_TRY(cudaMemcpyAsync(T->host, ncells_d, sizeof(int) * (L + 1), cudaMemcpyDeviceToHost, s));
   FVX_CUDA_TRY(cudaStreamSynchronize(s));
+  memcpy(ncells, T->host, sizeof(int) * (L + 1));
   nleaf = ncells[L];
   }
   int* cid = P<int>(T->cid);
@@ -2850,26 +2910,22 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
     FVX_LAUNCH_CHECK();
     iota_scaled_kernel<<<(nleaf + 255) / 256, 256, 0, s>>>(nleaf, kSlotNear, near_off);
     FVX_LAUNCH_CHECK();
-    if ((rc = scan_ints(LL.cnt, nleaf, P<int>(T->lrn_meta) + nleaf, 0, P<int>(T->scan_tmp), s)))
-      return rc;
-    if ((rc = scan_ints(par_cnt, npar, par_off, 0, P<int>(T->scan_tmp), s))) return rc;
-    // the near total through a scan into far_off (no far cells on this path)
-    if ((rc = scan_ints(near_cnt, nleaf, far_off, 0, P<int>(T->scan_tmp), s))) return rc;
-    int tl[6] = {0, 0, 0, 0, 0, 0};
-    unsigned flags = 0;
-    FVX_CUDA_TRY(cudaMemcpyAsync(&tl[0], LL.cnt + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
-    FVX_CUDA_TRY(cudaMemcpyAsync(&tl[1], LL.off + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
-    FVX_CUDA_TRY(cudaMemcpyAsync(&tl[2], par_cnt + npar - 1, 4, cudaMemcpyDeviceToHost, s));
-    FVX_CUDA_TRY(cudaMemcpyAsync(&tl[3], par_off + npar - 1, 4, cudaMemcpyDeviceToHost, s));
-    FVX_CUDA_TRY(cudaMemcpyAsync(&tl[4], near_cnt + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
-    FVX_CUDA_TRY(cudaMemcpyAsync(&tl[5], far_off + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
-    FVX_CUDA_TRY(cudaMemcpyAsync(&flags, ovf, 4, cudaMemcpyDeviceToHost, s));
+    // (the near total through a scan into far_off: no far cells on this path)
+    const ScanJobs J{{LL.cnt, par_cnt, near_cnt, nullptr},
+                     {P<int>(T->lrn_meta) + nleaf, par_off, far_off, nullptr},
+                     {nleaf, npar, nleaf, 0},
+                     P<int>(T->counts) + kMaxLevels};
+    if ((rc = scan_many(J, 3, 0, P<int>(T->scan_tmp), s))) return rc;
+    FVX_CUDA_TRY(cudaMemcpyAsync(T->host, J.total, 12, cudaMemcpyDeviceToHost, s));
+    FVX_CUDA_TRY(cudaMemcpyAsync(T->host + 4, ovf, 4, cudaMemcpyDeviceToHost, s));
     FVX_CUDA_TRY(cudaStreamSynchronize(s));
+    const int* tl = T->host;
+    const unsigned flags = static_cast<unsigned>(T->host[4]);
     if (!(flags & 4u)) {
-      near_total = int64_t(tl[4]) + tl[5];
+      lrn_total = tl[0];
+      par_total = tl[1];
+      near_total = tl[2];
       far_total = 0;
-      lrn_total = int64_t(tl[0]) + tl[1];
-      par_total = int64_t(tl[2]) + tl[3];
       if ((rc = grow(T->lrn_leaf, 4 * size_t(lrn_total + 1))) ||
           (rc = grow(T->lrn_cell, 4 * size_t(lrn_total + 1))) ||
           (rc = grow(T->par_par, 4 * size_t(par_total + 1))) ||
@@ -2907,37 +2963,24 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
         V, nullptr, nullptr, near_cnt, far_cnt, nullptr, nullptr, 0, 0, ovf, LL);
   }
   FVX_LAUNCH_CHECK();
-  if ((rc = scan_ints(near_cnt, nleaf, near_off, 0, P<int>(T->scan_tmp), s))) return rc;
-  if ((rc = scan_ints(far_cnt, nleaf, far_off, 0, P<int>(T->scan_tmp), s))) return rc;
-  int ltail[4] = {0, 0, 0, 0};
-  if (learned) {
-    if ((rc = scan_ints(LL.cnt, nleaf, P<int>(T->lrn_meta) + nleaf, 0, P<int>(T->scan_tmp), s)))
-      return rc;
-    FVX_CUDA_TRY(cudaMemcpyAsync(&ltail[0], LL.cnt + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
-    FVX_CUDA_TRY(cudaMemcpyAsync(&ltail[1], LL.off + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
-  }
-  if (dual) {
-    if ((rc = scan_ints(par_cnt, npar, par_off, 0, P<int>(T->scan_tmp), s))) return rc;
-    FVX_CUDA_TRY(cudaMemcpyAsync(&ltail[2], par_cnt + npar - 1, 4, cudaMemcpyDeviceToHost, s));
-    FVX_CUDA_TRY(cudaMemcpyAsync(&ltail[3], par_off + npar - 1, 4, cudaMemcpyDeviceToHost, s));
-  }
-  int tail[4];
-  FVX_CUDA_TRY(cudaMemcpyAsync(&tail[0], near_cnt + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
-  FVX_CUDA_TRY(cudaMemcpyAsync(&tail[1], near_off + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
-  FVX_CUDA_TRY(cudaMemcpyAsync(&tail[2], far_cnt + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
-  FVX_CUDA_TRY(cudaMemcpyAsync(&tail[3], far_off + nleaf - 1, 4, cudaMemcpyDeviceToHost, s));
+  const int* lt = T->host;
+  const ScanJobs J{{near_cnt, far_cnt, LL.cnt, par_cnt},
+                   {near_off, far_off, learned ? P<int>(T->lrn_meta) + nleaf : nullptr, par_off},
+                   {nleaf, nleaf, learned ? nleaf : 0, npar},
+                   P<int>(T->counts) + kMaxLevels};
+  if ((rc = scan_many(J, 4, 0, P<int>(T->scan_tmp), s))) return rc;
+  FVX_CUDA_TRY(cudaMemcpyAsync(T->host, J.total, 16, cudaMemcpyDeviceToHost, s));
   FVX_CUDA_TRY(cudaStreamSynchronize(s));
-  near_total = int64_t(tail[0]) + tail[1];
-  far_total = int64_t(tail[2]) + tail[3];
-  FVX_ARG_CHECK(near_total < (int64_t(1) << 31) && far_total < (int64_t(1) << 31),
-                "interaction lists too long");
+  near_total = lt[0];
+  far_total = lt[1];
+  // (a sum past 2^31 shows as a negative one)
+  FVX_ARG_CHECK(near_total >= 0 && far_total >= 0, "interaction lists too long");
   if ((rc = grow(T->near_list, 4 * size_t(near_total + 1))) ||
       (rc = grow(T->far_list, 4 * size_t(far_total + 1))))
     return rc;
-  lrn_total = int64_t(ltail[0]) + ltail[1];
-  par_total = int64_t(ltail[2]) + ltail[3];
-  FVX_ARG_CHECK(lrn_total < (int64_t(1) << 31) && par_total < (int64_t(1) << 31),
-                "local-expansion pair list too long");
+  lrn_total = lt[2];
+  par_total = lt[3];
+  FVX_ARG_CHECK(lrn_total >= 0 && par_total >= 0, "local-expansion pair list too long");
   if (learned) {
     if ((rc = grow(T->lrn_leaf, 4 * size_t(lrn_total + 1))) ||
         (rc = grow(T->lrn_cell, 4 * size_t(lrn_total + 1))))
@@ -3300,6 +3343,7 @@ void fvx_tree_destroy(fvx_tree* T) {
                          &T->pair_partial};
   for (auto* b : bufs)
     if (b->p) cudaFree(b->p);
+  if (T->host) cudaFreeHost(T->host);
   delete T;
 }
 
