@@ -355,18 +355,17 @@ __global__ void __launch_bounds__(256) radix_scatter_kernel(
 // idx_tmp) hold n each, table sort_table_ints(n) ints, scan_tmp 512 ints.
 int sort_table_ints(int n) { return 256 * ((n + tree::kSortItems - 1) / tree::kSortItems) * 2; }
 
-// passes: 8-bit digits sorted (an even number: the result is back in (keys, idx))
 int sort_pairs_u32(uint32_t* keys, int* idx, uint32_t* keys_tmp, int* idx_tmp, int n, int* table,
-                   int* scan_tmp, cudaStream_t s, int passes = 4);
+                   int* scan_tmp, cudaStream_t s);
 int sort_pairs_u32(uint32_t* keys, int* idx, uint32_t* keys_tmp, int* idx_tmp, int n, int* table,
-                   int* scan_tmp, cudaStream_t s, int passes) {
+                   int* scan_tmp, cudaStream_t s) {
   using namespace tree;
   if (n <= 0) return FVX_OK;
   const int nblk = (n + kSortItems - 1) / kSortItems;
   int* table_ex = table + 256 * nblk;
   uint32_t *ka = keys, *kb = keys_tmp;
   int *ia = idx, *ib = idx_tmp;
-  for (int pass = 0; pass < passes; ++pass) {
+  for (int pass = 0; pass < 4; ++pass) {
     radix_hist_kernel<<<nblk, 256, 0, s>>>(ka, n, 8 * pass, nblk, table);
     FVX_LAUNCH_CHECK();
     int rc = scan_ints(table, 256 * nblk, table_ex, 0, scan_tmp, s);
@@ -380,7 +379,7 @@ int sort_pairs_u32(uint32_t* keys, int* idx, uint32_t* keys_tmp, int* idx_tmp, i
     ia = ib;
     ib = ti;
   }
-  return FVX_OK;  // an even number of passes: the result is back in (keys, idx)
+  return FVX_OK;  // after an even number of passes the result is back in (keys, idx)
 }
 
 namespace tree {
@@ -842,16 +841,61 @@ __global__ void cell_centres_kernel(TreeView T, int total_cells, int4* __restric
                      (2 * static_cast<int>(compact10(k >> 2)) + 1) * sc, kids);
 }
 
-// Sort keys of the evaluation order: leaves by decreasing near-field work
-// (near leaves x own particles, 16 bits), ties in leaf order.
-__global__ void order_keys_kernel(int nleaf, const int* __restrict__ near_cnt,
-                                  const int* __restrict__ leaf_count, uint32_t* __restrict__ keys,
-                                  int* __restrict__ idx) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nleaf) return;
-  const long long w = static_cast<long long>(near_cnt[t]) * leaf_count[t];
-  keys[t] = 0xFFFFu - static_cast<uint32_t>(w < 0xFFFF ? w : 0xFFFF);
-  idx[t] = t;
+// The evaluation's work items: chunks of 32 and of 64 of a leaf's particles (what a
+// warp evaluates at a time, by mode), each list in decreasing order of near-field
+// work (near leaves x particles) to a 64th of 16,384, any order within.
+constexpr int kItemBuckets = 256;
+struct Items {
+  int2* item[2];  // (leaf, first particle) of the chunks of 32 and of 64
+  int* hist;      // [2][kItemBuckets], zero before
+  int* cursor;    // [2][kItemBuckets], zero before
+  int* count;     // [2]
+};
+
+__device__ __forceinline__ int item_bucket(int near, int particles) {
+  const long long w = static_cast<long long>(near) * particles >> 6;
+  return kItemBuckets - 1 - static_cast<int>(w < kItemBuckets ? w : kItemBuckets - 1);
+}
+
+template <bool FILL>
+__global__ void __launch_bounds__(kItemBuckets)
+    items_kernel(int nleaf, const int* __restrict__ near_cnt, const int* __restrict__ leaf_count,
+                 Items I) {
+  __shared__ int s_n[2][kItemBuckets], s_at[2][kItemBuckets], s_warp[32];
+  const int tid = threadIdx.x;
+  for (int l = 0; l < 2; ++l) s_n[l][tid] = 0;
+  __syncthreads();
+  const int t = blockIdx.x * kItemBuckets + tid;
+  const int near = t < nleaf ? near_cnt[t] : 0, n = t < nleaf ? leaf_count[t] : 0;
+  for (int l = 0; l < 2; ++l) {
+    const int step = 32 << l, full = n / step, rest = n - full * step;
+    if (full) atomicAdd(&s_n[l][item_bucket(near, step)], full);
+    if (rest) atomicAdd(&s_n[l][item_bucket(near, rest)], 1);
+  }
+  __syncthreads();
+  if (!FILL) {
+    for (int l = 0; l < 2; ++l)
+      if (s_n[l][tid]) atomicAdd(I.hist + l * kItemBuckets + tid, s_n[l][tid]);
+    return;
+  }
+  for (int l = 0; l < 2; ++l) {
+    int total;
+    const int h = I.hist[l * kItemBuckets + tid];
+    const int first = block_inclusive(h, s_warp, total) - h;
+    const int own = s_n[l][tid];
+    s_at[l][tid] = own ? first + atomicAdd(I.cursor + l * kItemBuckets + tid, own) : 0;
+    if (t == 0) I.count[l] = total;
+  }
+  __syncthreads();
+  for (int l = 0; l < 2; ++l) {
+    const int step = 32 << l, full = n / step, rest = n - full * step;
+    if (full) {
+      const int at = atomicAdd(&s_at[l][item_bucket(near, step)], full);
+      for (int c = 0; c < full; ++c) I.item[l][at + c] = make_int2(t, c * step);
+    }
+    if (rest)
+      I.item[l][atomicAdd(&s_at[l][item_bucket(near, rest)], 1)] = make_int2(t, full * step);
+  }
 }
 
 template <bool FILL>
@@ -1209,9 +1253,9 @@ struct EvalArgs {
   const float* leaf_local;  // [leaves][32] learned local expansions, or null
   const float* parent_local;  // [parents][32] expansions shared by a parent's leaves, or null
   const int* leaf_parent;     // parent index of each leaf (with parent_local)
-  int nleaf;
-  int* leaf_next;             // leaf counter of the resident evaluation warps (zeroed)
-  const int* leaf_order;      // the order the warps take the leaves in
+  int* item_next;             // leaf counter of the resident evaluation warps (zeroed)
+  const int2* items[2];       // (leaf, first particle) in chunks of 32 and 64, most work first
+  const int* n_items;         // [2]
 };
 
 // Learned local expansion of the leaf at offset d = x - c_T (u, J = du/dx,
@@ -1658,10 +1702,18 @@ struct EvalSmem {
   static constexpr int bytes = kNearBytes > kFarBytes ? kNearBytes : kFarBytes;
 };
 
-// Leaf t: its targets against its near leaves and far cells, plus the local
-// expansions (one warp).
+// A warp's targets: 16 TPT of a leaf on the paired path, 32 TPT on the others: the
+// list of chunks of 32 << eval_list.
+template <bool PACKED, int TPT>
+constexpr int eval_list() {
+  return (PACKED ? 16 : 32) * TPT == 64 ? 1 : 0;
+}
+
+// The chunk of leaf t's targets from its particle `chunk` on, against the leaf's
+// near leaves and far cells, plus the local expansions (one warp).
 template <int MODE, int KERNEL, int TPT, bool FACT>
-__device__ __forceinline__ void eval_leaf(const EvalArgs& A, int t, unsigned char* s_raw) {
+__device__ __forceinline__ void eval_chunk(const EvalArgs& A, int t, int chunk,
+                                           unsigned char* s_raw) {
   using namespace pair;
   constexpr int NC = ModeInfo<MODE>::ncomp;
   constexpr int NA = ModeInfo<MODE>::na;
@@ -1684,11 +1736,10 @@ __device__ __forceinline__ void eval_leaf(const EvalArgs& A, int t, unsigned cha
   // field.  Lanes past the g groups mirror group 0 and are not counted.  The
   // other paths take TPT targets per lane.
   constexpr int NP = TPT / 2;  // pairs of targets per lane (paired path)
-  const int chunk_step = PACKED ? (kEvalThreads / 2) * TPT : kEvalThreads * TPT;
   const int lane = threadIdx.x;
 
-  for (int chunk = 0; chunk < tcount; chunk += chunk_step) {
-    const int cend = min(tcount, chunk + chunk_step);
+  {
+    const int cend = min(tcount, chunk + (32 << eval_list<PACKED, TPT>()));
     int m = kEvalThreads, g = 1, grp = 0, tl = lane;
     bool spare = false;
     if constexpr (PACKED) {
@@ -2023,26 +2074,32 @@ __device__ __forceinline__ void eval_leaf(const EvalArgs& A, int t, unsigned cha
   }
 }
 
-// Resident evaluation warps (one per CTA) take leaves from a shared counter
-// until none are left: the SMs stay at their occupancy limit to the end, and
-// no CTA is launched per leaf.  The leaves come in decreasing order of their
-// near-field work, so the last ones taken are the shortest.
+// Resident evaluation warps (one per CTA) take chunks of leaves from a shared
+// counter until none are left: the SMs stay at their occupancy limit to the end,
+// and no CTA is launched per chunk.  The chunks come in decreasing order of their
+// near-field work, so the last ones taken are the shortest.  (Whole leaves, some
+// of them many times the mean, left the SMs idle for a fifth of a sweep of 131,072
+// particles: stretching 636 us against 568, velocity 407 against 386, vorticity
+// 862 against 765.)
 template <int MODE, int KERNEL, int TPT, bool FACT>
-__device__ __forceinline__ void eval_leaves(const EvalArgs& A) {
+__device__ __forceinline__ void eval_items(const EvalArgs& A) {
   __shared__ __align__(16) unsigned char s_raw[EvalSmem<MODE, KERNEL, TPT>::bytes];
+  constexpr int list = eval_list<EvalSmem<MODE, KERNEL, TPT>::PACKED, TPT>();
+  const int n = A.n_items[list];
   for (;;) {
     int c = 0;
-    if (threadIdx.x == 0) c = atomicAdd(A.leaf_next, 1);
+    if (threadIdx.x == 0) c = atomicAdd(A.item_next, 1);
     c = __shfl_sync(0xffffffffu, c, 0);
-    if (c >= A.nleaf) break;
-    eval_leaf<MODE, KERNEL, TPT, FACT>(A, A.leaf_order[c], s_raw);
-    __syncthreads();  // the next leaf restages the shared buffer
+    if (c >= n) break;
+    const int2 item = A.items[list][c];
+    eval_chunk<MODE, KERNEL, TPT, FACT>(A, item.x, item.y, s_raw);
+    __syncthreads();  // the next chunk restages the shared buffer
   }
 }
 
 template <int MODE, int KERNEL, int TPT>
 __global__ void __launch_bounds__(kEvalThreads) eval_kernel(EvalArgs A) {
-  eval_leaves<MODE, KERNEL, TPT, false>(A);
+  eval_items<MODE, KERNEL, TPT, false>(A);
 }
 
 // The factored loops (paired Winckelmans): stretching with two targets per
@@ -2053,7 +2110,7 @@ __global__ void __launch_bounds__(kEvalThreads) eval_kernel(EvalArgs A) {
 template <int MODE, int KERNEL, int TPT>
 __global__ void __launch_bounds__(kEvalThreads, TPT == 4 ? 20 : 24)
     eval_kernel_factored(EvalArgs A) {
-  eval_leaves<MODE, KERNEL, TPT, true>(A);
+  eval_items<MODE, KERNEL, TPT, true>(A);
 }
 
 // ---- the FP64 judge of the local-expansion path ------------------------------------
@@ -2493,8 +2550,8 @@ struct fvx_tree {
   // two-level traversal: per-parent lists and expansions
   fvx::DevBuf dual_meta, par_par, par_cell, parent_local;
   fvx::DevBuf cen;  // cell centres in units of h/2 (dual traversal)
-  fvx::DevBuf eval_next;  // leaf counter of the evaluation kernel
-  fvx::DevBuf leaf_order, order_table;  // evaluation order of the leaves (+ sort scratch)
+  fvx::DevBuf eval_next;  // work counter of the evaluation kernel
+  fvx::DevBuf items;      // the evaluation's work items (see items_bytes)
   fvx::DevBuf pair_partial;  // slices of the FP64 exact-expansion sums
   int n_parent_pairs = 0;
   fvx::DevBuf lrn_meta, lrn_leaf, lrn_cell, leaf_local;
@@ -2529,6 +2586,22 @@ struct fvx_tree {
 namespace fvx {
 namespace {
 
+// T->items: hist and cursor (2 x 256 each), the counts, then the items: a leaf of c
+// particles has at most c / 32 + 1 chunks of 32.
+size_t items_bytes(int n, int nleaf) {
+  return sizeof(int) * (4 * tree::kItemBuckets + 2) +
+         sizeof(int2) * (2 * size_t(nleaf) + n / 32 + n / 64 + 2);
+}
+tree::Items item_lists(const fvx_tree* T, int n, int nleaf) {
+  tree::Items I;
+  I.hist = static_cast<int*>(T->items.p);
+  I.cursor = I.hist + 2 * tree::kItemBuckets;
+  I.count = I.hist + 4 * tree::kItemBuckets;
+  I.item[0] = reinterpret_cast<int2*>(I.count + 2);
+  I.item[1] = I.item[0] + nleaf + n / 32 + 1;
+  return I;
+}
+
 template <int KERNEL>
 void launch_gather(int n, const int* perm, const int* leaf_of, const uint32_t* leaf_key,
                    tree::Grid g, const double* pos, const double* alpha, const double* sigma,
@@ -2537,22 +2610,22 @@ void launch_gather(int n, const int* perm, const int* leaf_of, const uint32_t* l
                                                              alpha, sigma, tgam, sp, sa, sg);
 }
 
-// Resident CTAs: the occupancy limit per SM times the SMs (at most one per leaf).
+// Resident CTAs: the occupancy limit per SM times the SMs (at most one per item).
 template <typename K>
-int resident_grid(K kernel, int nleaf) {
+int resident_grid(K kernel, int items) {
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tree::kEvalThreads, 0) !=
           cudaSuccess ||
       per_sm < 1)
     per_sm = 1;
   const int64_t g = static_cast<int64_t>(per_sm) * device_sm_count();
-  return static_cast<int>(g < nleaf ? g : nleaf);
+  return static_cast<int>(g < items ? g : items);
 }
 
 // Targets per thread: leaves of at most ~40 particles on average fill one
 // 32-target chunk per warp better than two.
 template <int KERNEL, int TPT>
-void launch_eval_tpt(int mode, int nleaf, const tree::EvalArgs& A, bool factored,
+void launch_eval_tpt(int mode, int items, const tree::EvalArgs& A, bool factored,
                      cudaStream_t s) {
   using namespace tree;
   constexpr bool F = KERNEL == FVX_KERNEL_WINCKELMANS && TPT == 2;  // the paired kernels
@@ -2561,24 +2634,24 @@ void launch_eval_tpt(int mode, int nleaf, const tree::EvalArgs& A, bool factored
       auto k = eval_kernel<FVX_PAIR_VELOCITY, KERNEL, TPT>;
       if constexpr (F)
         if (factored) k = eval_kernel_factored<FVX_PAIR_VELOCITY, KERNEL, 4>;
-      k<<<resident_grid(k, nleaf), kEvalThreads, 0, s>>>(A);
+      k<<<resident_grid(k, items), kEvalThreads, 0, s>>>(A);
       break;
     }
     case FVX_PAIR_STRETCH: {
       auto k = eval_kernel<FVX_PAIR_STRETCH, KERNEL, TPT>;
       if constexpr (F)
         if (factored) k = eval_kernel_factored<FVX_PAIR_STRETCH, KERNEL, TPT>;
-      k<<<resident_grid(k, nleaf), kEvalThreads, 0, s>>>(A);
+      k<<<resident_grid(k, items), kEvalThreads, 0, s>>>(A);
       break;
     }
     case FVX_PAIR_VELOCITY_STRETCH: {
       auto k = eval_kernel<FVX_PAIR_VELOCITY_STRETCH, KERNEL, TPT>;
-      k<<<resident_grid(k, nleaf), kEvalThreads, 0, s>>>(A);
+      k<<<resident_grid(k, items), kEvalThreads, 0, s>>>(A);
       break;
     }
     default: {
       auto k = eval_kernel<FVX_PAIR_VORTICITY, KERNEL, TPT>;
-      k<<<resident_grid(k, nleaf), kEvalThreads, 0, s>>>(A);
+      k<<<resident_grid(k, items), kEvalThreads, 0, s>>>(A);
       break;
     }
   }
@@ -2594,10 +2667,11 @@ void launch_eval(int mode, int nleaf, int n, const tree::EvalArgs& A, bool facto
   const bool paired = (KERNEL == FVX_KERNEL_WINCKELMANS &&
                        (mode == FVX_PAIR_VELOCITY || mode == FVX_PAIR_STRETCH)) ||
                       (KERNEL == FVX_KERNEL_GAUSSIANERF && mode == FVX_PAIR_VORTICITY);
+  const int items = nleaf + n / 32;  // at most
   if (!paired && n <= 40 * nleaf)
-    launch_eval_tpt<KERNEL, 1>(mode, nleaf, A, false, s);
+    launch_eval_tpt<KERNEL, 1>(mode, items, A, false, s);
   else
-    launch_eval_tpt<KERNEL, 2>(mode, nleaf, A, factored, s);
+    launch_eval_tpt<KERNEL, 2>(mode, items, A, factored, s);
 }
 
 template <int KERNEL>
@@ -3035,19 +3109,16 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   ST.far_total = far_total;
   ST.lrn_total = lrn_total;
   ST.par_total = par_total;
-  // the evaluation order: leaves by decreasing near-field work
-  if ((rc = grow(T->leaf_order, 4 * 4 * size_t(nleaf))) ||
-      (rc = grow(T->order_table, 4 * size_t(sort_table_ints(nleaf)))))
-    return rc;
+  // the evaluation's work items
+  if ((rc = grow(T->items, items_bytes(n, nleaf)))) return rc;
   {
-    uint32_t* ok0 = P<uint32_t>(T->leaf_order) + 2 * size_t(nleaf);
-    int* oi0 = P<int>(T->leaf_order);
-    order_keys_kernel<<<(nleaf + 255) / 256, 256, 0, s>>>(
-        nleaf, near_cnt, lvb + total_cells + base[L], ok0, oi0);
+    const Items I = item_lists(T, n, nleaf);
+    const int grid = (nleaf + kItemBuckets - 1) / kItemBuckets;
+    FVX_CUDA_TRY(cudaMemsetAsync(I.hist, 0, sizeof(int) * 4 * kItemBuckets, s));
+    items_kernel<false><<<grid, kItemBuckets, 0, s>>>(nleaf, near_cnt, leaves.count, I);
     FVX_LAUNCH_CHECK();
-    if ((rc = sort_pairs_u32(ok0, oi0, ok0 + nleaf, oi0 + nleaf, nleaf, P<int>(T->order_table),
-                             P<int>(T->scan_tmp), s, 2)))
-      return rc;
+    items_kernel<true><<<grid, kItemBuckets, 0, s>>>(nleaf, near_cnt, leaves.count, I);
+    FVX_LAUNCH_CHECK();
   }
   ST.valid = true;
   }
@@ -3248,9 +3319,10 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   // the resident evaluation warps' leaf counter
   if ((rc = grow(T->eval_next, 16))) return rc;
   FVX_CUDA_TRY(cudaMemsetAsync(T->eval_next.p, 0, sizeof(int), s));
-  A.nleaf = nleaf;
-  A.leaf_next = P<int>(T->eval_next);
-  A.leaf_order = P<int>(T->leaf_order);
+  A.item_next = P<int>(T->eval_next);
+  const Items items = item_lists(T, n, nleaf);
+  for (int l = 0; l < 2; ++l) A.items[l] = items.item[l];
+  A.n_items = items.count;
   FVX_CUDA_TRY(cudaEventRecord(T->ev0, s));
   // the factored stretching loop where leaves are at most 4 smallest cores
   // wide (the cores of the last full build; see near_tile_x2_factored)
@@ -3338,7 +3410,7 @@ void fvx_tree_destroy(fvx_tree* T) {
                          &T->judge_Y, &T->judge_err, &T->fb_queue, &T->fb_count,
                          &T->dual_meta, &T->par_par, &T->par_cell, &T->parent_local,
                          &T->cen, &T->res_slot, &T->res_cnt, &T->eval_next,
-                         &T->leaf_order, &T->order_table,
+                         &T->items,
                          &T->lrn_slot, &T->par_slot,
                          &T->pair_partial};
   for (auto* b : bufs)
