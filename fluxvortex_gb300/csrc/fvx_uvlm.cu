@@ -416,16 +416,18 @@ __global__ void __launch_bounds__(kLuThreads) lu_solve_kernel(int P, int T, doub
 // What a step costs is its chain -- pivot, reciprocal, multipliers, their way to
 // the other CTAs -- so that is all that stands between two steps: the owner of
 // column k + 1 brings that column up to date first, finds its pivot by integer
-// comparisons (one warp), forms the multipliers, writes them into every CTA's
-// shared memory and arrives at the cluster barrier; everybody's other columns
+// comparisons, forms the multipliers, writes them into every CTA's shared
+// memory and arrives at the cluster barrier; everybody's other columns
 // follow while the barrier fills.  Rows are permuted by index; every element sees
 // the operations of the single-CTA form in its order, so the factors and the
 // solution are the same.  The multipliers
 // go round three buffers: step k + 3's writer has passed barrier k + 2, at which
 // every thread arrived after its last use of step k's.
-// 120 unknowns: 199 us, 1.7 us a step (3.2 us while every step's pivot, swap,
-// division and the reading back of the multipliers stood in the chain); the
-// replayed solve takes 51 us (125 us with two barriers a column).
+// 120 unknowns: 168 us, 1.4 us a step (3.2 us while every step's pivot, swap,
+// division and the reading back of the multipliers stood in the chain; 1.7 us with
+// one warp's search and division after the column's update); what is left is
+// mostly the barrier and the stores to the other CTAs before it.  The replayed
+// solve takes 51 us (125 us with two barriers a column).
 namespace cg = cooperative_groups;
 constexpr int kLuCtas = 8;
 constexpr int kLuClusterThreads = 256;
@@ -441,10 +443,12 @@ __host__ __device__ constexpr int64_t lu_workspace_doubles(int P) {
 
 __device__ __forceinline__ int packed_u(int j) { return j * (j + 1) / 2; }  // column j's row 0
 
-// s / d from the correctly rounded reciprocal r of d: q = s r and one step
-// q + (s - q d) r is the correctly rounded quotient (Markstein, 1990), at a third
-// of a division's latency and 3 of its 7 FP64 operations.  Quotients and divisors
-// at the ends of the range (zeros, infinities and NaNs among them) are divided.
+// s / d from the reciprocal r of d, to an ulp: q = s r and one step q + (s - q d) r
+// (Markstein, 1990), the rounded quotient unless that lies within 2^-50 ulp of
+// half way, at 3 FP64 operations instead of a division's 7 (one holds a quarter of
+// an SM's FP64 pipe for 63 to 76 clocks, whatever the number of lanes).  Quotients
+// and divisors at the ends of the range (zeros, infinities and NaNs among them)
+// are divided.
 __device__ __forceinline__ double quotient(double s, double d, double r) {
   const double q = s * r;
   const int h = __double2hiint(q) & 0x7ff00000, hd = __double2hiint(d) & 0x7ff00000;
@@ -490,39 +494,22 @@ __device__ void back_substitute(int P, const double* s_u, double* s_x, int tid) 
   }
 }
 
-// The pivot of a column among logical rows k..P-1 (perm[i]: where row i is):
-// largest magnitude, first row on ties, by integer comparisons of the words
-// (NaNs count as zero); one warp, every lane returns the row, or P if all are zero.
-__device__ __forceinline__ int lu_warp_pivot(const double* col, const int* perm, int k, int P) {
-  constexpr int kRows = kLuClusterMaxP / 32;
-  const int lane = threadIdx.x & 31;
-  unsigned h[kRows], l[kRows];
-  unsigned hm = 0;
-#pragma unroll
-  for (int m = 0; m < kRows; ++m) {
-    const int i = k + lane + 32 * m;
-    h[m] = l[m] = 0;
-    if (i < P) {
-      const double v = col[perm[i]];
-      h[m] = __double2hiint(v) & 0x7fffffff;
-      l[m] = __double2loint(v);
-      if (h[m] > 0x7ff00000u || (h[m] == 0x7ff00000u && l[m] != 0)) h[m] = l[m] = 0;
-    }
-    hm = max(hm, h[m]);
-  }
-  hm = __reduce_max_sync(0xffffffffu, hm);
-  unsigned lm = 0;
-#pragma unroll
-  for (int m = 0; m < kRows; ++m)
-    if (h[m] == hm) lm = max(lm, l[m]);
-  lm = __reduce_max_sync(0xffffffffu, lm);
-  if ((hm | lm) == 0) return P;
-  int piv = P;
-#pragma unroll
-  for (int m = kRows - 1; m >= 0; --m)
-    if (k + lane + 32 * m < P && h[m] == hm && l[m] == lm) piv = k + lane + 32 * m;
-  return __reduce_min_sync(0xffffffffu, piv);
+// 1 / d to an ulp for d in the middle of the range: the hardware's approximation
+// (2^-20 or better) and a step of third order.
+__device__ __forceinline__ double reciprocal(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double e = fma(-d, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 }
+
+// What a warp of the owner offers for the pivot: its largest magnitude by integer
+// comparisons of the words (NaNs count as zero), first row on ties.
+struct LuCandidate {
+  unsigned h, l;
+  int row, place;      // logical row, row of A
+  double value, rcp;
+};
 
 // Dynamic shared memory per CTA: panel[ceil(P/kLuCtas)][P] (column-major),
 // l[3][P], x[P], packed U[P (P + 1) / 2] (x and U used in CTA 0).
@@ -553,7 +540,7 @@ __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThre
   double* s_u = s_x + P;
   __shared__ int s_perm[kLuClusterMaxP];
   __shared__ int s_piv[3];
-  __shared__ double s_rcp;
+  __shared__ LuCandidate s_cand[kLuClusterThreads / 32];
   const int tid = threadIdx.x;
   constexpr int NT = kLuClusterThreads;
   for (int e = tid; e < ncol * P; e += NT) {
@@ -565,65 +552,87 @@ __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThre
     for (int r = tid; r < P; r += NT) s_x[r] = xg[r];
   cl.sync();  // every CTA runs: its shared memory may be written
 
-  // pivot and multipliers of column k (this CTA's, up to date) into every CTA
-  auto prepare = [&](int k) {
-    const double* col = panel + (k / kLuCtas) * P;
-    const int par = k % 3;
-    if (tid < 32) {
-      int piv = lu_warp_pivot(col, s_perm, k, P);
-      if (tid == 0 && piv == P) flag_status(kStatusNonFinite);
-      if (piv == P) piv = k;
-      if (tid < kLuCtas) *cl.map_shared_rank(s_piv + par, tid) = piv;
-      if (tid == 0) {
-        s_piv[par] = piv;
-        s_rcp = 1.0 / col[s_perm[piv]];
-      }
-    }
-    __syncthreads();
-    const int piv = s_piv[par];
-    const double akk = col[s_perm[piv]];  // row k once swapped
-    const int i = k + 1 + tid;
+  // Pivot and multipliers of column k into every CTA; this thread holds v, the
+  // column's value in logical row i = k + tid, row r of A.  Each warp offers its
+  // largest with its reciprocal (worked out beside the comparisons).
+  auto prepare = [&](int k, int i, int r, double v) {
+    const int lane = tid & 31, warp = tid >> 5;
+    unsigned h = 0, w = 0;
     if (i < P) {
-      const int r = s_perm[i == piv ? k : i];
-      const double l = quotient(col[r], akk, s_rcp);
+      h = __double2hiint(v) & 0x7fffffff;
+      w = __double2loint(v);
+      if (h > 0x7ff00000u || (h == 0x7ff00000u && w != 0)) h = w = 0;
+    }
+    const double rcp = reciprocal(v);
+    const unsigned hm = __reduce_max_sync(0xffffffffu, h);
+    const unsigned wm = __reduce_max_sync(0xffffffffu, h == hm ? w : 0u);
+    const int first = __reduce_min_sync(0xffffffffu, i < P && h == hm && w == wm ? lane : 32);
+    if (first == 32 ? lane == 0 : lane == first)
+      s_cand[warp] = {h, w, first == 32 ? P : i, r, v, rcp};
+    __syncthreads();
+    LuCandidate best = s_cand[0];
+    const int nw = (P - k + 31) / 32;  // warps with rows
+    for (int c = 1; c < nw; ++c) {
+      const unsigned ch = s_cand[c].h, cw = s_cand[c].l;
+      if (ch > best.h || (ch == best.h && cw > best.l)) best = s_cand[c];
+    }
+    if (tid == 0 && (best.h | best.l) == 0) flag_status(kStatusNonFinite);
+    const int par = k % 3;
+    if (tid < kLuCtas) *cl.map_shared_rank(s_piv + par, tid) = best.row;
+    if (i < P && i != best.row) {
+      const double l = quotient(v, best.value, best.rcp);
 #pragma unroll
       for (int c = 0; c < kLuCtas; ++c) cl.map_shared_rank(s_l + par * P, c)[r] = l;
       if (FACTOR) wl[static_cast<int64_t>(k) * P + r] = l;
     }
   };
 
-  if (rank == 0) prepare(0);
+  if (rank == 0) prepare(0, tid, tid, tid < P ? panel[tid] : 0.0);
   auto token = cl.barrier_arrive();
   for (int k = 0; k < P; ++k) {
     cl.barrier_wait(std::move(token));
     const double* l = s_l + (k % 3) * P;
-    if (tid == 0) {
-      const int piv = s_piv[k % 3], t = s_perm[k];
-      s_perm[k] = s_perm[piv];
-      s_perm[piv] = t;
-    }
-    __syncthreads();  // the permutation, and the last step's updates
-    const int top = s_perm[k];
+    // rows k and piv change places: here for this step's reads, in s_perm once
+    // every thread has read (the next reads are past the next cluster barrier)
+    const int piv = s_piv[k % 3];
+    const int pk = s_perm[k], top = s_perm[piv];
     const int i = k + 1 + tid;
-    const int r = i < P ? s_perm[i] : 0;
+    const int r = i < P ? (i == piv ? pk : s_perm[i]) : 0;
+    __syncthreads();  // these reads, and the last step's updates
+    if (tid == 0) {
+      s_perm[k] = top;
+      s_perm[piv] = pk;
+    }
+    const double lr = i < P ? l[r] : 0.0;
     // the next column first, its pivot and multipliers
     const bool own = k + 1 < P && (k + 1) % kLuCtas == rank;
     if (own) {
       double* col = panel + ((k + 1) / kLuCtas) * P;
-      if (i < P) col[r] -= l[r] * col[top];
-      __syncthreads();
-      prepare(k + 1);
+      double v = 0.0;
+      if (i < P) {
+        v = col[r] - lr * col[top];
+        col[r] = v;
+      }
+      prepare(k + 1, i, r, v);
     }
     token = cl.barrier_arrive();
-    // then this CTA's other columns j > k + 1 (and the right-hand side)
+    // then this CTA's other columns j > k + 1 (and the right-hand side), loads
+    // of four columns at a time first
     const int first = k + 1 - rank + (own ? 1 : 0);  // least j - rank
     const int q0 = first > 0 ? (first + kLuCtas - 1) / kLuCtas : 0;
     if (i < P) {
-      const double lr = l[r];
       if (!FACTOR && rank == 0) s_x[r] -= lr * s_x[top];
-      for (int q = q0; q < ncol; ++q) {
-        double* col = panel + q * P;
-        col[r] -= lr * col[top];
+      for (int q = q0; q < ncol; q += 4) {
+        double a4[4], u4[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const double* col = panel + min(q + m, ncol - 1) * P;
+          a4[m] = col[r];
+          u4[m] = col[top];
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (q + m < ncol) panel[(q + m) * P + r] = a4[m] - lr * u4[m];
       }
     }
   }
