@@ -416,18 +416,16 @@ __global__ void __launch_bounds__(kLuThreads) lu_solve_kernel(int P, int T, doub
 // What a step costs is its chain -- pivot, reciprocal, multipliers, their way to
 // the other CTAs -- so that is all that stands between two steps: the owner of
 // column k + 1 brings that column up to date first, finds its pivot by integer
-// comparisons, forms the multipliers, writes them into every CTA's shared
-// memory and arrives at the cluster barrier; everybody's other columns
-// follow while the barrier fills.  Rows are permuted by index; every element sees
-// the operations of the single-CTA form in its order, so the factors and the
-// solution are the same.  The multipliers
-// go round three buffers: step k + 3's writer has passed barrier k + 2, at which
-// every thread arrived after its last use of step k's.
-// 120 unknowns: 168 us, 1.4 us a step (3.2 us while every step's pivot, swap,
-// division and the reading back of the multipliers stood in the chain; 1.7 us with
-// one warp's search and division after the column's update); what is left is
-// mostly the barrier and the stores to the other CTAs before it.  The replayed
-// solve takes 51 us (125 us with two barriers a column).
+// comparisons, forms the multipliers and sends them to every CTA, counted on an
+// mbarrier per step; everybody's other columns follow meanwhile.  Every step has
+// its own place for its multipliers, so nobody waits to write.  A thread holds a
+// row and knows where it stands: no rows move.  Every element sees the operations
+// of the single-CTA form in its order, so the factors and the solution are the
+// same.  120 unknowns: 128 us, 1.1 us a step (168 us with a cluster barrier per
+// step, which waits for the stores to the other CTAs; 390 us while every step's
+// pivot, swap, division and the reading back of the multipliers stood in the
+// chain); 192: 272 us (319 with barriers).  Four CTAs are slower (199 against 178 us
+// with barriers: their columns' updates).  The replayed solve takes 51 us (125 us with two barriers a column).
 namespace cg = cooperative_groups;
 constexpr int kLuCtas = 8;
 constexpr int kLuClusterThreads = 256;
@@ -511,8 +509,39 @@ struct LuCandidate {
   double value, rcp;
 };
 
-// Dynamic shared memory per CTA: panel[ceil(P/kLuCtas)][P] (column-major),
-// l[3][P], x[P], packed U[P (P + 1) / 2] (x and U used in CTA 0).
+// Doubles of dynamic shared memory per CTA: panel[ceil(P/kLuCtas)][P] (column-major),
+// the multipliers of all steps (step k's P - 1 - k in the rows' new order; CTA 0's
+// packed U takes their place), x[P], a word and an mbarrier per step.
+__host__ __device__ constexpr size_t lu_smem_doubles(int P) {
+  return static_cast<size_t>((P + kLuCtas - 1) / kLuCtas) * P + P * (P + 1) / 2 +
+         3 * static_cast<size_t>(P);
+}
+
+// 8 bytes into a CTA of the cluster, counted on its mbarrier (shared::cluster addresses)
+__device__ __forceinline__ void store_async(uint32_t addr, uint64_t v, uint32_t bar) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+      "l"(v), "r"(bar)
+      : "memory");
+}
+
+// Phase 0 of an mbarrier whose bytes come from the cluster; false after kWaitLimit polls.
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar) {
+  const uint32_t addr = smem_u32(bar);
+  for (uint32_t it = 0; it < kWaitLimit; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
 // FACTOR: the factorisation alone, no right-hand side: the multipliers, the
 // permutation and the packed upper triangle go to the workspace W
 // (lu_workspace_doubles), from which lu_solve_factored_kernel replays the same
@@ -520,7 +549,7 @@ struct LuCandidate {
 // solution bit for bit), so the factorisation can run while the right-hand
 // side is still being formed.
 template <bool FACTOR>
-__global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThreads)
+__global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThreads, 1)
     lu_cluster_kernel(int P, double* __restrict__ A, double* __restrict__ b,
                       double* __restrict__ W) {
   cg::cluster_group cl = cg::this_cluster();
@@ -536,29 +565,43 @@ __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThre
   const int ncol = rank < P ? (P - rank + kLuCtas - 1) / kLuCtas : 0;
   double* panel = lc_smem;
   double* s_l = panel + static_cast<size_t>(ncmax) * P;
-  double* s_x = s_l + 3 * P;
-  double* s_u = s_x + P;
+  double* s_x = s_l + P * (P + 1) / 2;
+  uint64_t* s_word = reinterpret_cast<uint64_t*>(s_x + P);  // pivot: new row | row of A << 32
+  uint64_t* s_bar = s_word + P;
   __shared__ int s_perm[kLuClusterMaxP];
-  __shared__ int s_piv[3];
   __shared__ LuCandidate s_cand[kLuClusterThreads / 32];
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NT = kLuClusterThreads;
   for (int e = tid; e < ncol * P; e += NT) {
     const int q = e / P, r = e - q * P;
     panel[q * P + r] = a[static_cast<int64_t>(r) * P + rank + kLuCtas * q];
   }
-  for (int r = tid; r < P; r += NT) s_perm[r] = r;
   if (!FACTOR && rank == 0)
     for (int r = tid; r < P; r += NT) s_x[r] = xg[r];
-  cl.sync();  // every CTA runs: its shared memory may be written
+  // step k brings P - 1 - k multipliers and the word
+  if (tid < P) mbar_init(s_bar + tid, 1);
+  fence_mbar_init();
+  if (tid < P) mbar_arrive_expect_tx(s_bar + tid, 8 * (P - tid));
+  uint32_t peer[kLuCtas];  // this CTA's shared memory as each CTA's
+#pragma unroll
+  for (int c = 0; c < kLuCtas; ++c)
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(peer[c])
+        : "r"(smem_u32(lc_smem)), "r"(c));
+  cl.sync();  // every CTA runs and counts its bytes: its shared memory may be written
 
-  // Pivot and multipliers of column k into every CTA; this thread holds v, the
-  // column's value in logical row i = k + tid, row r of A.  Each warp offers its
-  // largest with its reciprocal (worked out beside the comparisons).
-  auto prepare = [&](int k, int i, int r, double v) {
-    const int lane = tid & 31, warp = tid >> 5;
+  // thread r holds row r of A, which stands at row `at` of the elimination
+  const int r = tid;
+  int at = tid;
+  auto offset = [P](int k) { return k * (P - 1) - k * (k - 1) / 2; };
+
+  // Pivot and multipliers of column k into every CTA; v is the column's value in
+  // this thread's row.  Each warp offers its largest with its reciprocal (worked out
+  // beside the comparisons).
+  auto prepare = [&](int k, double v) {
+    const bool in = tid < P && at >= k;
     unsigned h = 0, w = 0;
-    if (i < P) {
+    if (in) {
       h = __double2hiint(v) & 0x7fffffff;
       w = __double2loint(v);
       if (h > 0x7ff00000u || (h == 0x7ff00000u && w != 0)) h = w = 0;
@@ -566,61 +609,72 @@ __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThre
     const double rcp = reciprocal(v);
     const unsigned hm = __reduce_max_sync(0xffffffffu, h);
     const unsigned wm = __reduce_max_sync(0xffffffffu, h == hm ? w : 0u);
-    const int first = __reduce_min_sync(0xffffffffu, i < P && h == hm && w == wm ? lane : 32);
-    if (first == 32 ? lane == 0 : lane == first)
-      s_cand[warp] = {h, w, first == 32 ? P : i, r, v, rcp};
+    const bool mine = in && h == hm && w == wm;
+    const int first = __reduce_min_sync(0xffffffffu, mine ? at : P);
+    if (first == P ? lane == 0 : mine && at == first) s_cand[warp] = {h, w, first, r, v, rcp};
     __syncthreads();
     LuCandidate best = s_cand[0];
-    const int nw = (P - k + 31) / 32;  // warps with rows
-    for (int c = 1; c < nw; ++c) {
-      const unsigned ch = s_cand[c].h, cw = s_cand[c].l;
-      if (ch > best.h || (ch == best.h && cw > best.l)) best = s_cand[c];
+    for (int c = 1; c < (P + 31) / 32; ++c) {
+      const LuCandidate& o = s_cand[c];
+      const bool more = o.h > best.h || (o.h == best.h && o.l > best.l);
+      if (more || (o.h == best.h && o.l == best.l && o.row < best.row)) best = o;
     }
     if (tid == 0 && (best.h | best.l) == 0) flag_status(kStatusNonFinite);
-    const int par = k % 3;
-    if (tid < kLuCtas) *cl.map_shared_rank(s_piv + par, tid) = best.row;
-    if (i < P && i != best.row) {
+    const uint32_t bar =
+        static_cast<uint32_t>(reinterpret_cast<char*>(s_bar + k) - reinterpret_cast<char*>(lc_smem));
+    if (tid < kLuCtas) {
+      const uint32_t to = static_cast<uint32_t>(reinterpret_cast<char*>(s_word + k) -
+                                                reinterpret_cast<char*>(lc_smem));
+      uint32_t p0;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p0) : "r"(smem_u32(lc_smem)), "r"(tid));
+      store_async(p0 + to, static_cast<uint32_t>(best.row) | static_cast<uint64_t>(best.place) << 32,
+                  p0 + bar);
+    }
+    if (in && r != best.place) {
       const double l = quotient(v, best.value, best.rcp);
+      const int i = at == k ? best.row : at;  // once rows k and the pivot's have changed places
+      const uint32_t to = static_cast<uint32_t>(
+          reinterpret_cast<char*>(s_l + offset(k) + i - k - 1) - reinterpret_cast<char*>(lc_smem));
 #pragma unroll
-      for (int c = 0; c < kLuCtas; ++c) cl.map_shared_rank(s_l + par * P, c)[r] = l;
+      for (int c = 0; c < kLuCtas; ++c)
+        store_async(peer[c] + to, __double_as_longlong(l), peer[c] + bar);
       if (FACTOR) wl[static_cast<int64_t>(k) * P + r] = l;
     }
   };
 
-  if (rank == 0) prepare(0, tid, tid, tid < P ? panel[tid] : 0.0);
-  auto token = cl.barrier_arrive();
+  if (rank == 0) prepare(0, tid < P ? panel[tid] : 0.0);
+  bool ok = true;
   for (int k = 0; k < P; ++k) {
-    cl.barrier_wait(std::move(token));
-    const double* l = s_l + (k % 3) * P;
-    // rows k and piv change places: here for this step's reads, in s_perm once
-    // every thread has read (the next reads are past the next cluster barrier)
-    const int piv = s_piv[k % 3];
-    const int pk = s_perm[k], top = s_perm[piv];
-    const int i = k + 1 + tid;
-    const int r = i < P ? (i == piv ? pk : s_perm[i]) : 0;
-    __syncthreads();  // these reads, and the last step's updates
-    if (tid == 0) {
-      s_perm[k] = top;
-      s_perm[piv] = pk;
+    ok = wait_cluster(s_bar + k);
+    // (and the last step's updates)
+    if (!__syncthreads_and(ok)) {
+      ok = false;
+      break;
     }
-    const double lr = i < P ? l[r] : 0.0;
+    const uint64_t word = s_word[k];
+    const int piv = static_cast<int>(word & 0xffffffffu), top = static_cast<int>(word >> 32);
+    if (r == top)
+      at = k;
+    else if (at == k)
+      at = piv;
+    const bool in = tid < P && at > k;
+    const double lr = in ? s_l[offset(k) + at - k - 1] : 0.0;
     // the next column first, its pivot and multipliers
     const bool own = k + 1 < P && (k + 1) % kLuCtas == rank;
     if (own) {
       double* col = panel + ((k + 1) / kLuCtas) * P;
       double v = 0.0;
-      if (i < P) {
+      if (in) {
         v = col[r] - lr * col[top];
         col[r] = v;
       }
-      prepare(k + 1, i, r, v);
+      prepare(k + 1, v);
     }
-    token = cl.barrier_arrive();
     // then this CTA's other columns j > k + 1 (and the right-hand side), loads
     // of four columns at a time first
     const int first = k + 1 - rank + (own ? 1 : 0);  // least j - rank
     const int q0 = first > 0 ? (first + kLuCtas - 1) / kLuCtas : 0;
-    if (i < P) {
+    if (in) {
       if (!FACTOR && rank == 0) s_x[r] -= lr * s_x[top];
       for (int q = q0; q < ncol; q += 4) {
         double a4[4], u4[4];
@@ -636,10 +690,11 @@ __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThre
       }
     }
   }
-  cl.barrier_wait(std::move(token));
-  __syncthreads();
+  if (!ok) flag_status(kStatusTimeout);
+  if (tid < P) s_perm[at] = r;
+  cl.sync();  // every CTA's multipliers are used: packed U may take their place in CTA 0
   // the upper triangle, packed by columns, into the workspace or CTA 0
-  double* u0 = FACTOR ? wu : cl.map_shared_rank(s_u, 0);
+  double* u0 = FACTOR ? wu : cl.map_shared_rank(s_l, 0);
   for (int q = 0; q < ncol; ++q) {
     const int j = rank + kLuCtas * q;
     for (int i = tid; i <= j; i += NT) u0[packed_u(j) + i] = panel[q * P + s_perm[i]];
@@ -657,7 +712,7 @@ __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThre
   __syncthreads();
   if (tid < P) s_x[tid] = x;
   __syncthreads();
-  back_substitute(P, s_u, s_x, tid);
+  back_substitute(P, s_l, s_x, tid);
   for (int i = tid; i < P; i += NT) xg[i] = s_x[i];
 }
 
@@ -1108,9 +1163,7 @@ int fvx_lu_solve_batched(int n_systems, int P, double* A, double* b, void* strea
   FVX_ARG_CHECK(n_systems >= 1 && P >= 1 && P <= fvx::kLuMaxP && A && b,
                 "bad solve arguments (P must be 1..%d)", fvx::kLuMaxP);
   if (P <= fvx::kLuClusterMaxP) {
-    const int ncmax = (P + fvx::kLuCtas - 1) / fvx::kLuCtas;
-    const size_t smem =
-        8 * (static_cast<size_t>(ncmax) * P + 4 * static_cast<size_t>(P) + P * (P + 1) / 2);
+    const size_t smem = 8 * fvx::lu_smem_doubles(P);
     FVX_CUDA_TRY(cudaFuncSetAttribute(fvx::lu_cluster_kernel<false>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(smem)));
@@ -1141,9 +1194,7 @@ int64_t fvx_lu_workspace_bytes(int P) {
 int fvx_lu_factor_batched(int n_systems, int P, double* A, double* work, void* stream) {
   FVX_ARG_CHECK(n_systems >= 1 && P >= 1 && P <= fvx::kLuClusterMaxP && A && work,
                 "bad factor arguments (P must be 1..%d)", fvx::kLuClusterMaxP);
-  const int ncmax = (P + fvx::kLuCtas - 1) / fvx::kLuCtas;
-  const size_t smem =
-      8 * (static_cast<size_t>(ncmax) * P + 4 * static_cast<size_t>(P));
+  const size_t smem = 8 * fvx::lu_smem_doubles(P);
   FVX_CUDA_TRY(cudaFuncSetAttribute(fvx::lu_cluster_kernel<true>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(smem)));
