@@ -8,9 +8,11 @@ Drop-in replacements for the five functions that
 (``warp_kernels.py:193-194, 224-225``).
 
 Two call forms:
-  * NumPy arrays (what PteraSoftware passes): one host-to-device transfer of
-    all inputs, one fused launch, one device-to-host transfer, synchronous; a
-    new NumPy array is returned.
+  * NumPy arrays (what PteraSoftware passes): synchronous, a new NumPy array is
+    returned.  Small collapsed calls are one launch that reads the inputs from
+    and writes the result to pinned host memory; the others make one
+    host-to-device transfer of all inputs, one fused launch and one
+    device-to-host transfer.
   * torch CUDA tensors: zero-copy, stream-ordered on torch's current stream;
     a new CUDA tensor is returned.
 

@@ -17,9 +17,9 @@ Everything runs on the tensor cores through the C ABI:
     kernel computes the features from the pair list, the analytic translation
     on the CUDA cores and the residual on the tensor cores, and accumulates the
     expansions per leaf);
-  * training (``FarFieldMLP.fit``): forward with stored activations, then per
-    layer the weight gradient dW = dZ^T H and the input gradient dH = dZ W as
-    BF16 tcgen05 GEMMs with FP32 accumulation, SiLU backward, Adam on FP32
+  * training (``FarFieldMLP.fit``): forward, then per layer the weight gradient
+    dW = dZ^T H and the input gradient dH = dZ W as BF16 tcgen05 products with
+    FP32 accumulation and SiLU backward, a batch in one kernel; Adam on FP32
     master weights with a BF16 copy for the kernels;
   * training data (``harvest``): pairs sampled from the local-expansion lists
     of the solver's own particle fields, with targets summed directly in FP64
