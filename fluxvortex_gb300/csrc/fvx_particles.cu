@@ -392,16 +392,6 @@ __device__ const __align__(16) float g_core_table[] = {FVX_CORE_TABLE};
 constexpr int kTableRows = x3::kCoreRows + x3::kFarRows;
 constexpr int kTableFloats = kTableRows * x3::kRowFloats;  // of F, and of G
 
-// coordinates up to 2^13, cores of 2^-22 .. 2^13 (high words; NaN and infinity
-// are beyond): the three-float arithmetic's range
-__device__ __forceinline__ bool x3_coord(double x) {
-  return (__double2hiint(x) & 0x7fffffff) < ((1023 + 13) << 20);
-}
-__device__ __forceinline__ bool x3_core(double s) {
-  const int h = __double2hiint(s);
-  return h >= ((1023 - 22) << 20) && h < ((1023 + 13) << 20);
-}
-
 // Sums of one pair in FP64 given f and f'/r (and, for the vorticity, iso = f'/r
 // r^2 + 2 f): accumulate() with every product fused into its sum.  The
 // Jacobian's antisymmetric part goes to acc[9..11] = sum of f a and is put in
@@ -517,7 +507,7 @@ __global__ void __launch_bounds__(kSlices* kThreads) pairs_f64_kernel(PairArgs A
       gz = A.tgt_gamma[3 * i + 2];
     }
   }
-  const bool tgt_ok = x3_coord(tx) && x3_coord(ty) && x3_coord(tz);
+  const bool tgt_ok = x3::coord_in_range(tx) && x3::coord_in_range(ty) && x3::coord_in_range(tz);
   const x3::F3 px = x3::split_fast(tx), py = x3::split_fast(ty), pz = x3::split_fast(tz);
 
   const int64_t jb = static_cast<int64_t>(blockIdx.y) * A.chunk;
@@ -569,13 +559,13 @@ __global__ void __launch_bounds__(kSlices* kThreads) pairs_f64_kernel(PairArgs A
     for (int k = threadIdx.x; k < n; k += kAll) {
       const double sg = raw.sigma[k];
       SrcX3 v = {};
-      in_range = in_range && x3_core(sg);
+      in_range = in_range && x3::core_in_range(sg);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const double p = raw.pos[3 * k + c];
         v.a[c] = kC * raw.alpha[3 * k + c];
         v.x[c] = x3::split_fast(p);
-        in_range = in_range && x3_coord(p);
+        in_range = in_range && x3::coord_in_range(p);
       }
       const x3::Core core = GAUSS ? x3::gaussian_core(sg) : x3::winckelmans_core(sg);
       v.s2 = core.s2;

@@ -31,6 +31,7 @@
 #include "fvx_common.cuh"
 #include "fvx_pair_math.cuh"
 #include "fvx_x2.cuh"
+#include "fvx_x3.cuh"
 
 namespace fvx {
 namespace tree {
@@ -2366,6 +2367,10 @@ __global__ void judge_repair_kernel(JudgeSampleBufs B, const float* __restrict__
 // classes) takes S = 8 slices of at least 128 and one phase.  Each warp takes
 // whole targets: its lanes stride over the slice, reduce by shuffles and add
 // one atomic per output component, with no block-wide barrier per target.
+// The FP64 pipe bounds it: a Winckelmans pair's scalar core (20 of its 38 FP64
+// operations) is formed in three-float arithmetic (fvx_x3.cuh) from the FP64 offset,
+// where that arithmetic's range holds.  A class of 100,000 particles' field 411 ->
+// 229 ms, of 120,000 656 -> 356 ms.
 constexpr int kFallbackThreads = 256;
 constexpr int kFallbackShortQueue = 2048;
 struct FallbackTargets {
@@ -2386,6 +2391,8 @@ __global__ void __launch_bounds__(kFallbackThreads) fallback_kernel(
   constexpr bool NEED_FPR = ModeInfo<MODE>::need_fpr;
   constexpr bool NEED_TG = ModeInfo<MODE>::need_tg;
   constexpr double kC = -0.07957747154594767;
+  // (the vorticity needs r^2 beside the core)
+  constexpr bool X3 = KERNEL == FVX_KERNEL_WINCKELMANS && MODE != FVX_PAIR_VORTICITY;
   const int nq = min(*n_fallback, fb_cap);
   const bool short_q = nq < kFallbackShortQueue;
   const int S = short_q ? 64 : 8, TP = short_q ? 8 : 1, min_slice = short_q ? 32 : 128;
@@ -2420,18 +2427,30 @@ __global__ void __launch_bounds__(kFallbackThreads) fallback_kernel(
       for (int q = lane; q < ns; q += 32) {
         const int j = perm[s0 + q];
         const double dx = x - pos[3 * j], dy = y - pos[3 * j + 1], dz = z - pos[3 * j + 2];
-        const double r2 = dx * dx + dy * dy + dz * dz;
         const double sg = sigma[j];
-        const double s2 = sg * sg;
-        const double k2 = KERNEL == FVX_KERNEL_WINCKELMANS ? 2.5 * s2 : 1.0 / sg;
-        double f, fpr = 0.0;
-        core_f64<KERNEL, NEED_FPR>(r2, s2, k2, f, fpr);
-        accumulate<MODE, double>(acc, dx, dy, dz, r2, kC * alpha[3 * j], kC * alpha[3 * j + 1],
-                                 kC * alpha[3 * j + 2], f, fpr, gx, gy, gz);
+        double f, fpr = 0.0, r2 = 0.0;
+        if (X3 && x3::core_in_range(sg) && x3::coord_in_range(dx) && x3::coord_in_range(dy) &&
+            x3::coord_in_range(dz)) {
+          x3::F3 f3, fpr3 = {}, none = {};
+          x3::winckelmans<NEED_FPR, false>(x3::split_fast(dx), x3::split_fast(dy),
+                                           x3::split_fast(dz),
+                                           x3::winckelmans_core(x3::split_fast(sg)), f3, fpr3, none);
+          f = x3::to_double(f3);
+          if (NEED_FPR) fpr = x3::to_double(fpr3);
+        } else {
+          r2 = dx * dx + dy * dy + dz * dz;
+          const double s2 = sg * sg;
+          const double k2 = KERNEL == FVX_KERNEL_WINCKELMANS ? 2.5 * s2 : 1.0 / sg;
+          core_f64<KERNEL, NEED_FPR>(r2, s2, k2, f, fpr);
+        }
+        accumulate<MODE, double>(acc, dx, dy, dz, r2, alpha[3 * j], alpha[3 * j + 1],
+                                 alpha[3 * j + 2], f, fpr, gx, gy, gz);
       }
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
+      for (int c = 0; c < NC; ++c) {
         for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        acc[c] *= kC;
+      }
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         if (lane != c) continue;

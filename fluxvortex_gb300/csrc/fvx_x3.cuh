@@ -70,6 +70,16 @@ FVX_X3 int to_int_down(float x) { return (int)floorf(x); }
 FVX_X3 float round_int(float x) { return rintf(x); }
 #endif
 
+// The ranges of coordinates (or offsets) and cores: magnitudes below 2^13, cores of
+// 2^-22 .. 2^13; not NaN.
+FVX_X3 bool coord_in_range(double x) {
+  return ((uint32_t)(words(x) >> 32) & 0x7fffffffu) < (uint32_t)((1023 + 13) << 20);
+}
+FVX_X3 bool core_in_range(double s) {
+  const uint32_t h = (uint32_t)(words(s) >> 32);
+  return h >= (uint32_t)((1023 - 22) << 20) && h < (uint32_t)((1023 + 13) << 20);
+}
+
 // s + e = a + b exactly
 FVX_X3 float two_sum(float a, float b, float& e) {
   const float s = add(a, b);
@@ -315,13 +325,14 @@ FVX_X3 F3 twice_f_plus(const F3& f, const F3& fpr, const F3& r2) {
   return diff(F3{add(f.h, f.h), add(f.m, f.m), add(f.l, f.l)}, F3{-p.h, -p.m, -p.l});
 }
 
-FVX_X3 Core winckelmans_core(double sigma) {
-  const F3 s = split(sigma), p = prod(s, s);
+FVX_X3 Core winckelmans_core(const F3& s) {
+  const F3 p = prod(s, s);
   Core c = {};
   c.s2 = renorm(p.h, p.m, p.l);
   c.k = scale_float(c.s2, 1.5f);
   return c;
 }
+FVX_X3 Core winckelmans_core(double sigma) { return winckelmans_core(split(sigma)); }
 // (to three floats, so that sigma cancels where the core is the singular one)
 FVX_X3 Core gaussian_core(double sigma) {
   const double r = 1.0 / sigma;
