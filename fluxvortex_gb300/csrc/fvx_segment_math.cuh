@@ -273,7 +273,8 @@ __device__ __forceinline__ void vortex_velocity(const VortexRec& R, double px, d
     dy[c] = R.c[c][1] - py;
     dz[c] = R.c[c][2] - pz;
     sq[c] = dx[c] * dx[c] + dy[c] * dy[c] + dz[c] * dz[c];
-    const int h = __double2hiint(sq[c]);   // squares: no sign bit (but a NaN's)
+    // (a NaN may carry a sign, inf - inf on x86 does: it is above kHiMax either way)
+    const int h = __double2hiint(sq[c]) & 0x7fffffff;
     lo = min(lo, h);
     hi = max(hi, h);
   }
