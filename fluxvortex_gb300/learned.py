@@ -82,6 +82,7 @@ class FarFieldMLP:
         # gradients and loss side by side: one fill clears them
         self._grads = torch.zeros(NW + NB + 1, dtype=torch.float32, device=self.device)
         self.gw, self.gb, self.loss = self._grads.split([NW, NB, 1])
+        self._clear, self._loss_rows = [self._grads], None
         self.step_count = 0
         self.lib = _capi.load()
         self.meta = {}
@@ -126,12 +127,17 @@ class FarFieldMLP:
     # ---- training ----------------------------------------------------------------
     def gradients(self, X, T, weights=None):
         """Loss sum(w_r (Y - T)^2) over the 30 used outputs (device scalar; w_r = 1
-        without row weights) and the gradients of the mean loss into self.gw /
-        self.gb."""
+        without row weights; the next batch of as many rows overwrites it) and the
+        gradients of the mean loss into self.gw / self.gb."""
         rows = X.shape[0]
         assert X.dtype == torch.bfloat16 and X.shape[1] == IN and X.is_contiguous()
         Y = torch.empty((rows, OUT), dtype=torch.float32, device=self.device)
-        self._grads.zero_()
+        if self._loss_rows not in (None, rows):      # the last loss stays its caller's
+            self.loss = torch.zeros(1, dtype=torch.float32, device=self.device)
+            self._clear = [self._grads[:NW + NB], self.loss]
+        self._loss_rows = rows
+        for t in self._clear:
+            t.zero_()
         _capi.check(self.lib.fvx_mlp_gradients(
             X.data_ptr(), T.data_ptr(), None if weights is None else weights.data_ptr(), rows,
             self.wb.data_ptr(), self.b.data_ptr(), Y.data_ptr(), self.gw.data_ptr(),
