@@ -70,15 +70,34 @@ __device__ __forceinline__ int block_inclusive(int v, int* s_warp, int& total) {
   return warp ? v + before : v;
 }
 
-// One CTA's scan of kScanBlock elements from base, `run` before them; returns their sum.
+// Sum over the CTA in 64 bits, in thread 0.
+__device__ __forceinline__ int64_t block_sum64(int64_t v) {
+  __shared__ int64_t s[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = threadIdx.x < blockDim.x >> 5 ? s[threadIdx.x] : 0;
+  if (threadIdx.x < 32)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// One CTA's scan of kScanBlock elements from base, `run` before them; returns their
+// sum modulo 2^32 and adds this thread's elements to `own_sum`.
 // Each warp takes kScanItems runs of 32 (coalesced).
 __device__ __forceinline__ int scan_tile(const int* __restrict__ in, int n, int* __restrict__ out,
-                                         int base, int run, int inclusive, int* s_warp) {
+                                         int base, int run, int inclusive, int* s_warp,
+                                         int64_t& own_sum) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i0 = base + warp * 32 * kScanItems + lane;
   int own[kScanItems], v[kScanItems];
 #pragma unroll
-  for (int e = 0; e < kScanItems; ++e) v[e] = own[e] = i0 + 32 * e < n ? in[i0 + 32 * e] : 0;
+  for (int e = 0; e < kScanItems; ++e) {
+    v[e] = own[e] = i0 + 32 * e < n ? in[i0 + 32 * e] : 0;
+    own_sum += own[e];
+  }
   int sum = 0;  // of the warp's runs
 #pragma unroll
   for (int e = 0; e < kScanItems; ++e) {
@@ -100,48 +119,56 @@ __device__ __forceinline__ int scan_tile(const int* __restrict__ in, int n, int*
   return total;
 }
 
-// Up to four arrays of at most kScanOneCta elements, a CTA each, and their sums.
+// Up to four arrays of at most kScanOneCta elements, a CTA each, and their sums.  The
+// prefix sums are modulo 2^32; the total is not, so that a list longer than
+// its 32-bit offsets is seen.
 struct ScanJobs {
   const int* in[4];
   int* out[4];
   int n[4];
-  int* total;  // null, or one per job
+  int64_t* total;  // null, or one per job
 };
 __global__ void __launch_bounds__(kScanThreads) scan_jobs_kernel(ScanJobs J, int inclusive) {
   __shared__ int s_warp[32];
   const int j = blockIdx.x;
   int run = 0;
+  int64_t own = 0;
   for (int base = 0; base < J.n[j]; base += kScanBlock)
-    run += scan_tile(J.in[j], J.n[j], J.out[j], base, run, inclusive, s_warp);
-  if (J.total && threadIdx.x == 0) J.total[j] = run;
+    run += scan_tile(J.in[j], J.n[j], J.out[j], base, run, inclusive, s_warp, own);
+  if (!J.total) return;
+  const int64_t total = block_sum64(own);
+  if (threadIdx.x == 0) J.total[j] = total;
 }
 
 __global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(const int* __restrict__ in, int n,
-                                                                 int* __restrict__ sums) {
-  __shared__ int s_warp[32];
+                                                                 int64_t* __restrict__ sums) {
   const int i0 = blockIdx.x * kScanBlock + threadIdx.x;
-  int v = 0, total;
+  int64_t v = 0;
 #pragma unroll
   for (int e = 0; e < kScanItems; ++e)
     if (i0 + e * kScanThreads < n) v += in[i0 + e * kScanThreads];
-  block_inclusive(v, s_warp, total);
-  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+  v = block_sum64(v);
+  if (threadIdx.x == 0) sums[blockIdx.x] = v;
 }
 
 // (every block adds up the sums of the blocks before it: at most 512)
 __global__ void __launch_bounds__(kScanThreads)
     scan_blocks_kernel(const int* __restrict__ in, int n, int* __restrict__ out,
-                       const int* __restrict__ sums, int inclusive, int* __restrict__ total) {
+                       const int64_t* __restrict__ sums, int inclusive,
+                       int64_t* __restrict__ total) {
   __shared__ int s_warp[32];
   int before;
-  block_inclusive(threadIdx.x < blockIdx.x ? sums[threadIdx.x] : 0, s_warp, before);
-  const int sum = scan_tile(in, n, out, blockIdx.x * kScanBlock, before, inclusive, s_warp);
-  if (total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = before + sum;
+  int64_t own = threadIdx.x < blockIdx.x ? sums[threadIdx.x] : 0;
+  block_inclusive(static_cast<int>(own), s_warp, before);
+  scan_tile(in, n, out, blockIdx.x * kScanBlock, before, inclusive, s_warp, own);
+  if (!total || blockIdx.x != gridDim.x - 1) return;
+  own = block_sum64(own);  // the blocks before and this one
+  if (threadIdx.x == 0) *total = own;
 }
 
 }  // namespace tree
 
-// Device-wide scans of n <= 2^22 ints each (in -> out); tmp holds >= 512 ints;
+// Device-wide scans of n <= 2^22 ints each (in -> out); tmp holds 512 x 8 bytes;
 // total: null, or where the arrays' sums go.  Arrays of at most kScanOneCta
 // elements share one launch, a CTA each: 32,768 elements take 10 us (12 in the
 // three launches of a scan by blocks, a scan of their sums and an addition, the
@@ -158,14 +185,15 @@ int scan_many(const tree::ScanJobs& J, int jobs, int inclusive, int* tmp, cudaSt
   for (int j = 0; j < jobs; ++j) {
     const int nb = (J.n[j] + kScanBlock - 1) / kScanBlock;
     FVX_ARG_CHECK(J.n[j] <= (1 << 22), "scan of %d elements exceeds 2^22", J.n[j]);
-    int* total = J.total ? J.total + j : nullptr;
+    int64_t* total = J.total ? J.total + j : nullptr;
     if (nb == 0) {
-      if (total) FVX_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(int), s));
+      if (total) FVX_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(int64_t), s));
       continue;
     }
-    scan_sums_kernel<<<nb, kScanThreads, 0, s>>>(J.in[j], J.n[j], tmp);
+    int64_t* sums = reinterpret_cast<int64_t*>(tmp);
+    scan_sums_kernel<<<nb, kScanThreads, 0, s>>>(J.in[j], J.n[j], sums);
     FVX_LAUNCH_CHECK();
-    scan_blocks_kernel<<<nb, kScanThreads, 0, s>>>(J.in[j], J.n[j], J.out[j], tmp, inclusive,
+    scan_blocks_kernel<<<nb, kScanThreads, 0, s>>>(J.in[j], J.n[j], J.out[j], sums, inclusive,
                                                    total);
     FVX_LAUNCH_CHECK();
   }
@@ -353,7 +381,7 @@ __global__ void __launch_bounds__(256) radix_scatter_kernel(
 
 // Stable LSD radix sort of (key, index) pairs by 32-bit keys, four 8-bit
 // passes: the pairs are read from (keys, idx) and returned there, (keys_tmp,
-// idx_tmp) hold n each, table sort_table_ints(n) ints, scan_tmp 512 ints.
+// idx_tmp) hold n each, table sort_table_ints(n) ints, scan_tmp 512 x 8 bytes.
 int sort_table_ints(int n) { return 256 * ((n + tree::kSortItems - 1) / tree::kSortItems) * 2; }
 
 int sort_pairs_u32(uint32_t* keys, int* idx, uint32_t* keys_tmp, int* idx_tmp, int n, int* table,
@@ -387,6 +415,7 @@ namespace tree {
 
 // ---- cells ----------------------------------------------------------------------
 constexpr int kMaxLevels = 11;
+constexpr int64_t kMaxList = 0x7fffffff;  // entries of an interaction list (32-bit offsets)
 
 struct Level {
   int* start;     // first sorted particle of each cell
@@ -2833,9 +2862,9 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   if ((rc = grow(T->keys0, 4 * size_t(n))) || (rc = grow(T->keys1, 4 * size_t(n))) ||
       (rc = grow(T->idx0, 4 * size_t(n))) || (rc = grow(T->idx1, 4 * size_t(n))) ||
       (rc = grow(T->table, 4 * size_t(256) * nblk * 2)) ||
-      (rc = grow(T->scan_tmp, 4 * 512)) ||
+      (rc = grow(T->scan_tmp, 8 * 512)) ||
       (rc = grow(T->cid, 4 * size_t(n))) || (rc = grow(T->levels, 4 * size_t(total_cells) * 7)) ||
-      (rc = grow(T->counts, 4 * (kMaxLevels + 4))) ||
+      (rc = grow(T->counts, 4 * (kMaxLevels + 1) + 8 * 4)) ||
       (rc = grow(T->rec, 4 * size_t(total_cells) * kRecFloats)) ||
       (rc = grow(T->sp, 16 * size_t(n))) || (rc = grow(T->sa, 16 * size_t(n))) ||
       (rc = grow(T->sg, 16 * size_t(n))))
@@ -2955,6 +2984,8 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
   int* par_off = dual ? par_cnt + npar : nullptr;
   const int* leaf_parent = dual ? cells().parent + base[L] : nullptr;
   int64_t near_total = 0, far_total = 0, lrn_total = 0, par_total = 0;
+  int64_t* list_totals = reinterpret_cast<int64_t*>(P<int>(T->counts) + kMaxLevels + 1);
+  static_assert((kMaxLevels + 1) % 2 == 0, "the totals are 8-byte aligned");
   if (reuse) {
     near_total = ST.near_total;
     far_total = ST.far_total;
@@ -3010,18 +3041,21 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
     const ScanJobs J{{LL.cnt, par_cnt, near_cnt, nullptr},
                      {P<int>(T->lrn_meta) + nleaf, par_off, far_off, nullptr},
                      {nleaf, npar, nleaf, 0},
-                     P<int>(T->counts) + kMaxLevels};
+                     list_totals};
     if ((rc = scan_many(J, 3, 0, P<int>(T->scan_tmp), s))) return rc;
-    FVX_CUDA_TRY(cudaMemcpyAsync(T->host, J.total, 12, cudaMemcpyDeviceToHost, s));
-    FVX_CUDA_TRY(cudaMemcpyAsync(T->host + 4, ovf, 4, cudaMemcpyDeviceToHost, s));
+    FVX_CUDA_TRY(cudaMemcpyAsync(T->host, J.total, 24, cudaMemcpyDeviceToHost, s));
+    FVX_CUDA_TRY(cudaMemcpyAsync(T->host + 6, ovf, 4, cudaMemcpyDeviceToHost, s));
     FVX_CUDA_TRY(cudaStreamSynchronize(s));
-    const int* tl = T->host;
-    const unsigned flags = static_cast<unsigned>(T->host[4]);
+    int64_t tl[3];
+    memcpy(tl, T->host, sizeof(tl));
+    const unsigned flags = static_cast<unsigned>(T->host[6]);
     if (!(flags & 4u)) {
       lrn_total = tl[0];
       par_total = tl[1];
       near_total = tl[2];
       far_total = 0;
+      FVX_ARG_CHECK(lrn_total <= kMaxList && par_total <= kMaxList,
+                    "local-expansion pair list too long");
       if ((rc = grow(T->lrn_leaf, 4 * size_t(lrn_total + 1))) ||
           (rc = grow(T->lrn_cell, 4 * size_t(lrn_total + 1))) ||
           (rc = grow(T->par_par, 4 * size_t(par_total + 1))) ||
@@ -3059,24 +3093,25 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
         V, nullptr, nullptr, near_cnt, far_cnt, nullptr, nullptr, 0, 0, ovf, LL);
   }
   FVX_LAUNCH_CHECK();
-  const int* lt = T->host;
   const ScanJobs J{{near_cnt, far_cnt, LL.cnt, par_cnt},
                    {near_off, far_off, learned ? P<int>(T->lrn_meta) + nleaf : nullptr, par_off},
                    {nleaf, nleaf, learned ? nleaf : 0, npar},
-                   P<int>(T->counts) + kMaxLevels};
+                   list_totals};
   if ((rc = scan_many(J, 4, 0, P<int>(T->scan_tmp), s))) return rc;
-  FVX_CUDA_TRY(cudaMemcpyAsync(T->host, J.total, 16, cudaMemcpyDeviceToHost, s));
+  FVX_CUDA_TRY(cudaMemcpyAsync(T->host, J.total, 32, cudaMemcpyDeviceToHost, s));
   FVX_CUDA_TRY(cudaStreamSynchronize(s));
+  int64_t lt[4];
+  memcpy(lt, T->host, sizeof(lt));
   near_total = lt[0];
   far_total = lt[1];
-  // (a sum past 2^31 shows as a negative one)
-  FVX_ARG_CHECK(near_total >= 0 && far_total >= 0, "interaction lists too long");
+  FVX_ARG_CHECK(near_total <= kMaxList && far_total <= kMaxList, "interaction lists too long");
   if ((rc = grow(T->near_list, 4 * size_t(near_total + 1))) ||
       (rc = grow(T->far_list, 4 * size_t(far_total + 1))))
     return rc;
   lrn_total = lt[2];
   par_total = lt[3];
-  FVX_ARG_CHECK(lrn_total >= 0 && par_total >= 0, "local-expansion pair list too long");
+  FVX_ARG_CHECK(lrn_total <= kMaxList && par_total <= kMaxList,
+                "local-expansion pair list too long");
   if (learned) {
     if ((rc = grow(T->lrn_leaf, 4 * size_t(lrn_total + 1))) ||
         (rc = grow(T->lrn_cell, 4 * size_t(lrn_total + 1))))
@@ -3556,6 +3591,18 @@ int fvx_tree_sample_pairs(fvx_tree* T, int list, int max_pairs, void* X, float* 
   if (rc) return rc;
   *n_out = np;
   return FVX_OK;
+}
+
+int fvx_probe_scan(const int* in, int n, int inclusive, int* out, int64_t* total, void* tmp,
+                   void* stream) {
+  FVX_ARG_CHECK(in && out && total && tmp && n >= 0, "bad scan arguments");
+  fvx::tree::ScanJobs J{};
+  J.in[0] = in;
+  J.out[0] = out;
+  J.n[0] = n;
+  J.total = total;
+  return fvx::scan_many(J, 1, inclusive, static_cast<int*>(tmp),
+                        static_cast<cudaStream_t>(stream));
 }
 
 int fvx_tree_last_eval_ms(fvx_tree* T, float* ms) {

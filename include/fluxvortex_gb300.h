@@ -537,6 +537,10 @@ int fvx_tc_gemm_probe(const void* A, const void* B, int N, int K, float* C, int 
  * measured FP32 CUDA-core peak used as the particle sweeps' roofline.  No
  * reference counterpart (measurement only). */
 int fvx_probe_fp32_fma(int blocks_per_sm, int iters, float* sink, void* stream);
+/* The prefix sums that size the tree's lists, on one array of n <= 2^22 counts
+ * (device pointers; tmp: 4,096 bytes): out modulo 2^32, *total in 64 bits. */
+int fvx_probe_scan(const int* in, int n, int inclusive, int* out, int64_t* total, void* tmp,
+                   void* stream);
 
 #ifdef __cplusplus
 }
