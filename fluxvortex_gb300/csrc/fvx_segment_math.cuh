@@ -184,14 +184,19 @@ __device__ __forceinline__ void vortex_legs(const VortexRec& R, double px, doubl
       skip(l, 0);
       continue;
     }
-    const double tol = TOL ? R.tol[l] : sqrt(R.r0sq[l]) * kTol;
-    if (in_range ? __double_as_longlong(len[a]) < __double_as_longlong(tol) : len[a] < tol) {
-      skip(l, 1);
-      continue;
-    }
-    if (in_range ? __double_as_longlong(len[b]) < __double_as_longlong(tol) : len[b] < tol) {
-      skip(l, 2);
-      continue;
+    // without a kept tolerance its root is taken only where a corner may be
+    // within it
+    const int near = __double2hiint(R.r0sq[l]) - kHiNear;
+    if (TOL || !in_range || min(__double2hiint(sq[a]), __double2hiint(sq[b])) <= near) {
+      const double tol = TOL ? R.tol[l] : sqrt(R.r0sq[l]) * kTol;
+      if (in_range ? __double_as_longlong(len[a]) < __double_as_longlong(tol) : len[a] < tol) {
+        skip(l, 1);
+        continue;
+      }
+      if (in_range ? __double_as_longlong(len[b]) < __double_as_longlong(tol) : len[b] < tol) {
+        skip(l, 2);
+        continue;
+      }
     }
     double r3x = dy[a] * dz[b] - dz[a] * dy[b];
     double r3y = dz[a] * dx[b] - dx[a] * dz[b];

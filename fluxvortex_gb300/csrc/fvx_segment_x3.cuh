@@ -22,7 +22,7 @@ struct RingX3 {
   x3::F3 r0sq[4];   // |end - start|^2 per leg
   double c2[4];     // |end - start|^2 r_c^2 per leg
   double half_c1;   // Gamma / (8 pi)
-  float near;       // |d|^2 below this at a corner: general path, unless zero
+  float near;       // |d|^2 below this at a corner: general path, unless zero (all: > kNoX3)
   int pad;
 };
 
@@ -32,6 +32,8 @@ struct RingX3 {
 // (1e-10 of 2^-20).
 constexpr int kX3LegMin = (1023 - 40) << 20, kX3LegMax = (1023 + 30) << 20;
 constexpr int kX3CoreMax = (1023 + 50) << 20;
+
+constexpr float kNoX3 = 1e30f;
 
 __device__ __forceinline__ bool x3_range(double x) {
   return (__double2hiint(x) & 0x7fffffff) < ((1023 + 13) << 20);
@@ -100,7 +102,7 @@ __device__ __forceinline__ CornerX3 see_corner(const View& V, int c, const x3::F
   C.sq = q.h;
   C.on = !(q.h > V.near());
   if (C.on) {
-    general = general || q.h != 0.0f || V.near() > 1e30f;
+    general = general || q.h != 0.0f;
     q.h = 1.0f;
   }
   const x3::Root R = x3::root(q);
@@ -109,16 +111,16 @@ __device__ __forceinline__ CornerX3 see_corner(const View& V, int c, const x3::F
   return C;
 }
 
-// Velocity of one vortex (all legs) at the point p; in_range: p is within 2^13;
-// rare(v, cnt): the general path's velocity and skips.  The legs are a loop, not
+// Velocity of one vortex (all legs), its `near` at most kNoX3, at the point p, within
+// 2^13; rare(v, cnt): the general path's velocity and skips.  The legs are a loop, not
 // unrolled: 3,000 instructions in a row run from the instruction cache's next
 // level (14.6 ms for 10,000 x 10,000 rings, against 12.5 ms so).
 template <int LEGS, typename View, typename Rare>
-__device__ __forceinline__ void vortex_velocity_x3(const View& V, const x3::F3* p, bool in_range,
-                                                   double& vx, double& vy, double& vz,
-                                                   int cnt[4], Rare rare) {
+__device__ __forceinline__ void vortex_velocity_x3(const View& V, const x3::F3* p, double& vx,
+                                                   double& vy, double& vz, int cnt[4],
+                                                   Rare rare) {
   constexpr bool kChain = LEGS != FVX_LEGS_CHORDWISE;  // a leg starts where the last one ended
-  bool general = !in_range;
+  bool general = false;
   double ux = 0.0, uy = 0.0, uz = 0.0;
   int on_start = 0, on_end = 0, on_line = 0;
   CornerX3 a, first;

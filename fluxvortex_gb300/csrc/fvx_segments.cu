@@ -152,6 +152,19 @@ __device__ void load_tile(const SegArgs& A, RawTile& raw, int64_t v0, int n) {
 }
 
 template <int LEGS>
+__device__ __forceinline__ void add_general(const VortexRec& R, double px, double py, double pz,
+                                            double& vx, double& vy, double& vz, int* cnt) {
+  double v[3] = {0.0, 0.0, 0.0};
+  int c[4] = {0, 0, 0, 0};
+  vortex_velocity_rare<LEGS>(R, px, py, pz, v, c);
+  vx += v[0];
+  vy += v[1];
+  vz += v[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) cnt[i] += c[i];
+}
+
+template <int LEGS>
 __global__ void __launch_bounds__(kCollSlices* kCollThreads) collapsed_kernel(SegArgs A) {
   __shared__ __align__(128) RawTile raw[2];
   __shared__ __align__(16) VortexRec rec[kTile];
@@ -221,11 +234,16 @@ __global__ void __launch_bounds__(kCollSlices* kCollThreads) collapsed_kernel(Se
       __syncthreads();
       if (active) {
 #pragma unroll 1
-        for (int k = slice; k < n; k += kCollSlices)
-          vortex_velocity_x3<LEGS>(RingView{recx[k]}, p, in_range, vx, vy, vz, cnt,
+        for (int k = slice; k < n; k += kCollSlices) {
+          if (!in_range || recx[k].near > kNoX3) {  // nothing of the three-float path is run
+            add_general<LEGS>(rec[k], px, py, pz, vx, vy, vz, cnt);
+            continue;
+          }
+          vortex_velocity_x3<LEGS>(RingView{recx[k]}, p, vx, vy, vz, cnt,
                                    [&](double* v, int* c) {
                                      vortex_velocity_rare<LEGS>(rec[k], px, py, pz, v, c);
                                    });
+        }
       }
       __syncthreads();
     }
@@ -290,6 +308,34 @@ __device__ __noinline__ void expanded_rare(const SegArgs& A, int64_t m, int64_t 
   vortex_velocity_rare<LEGS>(R, A.points[3 * p], A.points[3 * p + 1], A.points[3 * p + 2], v, cnt);
 }
 
+// The general path for a thread's vortex at the points of an expanded call that take
+// it: all of them, or those that are out of the three-float range.  One
+// preparation for all points (501 points x 1,003 rings in millimetres: 216 us,
+// 319 us with one per pair after the three-float path; 252 us is the reference's
+// sequence throughout).
+__device__ __forceinline__ bool point_in_range(const x3::F3* p) {
+  return p[0].h == p[0].h && p[1].h == p[1].h && p[2].h == p[2].h;  // (NaN: out of range)
+}
+template <int LEGS>
+__device__ __noinline__ void expanded_general(const SegArgs& A, int64_t m, int64_t p0, int np,
+                                              const x3::F3* pts, bool all, int* cnt) {
+  VortexRec R;
+  prep_vortex<LEGS>(R, A.corner[0] + 3 * m, A.corner[1] + 3 * m, A.corner[2] + 3 * m,
+                    A.corner[3] + 3 * m, A.strengths[m], A.rc0s[m], A.ages ? A.ages[m] : 0.0,
+                    A.nu);
+#pragma unroll 1
+  for (int k = 0; k < np; ++k) {
+    if (!all && point_in_range(pts + 3 * k)) continue;
+    const double* p = A.points + 3 * (p0 + k);
+    double v[3] = {0.0, 0.0, 0.0};
+    vortex_velocity_rare<LEGS>(R, p[0], p[1], p[2], v, cnt);
+    double* o = A.out + ((p0 + k) * A.n_vort + m) * 3;
+    o[0] = v[0];
+    o[1] = v[1];
+    o[2] = v[2];
+  }
+}
+
 // A thread's own vortex in shared memory, word w of thread t at [w][t] (no bank
 // conflicts; the legs' loop indexes corners and legs, which registers cannot).
 constexpr int kRingWords = 48;  // 12 coordinates and 4 leg lengths as three floats
@@ -316,10 +362,14 @@ __global__ void __launch_bounds__(kExpThreads) expanded_kernel(SegArgs A, int po
   const int64_t m = static_cast<int64_t>(blockIdx.x) * kExpThreads + threadIdx.x;
   const int64_t p0 = static_cast<int64_t>(blockIdx.y) * points_per_cta;
   const int np = static_cast<int>(min64(points_per_cta, A.n_points - p0));
+  bool far = false;  // points out of the three-float range
   for (int k = threadIdx.x; k < 3 * np; k += kExpThreads) {
     const double x = A.points[3 * p0 + k];
     pts[k] = x3::split_fast(x);
-    if (!x3_range(x)) pts[k].h = __int_as_float(0x7fffffff);  // NaN: the general path
+    if (!x3_range(x)) {
+      pts[k].h = __int_as_float(0x7fffffff);
+      far = true;
+    }
   }
   RingColumn col{words + threadIdx.x, consts + threadIdx.x, 0.0f};
   if (m < A.n_vort) {
@@ -341,14 +391,24 @@ __global__ void __launch_bounds__(kExpThreads) expanded_kernel(SegArgs A, int po
     consts[4 * kExpThreads + threadIdx.x] = X.half_c1;
     col.near_ = X.near;
   }
-  __syncthreads();
+  far = __syncthreads_or(far);
   if (np <= 0) return;
   int cnt[4] = {0, 0, 0, 0};
+  // a warp with a vortex out of range takes the general path as a whole, as it
+  // has to run it anyway
+  const bool all = __any_sync(0xffffffffu, col.near_ > kNoX3);
   if (m < A.n_vort) {
+    if (all || far) {
+      int c[4] = {0, 0, 0, 0};
+      expanded_general<LEGS>(A, m, p0, np, pts, all, c);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) cnt[i] += c[i];
+    }
 #pragma unroll 1
-    for (int k = 0; k < np; ++k) {
+    for (int k = 0; k < np && !all; ++k) {
+      if (far && !point_in_range(pts + 3 * k)) continue;
       double vx = 0.0, vy = 0.0, vz = 0.0;
-      vortex_velocity_x3<LEGS>(col, pts + 3 * k, true, vx, vy, vz, cnt, [&](double* v, int* c) {
+      vortex_velocity_x3<LEGS>(col, pts + 3 * k, vx, vy, vz, cnt, [&](double* v, int* c) {
         expanded_rare<LEGS>(A, m, p0 + k, v, c);
       });
       double* o = A.out + ((p0 + k) * A.n_vort + m) * 3;
