@@ -750,6 +750,9 @@ __global__ void __launch_bounds__(kLuClusterThreads)
     if ((tid >> 5) == (k0 >> 5)) {
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
+        // (missing columns would cost as much: a step is its shuffle and an FP64
+        // instruction; more exits slow down the blocks that are nearly full)
+        if (c < 16 ? n <= 16 && c >= n : n <= 16) break;
         const double xc = __shfl_sync(0xffffffffu, x, c);
         if (c < n && lane > c) x -= l[c] * xc;
       }
