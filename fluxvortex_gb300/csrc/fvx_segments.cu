@@ -438,9 +438,12 @@ int collapsed_splits(int64_t n_points, int64_t n_vort, int64_t* chunk) {
   return static_cast<int>(s);
 }
 
-// Work per CTA: an equal share of all (block, vortex) work for two CTAs per SM
-// (even, so that a run starts on a 16-byte boundary of the vortex arrays), or
-// whole blocks where those fill the GPU.
+// Work per CTA: an equal share of all (block, vortex) work for two CTAs per SM, or
+// whole blocks where those fill the GPU.  Shares are even, so that with an even
+// number of vortices a run starts on a 16-byte boundary of their arrays; from an
+// odd vortex on no bulk copy runs, which costs nothing that shows (reading the
+// first tile in one go and the others in bulk: 200 points x 101 rings 28.5 us
+// against 28.3, 1,000 x 1,001 155.8 against 155.5).
 int64_t collapsed_share(int64_t n_points, int64_t n_vort) {
   int64_t chunk = 0;
   if (collapsed_splits(n_points, n_vort, &chunk) == 1) return n_vort;
@@ -566,8 +569,11 @@ int segments_expanded_launch(const double* points, int64_t n_points, const doubl
   A.counts = counts;
   A.use_tma = 0;
   const int64_t gx = (n_vort + kExpThreads - 1) / kExpThreads;
-  // eight CTAs per SM: 501 points x 1,003 horseshoes take 125, 95, 87 and 97 us with
-  // 4, 6, 8 and 12 (fewer leave the FP32 pipe waiting, more repeat the prologue)
+  // eight CTAs per SM: fewer leave the FP32 pipe waiting, more repeat the prologue.
+  // Rings with 4, 6, 8, 10 and 12, us: 200 points x 501 rings 28.9, 28.8, 28.8, 28.7,
+  // 40.3; 200 x 3,000 128, 107, 93, 98, 111; 501 x 1,003 96, 83, 83, 86, 97; 1,500 x 501
+  // 132, 121, 112, 112, 128; 3,000 x 3,000 1,674, 1,385, 1,305, 1,330, 1,246; horseshoes
+  // alike; ten is better at 501 x 3,000 (293, 252, 240, 203, 223)
   const int64_t want = 8LL * device_sm_count();
   int64_t gy = gx >= want ? 1 : (want + gx - 1) / gx;
   if (gy > n_points) gy = n_points;

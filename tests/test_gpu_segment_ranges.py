@@ -4,7 +4,9 @@ warp and in one CTA, take different paths.  Against the FP64 oracle at the
 path's parity bar of 1e-12 (max |d| / max |ref|), with equal skip counts."""
 import numpy as np
 import pytest
+import torch
 
+from fluxvortex_gb300 import _capi
 from fluxvortex_gb300 import aerodynamics as A
 from oracle import oracle as O
 from tests.conftest import rel_err
@@ -78,3 +80,31 @@ def test_skip_tolerances_out_of_the_range(cuda, name):
     for j in (0, 17, 32):
         _check(name, np.concatenate([p[j:j + 1] for p in pts]), [q[j:j + 1] for q in c], 300.0)
     _check(name, np.concatenate(pts), c, 300.0)
+
+
+# odd counts over several blocks of 128 points: runs that start at odd vortices, where
+# no bulk copy is aligned; runs of less than a tile, around it and of several;
+# arrays of their own alignment and 8 bytes off it
+@pytest.mark.parametrize("name", FUNCTIONS[:3])
+@pytest.mark.parametrize("n,m", [(129, 1), (129, 3), (300, 101), (1000, 333), (2500, 1025),
+                                 (2500, 1153), (9001, 577)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_runs_from_odd_vortices(cuda, name, n, m, offset):
+    rng = np.random.default_rng(m)
+    c = _wake(m, 9)
+    pts = rng.uniform(-2, 2, (n, 3))
+    s, rc, ages = rng.standard_normal(m), np.full(m, 0.03), rng.uniform(0, 1, m)
+
+    def device(a):
+        flat = torch.empty(a.size + offset, dtype=torch.float64, device=cuda)[offset:]
+        return flat.copy_(torch.as_tensor(a.reshape(-1))).reshape(a.shape)
+
+    tail = (1.5e-5,) if "horseshoe" in name else (ages, 1.5e-5)
+    co = np.zeros(4, np.int64)
+    want = getattr(O, name)(pts, *c, s, rc, co, *tail)
+    cg = torch.zeros(4, dtype=torch.int64, device=cuda)
+    tail = (1.5e-5,) if "horseshoe" in name else (device(ages), 1.5e-5)
+    got = getattr(A, name)(*[device(a) for a in (pts, *c, s, rc)], cg, *tail)
+    assert rel_err(got.cpu().numpy(), want) < TOL
+    assert cg.tolist() == list(co)
+    assert _capi.status_read_and_clear() == 0
