@@ -33,6 +33,7 @@
 
 #include "fvx_common.cuh"
 #include "fvx_pair_math.cuh"
+#include "fvx_parts.cuh"
 #include "fvx_segment_math.cuh"
 
 namespace fvx {
@@ -48,11 +49,6 @@ constexpr double kC = -0.07957747154594767;  // -1/(4 pi): particle strength sca
 
 constexpr int kLegItems = 256;  // (point, ring) pairs per pass of the loads' leg terms
 constexpr int kLegStride = 17;  // doubles per pair: 4 legs of (c4, r3), one of padding
-
-// An FP64 number as three floats, exactly (24 + 24 + 5 bits).
-struct Parts {
-  float h, l, r;
-};
 
 // A wake ring for the mixed-precision sweep: corners in FP64 and in parts
 // (split_f32), and the leg constants rounded once here instead of per point.
@@ -95,39 +91,6 @@ struct Smem {
 };
 
 static_assert(sizeof(Smem) <= 227 * 1024, "the environment's state must fit shared memory");
-
-__device__ __forceinline__ Parts split_f32(double x) {
-  Parts p;
-  p.h = static_cast<float>(x);
-  const double y = x - static_cast<double>(p.h);
-  p.l = static_cast<float>(y);
-  p.r = static_cast<float>(y - static_cast<double>(p.l));
-  return p;
-}
-
-// float(x - y) of FP64 x and y in parts: the float of the rounded FP64
-// difference, bit for bit, without the FP64 pipe (one subtraction and one
-// conversion cost it about 130 FP32 issue slots).  x - y is h + l exactly, h the
-// leading parts' rounded difference and l the error of that (Knuth's two_sum)
-// plus the differences of the others; l rounds four times, by 2^-24 of at most
-// |e| + |a| + |b| each, and FP64's own rounding is 2^-53 |h|.  Where adding and
-// taking off that bound rounds to the same float, that float is the answer;
-// else (about 2^-20 of the pairs) `same` is cleared and the caller takes the
-// FP64 way.  Equal coordinates (particles on a point's span station) give zero
-// bounds and a zero.
-__device__ __forceinline__ float diff_f32(const Parts& x, const Parts& y, bool& same) {
-  const float h = x.h - y.h;
-  const float bb = h - x.h;
-  const float e = (x.h - (h - bb)) - (y.h + bb);
-  const float a = x.l - y.l, b = x.r - y.r;
-  const float l = e + (a + b);
-  const float w = fmaf(fabsf(h), 2.220446049250313e-16f,                            // 2^-52
-                       (fabsf(e) + (fabsf(a) + fabsf(b))) * 2.384185791015625e-07f);  // 2^-22
-  const float r0 = h + (l - w);
-  const float r1 = h + (l + w);
-  same = same && r0 == r1;
-  return r0;
-}
 
 // Deformed vertices and their velocities from the beam state in S.d / S.v.
 __device__ void deform(Smem& S, const FlutterParams& p) {
