@@ -21,12 +21,15 @@
 //   * every skip test is first a comparison of the high words, as integers,
 //     with a threshold on the safe side; only a pair inside that margin takes
 //     the tests themselves.
-// About 140 FP64 operations per ring and point against about 300.  The sweeps
-// (fvx_segments.cu) go further and form the scalar parts in three floats
-// (fvx_segment_x3.cuh), which pays where a vortex's record serves many points.
-// Against extended precision the error of a wake's velocities falls from
-// 1.4e-14 to 1.2e-15 (collapsed rings; 4e-16 in three floats): it was
-// la lb - c3's.
+// About 140 FP64 operations per ring and point against about 300: the AIC of 192
+// panels 20.6 us (26.7 with the reference's sequence), of 64 systems 955 us
+// (1,370).  The sweeps (fvx_segments.cu) go further and form the scalar parts in
+// three floats (fvx_segment_x3.cuh), which pays where a vortex's record serves
+// many points.
+// Against 113-bit arithmetic (max |error| / max |velocity|) the AIC of 120 panels
+// is off by 3.1e-16 (1.8e-15 by the reference's sequence), 400 points of a wake of
+// 1,000 rings by 2.4e-16 in three floats (9.4e-15): it was la lb - c3's
+// cancellation (tests/test_gpu_ring_precision.py).
 #pragma once
 
 #include "fvx_common.cuh"

@@ -492,15 +492,6 @@ __device__ void back_substitute(int P, const double* s_u, double* s_x, int tid) 
   }
 }
 
-// 1 / d to an ulp for d in the middle of the range: the hardware's approximation
-// (2^-20 or better) and a step of third order.
-__device__ __forceinline__ double reciprocal(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 // What a warp of the owner offers for the pivot: its largest magnitude by integer
 // comparisons of the words (NaNs count as zero), first row on ties.
 struct LuCandidate {
@@ -606,7 +597,7 @@ __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuClusterThre
       w = __double2loint(v);
       if (h > 0x7ff00000u || (h == 0x7ff00000u && w != 0)) h = w = 0;
     }
-    const double rcp = reciprocal(v);
+    const double rcp = seg::rcp_newton(v);
     const unsigned hm = __reduce_max_sync(0xffffffffu, h);
     const unsigned wm = __reduce_max_sync(0xffffffffu, h == hm ? w : 0u);
     const bool mine = in && h == hm && w == wm;
