@@ -561,7 +561,7 @@ def run_ours(args, rank, world):
     (mname, kern, nt, ns), durs = dom
     avg_ms = sum(durs) / len(durs)
     flop = FLOP_PER_PAIR.get((mname, kern), 0) * nt * ns
-    kname = f"pairs_kernel<{mname},{kern}>"
+    kname = f"pairs_{'f64' if args.precision == 'f64' else 'f32'}_kernel<{mname},{kern}>"
     if kern.startswith("tree/"):
         # treecode: the evaluation kernel's algorithmic work is its near pairs
         # plus its far (target, cell) expansions; its own launch time is timed

@@ -1283,7 +1283,7 @@ struct EvalArgs {
   const float* leaf_local;  // [leaves][32] learned local expansions, or null
   const float* parent_local;  // [parents][32] expansions shared by a parent's leaves, or null
   const int* leaf_parent;     // parent index of each leaf (with parent_local)
-  int* item_next;             // leaf counter of the resident evaluation warps (zeroed)
+  int* item_next;             // chunk counter of the resident evaluation warps (zeroed)
   const int2* items[2];       // (leaf, first particle) in chunks of 32 and 64, most work first
   const int* n_items;         // [2]
 };
@@ -3373,7 +3373,7 @@ int tree_sweep(fvx_tree* T, int mode, int kernel, const double* pos, const doubl
     FVX_CUDA_TRY(cudaEventCreate(&T->ev0));
     FVX_CUDA_TRY(cudaEventCreate(&T->ev1));
   }
-  // the resident evaluation warps' leaf counter
+  // the resident evaluation warps' chunk counter
   if ((rc = grow(T->eval_next, 16))) return rc;
   FVX_CUDA_TRY(cudaMemsetAsync(T->eval_next.p, 0, sizeof(int), s));
   A.item_next = P<int>(T->eval_next);
