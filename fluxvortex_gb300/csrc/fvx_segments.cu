@@ -308,24 +308,19 @@ __device__ __noinline__ void expanded_rare(const SegArgs& A, int64_t m, int64_t 
   vortex_velocity_rare<LEGS>(R, A.points[3 * p], A.points[3 * p + 1], A.points[3 * p + 2], v, cnt);
 }
 
-// The general path for a thread's vortex at the points of an expanded call that take
-// it: all of them, or those that are out of the three-float range.  One
-// preparation for all points (501 points x 1,003 rings in millimetres: 216 us,
-// 319 us with one per pair after the three-float path; 252 us is the reference's
-// sequence throughout).
-__device__ __forceinline__ bool point_in_range(const x3::F3* p) {
-  return p[0].h == p[0].h && p[1].h == p[1].h && p[2].h == p[2].h;  // (NaN: out of range)
-}
+// The general path for a thread's vortex at all points of the CTA.  One preparation
+// for all of them (501 points x 1,003 rings in millimetres: 216 us, 319 us with one
+// per pair after the three-float path; 252 us is the reference's sequence
+// throughout).
 template <int LEGS>
 __device__ __noinline__ void expanded_general(const SegArgs& A, int64_t m, int64_t p0, int np,
-                                              const x3::F3* pts, bool all, int* cnt) {
+                                              int* cnt) {
   VortexRec R;
   prep_vortex<LEGS>(R, A.corner[0] + 3 * m, A.corner[1] + 3 * m, A.corner[2] + 3 * m,
                     A.corner[3] + 3 * m, A.strengths[m], A.rc0s[m], A.ages ? A.ages[m] : 0.0,
                     A.nu);
 #pragma unroll 1
   for (int k = 0; k < np; ++k) {
-    if (!all && point_in_range(pts + 3 * k)) continue;
     const double* p = A.points + 3 * (p0 + k);
     double v[3] = {0.0, 0.0, 0.0};
     vortex_velocity_rare<LEGS>(R, p[0], p[1], p[2], v, cnt);
@@ -362,14 +357,11 @@ __global__ void __launch_bounds__(kExpThreads) expanded_kernel(SegArgs A, int po
   const int64_t m = static_cast<int64_t>(blockIdx.x) * kExpThreads + threadIdx.x;
   const int64_t p0 = static_cast<int64_t>(blockIdx.y) * points_per_cta;
   const int np = static_cast<int>(min64(points_per_cta, A.n_points - p0));
-  bool far = false;  // points out of the three-float range
+  bool far = false;  // a point out of the three-float range
   for (int k = threadIdx.x; k < 3 * np; k += kExpThreads) {
     const double x = A.points[3 * p0 + k];
     pts[k] = x3::split_fast(x);
-    if (!x3_range(x)) {
-      pts[k].h = __int_as_float(0x7fffffff);
-      far = true;
-    }
+    far = far || !x3_range(x);
   }
   RingColumn col{words + threadIdx.x, consts + threadIdx.x, 0.0f};
   if (m < A.n_vort) {
@@ -391,22 +383,19 @@ __global__ void __launch_bounds__(kExpThreads) expanded_kernel(SegArgs A, int po
     consts[4 * kExpThreads + threadIdx.x] = X.half_c1;
     col.near_ = X.near;
   }
-  far = __syncthreads_or(far);
+  // a CTA with a point or a warp with a vortex out of range takes the general path
+  // as a whole: its lanes would have to run both
+  const bool general = __syncthreads_or(far) || __any_sync(0xffffffffu, col.near_ > kNoX3);
   if (np <= 0) return;
   int cnt[4] = {0, 0, 0, 0};
-  // a warp with a vortex out of range takes the general path as a whole, as it
-  // has to run it anyway
-  const bool all = __any_sync(0xffffffffu, col.near_ > kNoX3);
-  if (m < A.n_vort) {
-    if (all || far) {
-      int c[4] = {0, 0, 0, 0};
-      expanded_general<LEGS>(A, m, p0, np, pts, all, c);
+  if (m < A.n_vort && general) {
+    int c[4] = {0, 0, 0, 0};
+    expanded_general<LEGS>(A, m, p0, np, c);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) cnt[i] += c[i];
-    }
+    for (int i = 0; i < 4; ++i) cnt[i] = c[i];
+  } else if (m < A.n_vort) {
 #pragma unroll 1
-    for (int k = 0; k < np && !all; ++k) {
-      if (far && !point_in_range(pts + 3 * k)) continue;
+    for (int k = 0; k < np; ++k) {
       double vx = 0.0, vy = 0.0, vz = 0.0;
       vortex_velocity_x3<LEGS>(col, pts + 3 * k, vx, vy, vz, cnt, [&](double* v, int* c) {
         expanded_rare<LEGS>(A, m, p0 + k, v, c);
