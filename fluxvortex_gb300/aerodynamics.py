@@ -9,9 +9,9 @@ Drop-in replacements for the five functions that
 
 Two call forms:
   * NumPy arrays (what PteraSoftware passes): synchronous, a new NumPy array is
-    returned.  Small collapsed calls are one launch that reads the inputs from
-    and writes the result to pinned host memory; the others make one
-    host-to-device transfer of all inputs, one fused launch and one
+    returned.  Small collapsed calls read the inputs from and write the result
+    to pinned host memory (a sweep and a sum of its partial results); the others
+    make one host-to-device transfer of all inputs, the same launches and one
     device-to-host transfer.
   * torch CUDA tensors: zero-copy, stream-ordered on torch's current stream;
     a new CUDA tensor is returned.
