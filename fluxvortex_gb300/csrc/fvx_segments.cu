@@ -27,8 +27,8 @@
 // Arithmetic per (point, leg): fvx_segment_x3.cuh.  The four skip tests take
 // the reference's decisions (warp_kernels.py:46-96).  10,000 points x 10,000
 // rings: 61.4 ms with the reference's sequence in FP64, 25.4 ms with its roots,
-// divisions and tests replaced (fvx_segment_math.cuh), 12.5 ms so; 501 points x
-// 1,003 horseshoes expanded 213, 145 and 87 us; 200 points x 100 rings 30, 27
+// divisions and tests replaced (fvx_segment_math.cuh), 12.6 ms so; 501 points x
+// 1,003 horseshoes expanded 213, 145 and 73 us; 200 points x 100 rings 30, 27
 // and 18 us on the device.
 #include "fvx_common.cuh"
 #include "fvx_segment_math.cuh"
